@@ -115,7 +115,6 @@ struct glst_handle {
   uint32_t k_begin = 0;             // first node (internal order) of this shard
   uint32_t lr_waves = 8;            // long-range CTAs ~ lr_waves x resident slots
   uint32_t lr_variant = 0;          // gather's FMA-pipe sin/cos share (kLrPolyMasks)
-  uint32_t sf_max_npt = dev::kSfMaxNpt;  // radial nodes per thread, at most, in the structure-factor units
   size_t part_cap = 0;              // rows the part buffer holds
   size_t sat_per_node = 0;          // shell-sum shared bytes per node
   size_t sat_budget = 0;            // shell-sum shared bytes per CTA, at most
@@ -149,12 +148,16 @@ struct glst_handle {
   float4 *dirs = nullptr;       // unit directions, FP32
   float *kappa = nullptr;       // radial scales per group, FP32
   dev::LrChunk *chunks = nullptr;
-  dev::SfUnit *sf_units = nullptr;  // structure-factor work units (whole directions)
-  size_t chunk_cap = 0, unit_cap = 0;         // entries the tables hold
-  bool chunks_owned = false, units_owned = false, part_owned = false;  // own cudaMalloc (else arena)
+  dev::DirTile *tiles = nullptr;    // runs of up to 32 directions of one group
+  float *cheb = nullptr;            // per group, n_radial x P: Chebyshev series of the phases (product basis)
+  dev::ChebScale cheb_scale{};
+  std::vector<uint32_t> g_cheb_P, g_cheb_tab;  // per group: series terms, offset of its table
+  uint32_t max_rad = 1;             // radial nodes per direction, at most
+  size_t chunk_cap = 0, tile_cap = 0;         // entries the tables hold
+  bool chunks_owned = false, tiles_owned = false, part_owned = false;  // own cudaMalloc (else arena)
   std::vector<dev::LrChunk> host_chunks;      // set-up: uploaded after the arena is committed
-  std::vector<dev::SfUnit> host_units;
-  uint32_t n_sf_units = 0;
+  std::vector<dev::DirTile> host_tiles;
+  uint32_t n_tiles = 0;
   // far field
   float2 *S = nullptr;
   float2 *R = nullptr;
@@ -176,7 +179,7 @@ struct glst_handle {
   // operand the whole node set would take.
   struct FarRange {
     uint32_t kb, ke, c0, c1;  // nodes and long-range chunks of one stage
-    uint32_t u0, u1;          // structure-factor units of the same nodes
+    uint32_t u0, u1;          // direction tiles of the same nodes
   };
   std::vector<FarRange> ranges;
   uint32_t stage_kmax = 0;    // nodes of the largest stage (S and R hold this many)
@@ -267,13 +270,13 @@ static void release(glst_handle *h, bool device_idle = false) {
   h->bufs.clear();
   h->pending.clear();
   if (h->chunks_owned && h->chunks) cudaFree(h->chunks);
-  if (h->units_owned && h->sf_units) cudaFree(h->sf_units);
+  if (h->tiles_owned && h->tiles) cudaFree(h->tiles);
   if (h->part_owned && h->part) cudaFree(h->part);
   h->chunks = nullptr;
-  h->sf_units = nullptr;
+  h->tiles = nullptr;
   h->part = nullptr;
-  h->chunks_owned = h->units_owned = h->part_owned = false;
-  h->chunk_cap = h->unit_cap = h->part_cap = 0;
+  h->chunks_owned = h->tiles_owned = h->part_owned = false;
+  h->chunk_cap = h->tile_cap = h->part_cap = 0;
   h->bytes = 0;
   if (h->side) cudaStreamDestroy(h->side);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -288,7 +291,7 @@ static void release(glst_handle *h, bool device_idle = false) {
 // bucket) for every later handle of that shape in this process.
 struct Tuning {
   uint32_t sat_nb = 0, lr_waves = 0;  // 0 = default
-  uint32_t lr_variant = 0, sf_max_npt = 0;
+  uint32_t lr_variant = 0;
 };
 static std::mutex g_tune_mu;
 static std::map<std::tuple<uint32_t, uint32_t, uint32_t>, Tuning> g_tune;
@@ -407,19 +410,14 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
   nst = std::min<uint64_t>(nst, std::max<size_t>(1, d1 - d0));
   std::vector<std::pair<size_t, size_t>> stage_dirs;  // [first, last) direction of each stage
   {
-    // directions per structure-factor unit of group gi: a stage ends on a
-    // unit boundary of its group (no partial unit inside a group's run but
-    // at its end), or at the end of a group
-    auto dpu = [&](uint32_t gi) {
-      const uint32_t nr = p.groups[gi].n_radial;
-      return (uint32_t)dev::kSfThreads / ((nr + h->sf_max_npt - 1) / h->sf_max_npt);
-    };
+    // a stage ends on a tile boundary of its group (no partial tile inside a
+    // group's run but at its end), or at the end of a group
     size_t i = d0;
     for (uint64_t st = 0; st < nst && i < d1; st++) {
       const uint64_t target_end = kb + K * (st + 1) / nst;  // node where this stage should end
       size_t e = i + 1;
       while (e < d1 && dirs_all[e].k < target_end) e++;
-      while (e < d1 && dirs_all[e].gi == dirs_all[e - 1].gi && dirs_all[e].j % dpu(dirs_all[e].gi) != 0) e++;
+      while (e < d1 && dirs_all[e].gi == dirs_all[e - 1].gi && dirs_all[e].j % 32 != 0) e++;
       if (st + 1 == nst) e = d1;
       stage_dirs.push_back({i, e});
       i = e;
@@ -427,7 +425,7 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
   }
   // chunks and units per stage
   std::vector<dev::LrChunk> chunks;
-  std::vector<dev::SfUnit> units;
+  std::vector<dev::DirTile> tiles;
   h->ranges.clear();
   h->stage_kmax = 0;
   h->part_rows = 1;
@@ -440,7 +438,7 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
     // kMinChunkNodes (partial-row traffic on small systems)
     const size_t target_nodes = chunk_nodes(h->nshards > 1 ? Kall / nst_sys : rg.ke - rg.kb);
     rg.c0 = (uint32_t)chunks.size();
-    rg.u0 = (uint32_t)units.size();
+    rg.u0 = (uint32_t)tiles.size();
     size_t i = sd.first;
     while (i < sd.second) {
       // this group's run of directions inside the stage
@@ -460,28 +458,23 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
         c.pad[0] = h->g_quad_base[gi];
         chunks.push_back(c);
       }
-      // Structure-factor units: the group's whole run cut into units of
-      // kSfThreads / nb directions, nb threads per direction of npt <=
-      // kSfMaxNpt radial nodes (cutting the whole run, not each chunk, keeps
-      // the units full).
-      const uint32_t nb = (g.n_radial + h->sf_max_npt - 1) / h->sf_max_npt;
-      const uint32_t npt = (g.n_radial + nb - 1) / nb;
-      const uint32_t dpu = dev::kSfThreads / nb;
-      for (uint32_t j0 = 0; j0 < n_dir; j0 += dpu) {
-        dev::SfUnit u{};
+      // Direction tiles: the group's whole run cut into runs of 32
+      // directions, one warp of the structure factors each.
+      for (uint32_t j0 = 0; j0 < n_dir; j0 += 32) {
+        dev::DirTile u{};
         u.node_begin = dirs_all[i].k + j0 * g.n_radial - kb;
         u.dir_begin = h->g_dir_base[gi] + j_first + j0;
-        u.n_dir = std::min(dpu, n_dir - j0);
+        u.n_dir = std::min(32u, n_dir - j0);
         u.n_rad = g.n_radial;
-        u.nb = nb;
-        u.npt = npt;
+        u.P = h->g_cheb_P[gi];
+        u.tab = h->g_cheb_tab[gi];
         u.kappa_begin = h->g_kappa_base[gi];
-        units.push_back(u);
+        tiles.push_back(u);
       }
       i = e;
     }
     rg.c1 = (uint32_t)chunks.size();
-    rg.u1 = (uint32_t)units.size();
+    rg.u1 = (uint32_t)tiles.size();
     if (rg.c1 - rg.c0 > 65535) return fail(GLST_ERR_SIZE, "too many long-range chunks in a node stage");
     h->stage_kmax = std::max(h->stage_kmax, rg.ke - rg.kb);
     h->part_rows = std::max(h->part_rows, rg.c1 - rg.c0);
@@ -490,8 +483,7 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
   // rows a later stage writes beyond what stage 0 writes start at zero
   h->part_zero_from = h->ranges.empty() ? h->part_rows : h->ranges[0].c1 - h->ranges[0].c0;
   h->nsplit = (uint32_t)chunks.size();
-  h->n_sf_units = (uint32_t)units.size();
-  if (units.size() > 0x7FFFFFFFu) return fail(GLST_ERR_SIZE, "too many structure-factor units");
+  h->n_tiles = (uint32_t)tiles.size();
   const size_t part_rows = h->part_rows;
   if (in_arena) {
     // first build (set-up): carve the tables and partial rows out of the
@@ -499,13 +491,13 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
     // small cudaMalloc calls here took 25-270 ms while a server's other
     // requests kept the GPU busy.
     GLST_TRY(dalloc_n(h, &h->chunks, std::max<size_t>(1, chunks.size())));
-    GLST_TRY(dalloc_n(h, &h->sf_units, std::max<size_t>(1, units.size())));
+    GLST_TRY(dalloc_n(h, &h->tiles, std::max<size_t>(1, tiles.size())));
     GLST_TRY(dalloc_n(h, &h->part, part_rows * std::max<size_t>(1, N)));
     h->chunk_cap = std::max<size_t>(1, chunks.size());
-    h->unit_cap = std::max<size_t>(1, units.size());
+    h->tile_cap = std::max<size_t>(1, tiles.size());
     h->part_cap = part_rows;
     h->host_chunks = std::move(chunks);
-    h->host_units = std::move(units);
+    h->host_tiles = std::move(tiles);
     return GLST_OK;
   }
   // rebuild (autotune): reuse the buffers when the new tables fit, else
@@ -526,16 +518,16 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
   };
   GLST_TRY(regrow(reinterpret_cast<void **>(&h->chunks), h->chunks_owned, h->chunk_cap,
                   std::max<size_t>(1, chunks.size()), sizeof(dev::LrChunk)));
-  GLST_TRY(regrow(reinterpret_cast<void **>(&h->sf_units), h->units_owned, h->unit_cap,
-                  std::max<size_t>(1, units.size()), sizeof(dev::SfUnit)));
+  GLST_TRY(regrow(reinterpret_cast<void **>(&h->tiles), h->tiles_owned, h->tile_cap,
+                  std::max<size_t>(1, tiles.size()), sizeof(dev::DirTile)));
   size_t part_cap_elems = h->part_cap * std::max<size_t>(1, N);
   GLST_TRY(regrow(reinterpret_cast<void **>(&h->part), h->part_owned, part_cap_elems,
                   part_rows * std::max<size_t>(1, N), sizeof(double4)));
   h->part_cap = part_cap_elems / std::max<size_t>(1, N);
   if (!chunks.empty())
     CUDA_TRY(cudaMemcpy(h->chunks, chunks.data(), chunks.size() * sizeof(dev::LrChunk), cudaMemcpyHostToDevice));
-  if (!units.empty())
-    CUDA_TRY(cudaMemcpy(h->sf_units, units.data(), units.size() * sizeof(dev::SfUnit), cudaMemcpyHostToDevice));
+  if (!tiles.empty())
+    CUDA_TRY(cudaMemcpy(h->tiles, tiles.data(), tiles.size() * sizeof(dev::DirTile), cudaMemcpyHostToDevice));
   return GLST_OK;
 }
 
@@ -549,6 +541,8 @@ static glst_status set_kernel_attributes(int device, size_t shell_smem) {
   std::lock_guard<std::mutex> lk(mu);
   int &d = done[device];
   if (!(d & 1)) {
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)dev::sf_smem_bytes(dev::kSfRadChunk)));
     CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(dev::kSortCap * sizeof(uint32_t))));
     d |= 1;
@@ -605,6 +599,17 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   std::vector<float4> dirs;
   std::vector<float> kap;
   std::vector<uint32_t> quad_base;  // per group, the first of its radial-scale quads
+  // Chebyshev series of the phases on |u| <= U, U the radius of the cell's
+  // circumscribed sphere and 2 % (atoms slightly outside the box stay within)
+  // Coordinates are scaled by 1 / U in FP32, so U is the reciprocal of an
+  // FP32 number: a rounded scale would stretch every phase alike.
+  const float cheb_inv = (float)(1.0 / (1.02 * 0.5 * std::sqrt(3.0) * p.cell_dim));
+  const double cheb_u = 1.0 / (double)cheb_inv;
+  h->cheb_scale = dev::ChebScale{cheb_inv, (float)(cheb_u * cheb_u)};
+  h->g_cheb_P.clear();
+  h->g_cheb_tab.clear();
+  h->max_rad = 1;
+  std::vector<float> cheb;
   dev::LrKappaQuads kq{};
   uint32_t nquad = 0;
   {
@@ -612,6 +617,19 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     for (size_t gi = 0; gi < (K ? p.groups.size() : 0); gi++) {
       const auto &g = p.groups[gi];
       kappa_base.push_back((uint32_t)kap.size());
+      h->max_rad = std::max(h->max_rad, g.n_radial);
+      {
+        const uint32_t P = glst::series_terms(*std::max_element(g.kappa.begin(), g.kappa.end()) * cheb_u, dev::kChebMaxP);
+        h->g_cheb_P.push_back(P);
+        h->g_cheb_tab.push_back((uint32_t)cheb.size());
+        std::vector<double> c(P);
+        for (unsigned r = 0; P && r < g.n_radial; r++) {
+          glst::phase_series(g.kappa[r] * cheb_u, P, c.data());
+          glst::product_basis(P, dev::cheb_b((int)P), c.data());
+          for (double v : c) cheb.push_back((float)v);
+          cheb.resize(cheb.size() + dev::cheb_row((int)P) - P, 0.f);
+        }
+      }
       dir_base.push_back((uint32_t)dirs.size());
       node_base.push_back(ibase);
       for (unsigned r = 0; r < g.n_radial; r++) kap.push_back((float)g.kappa[r]);
@@ -646,6 +664,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     GLST_TRY(dalloc_n(h, &h->node_radii, K));
     GLST_TRY(dalloc_n(h, &h->dirs, dirs.size()));
     GLST_TRY(dalloc_n(h, &h->kappa, kap.size()));
+    GLST_TRY(dalloc_n(h, &h->cheb, cheb.size()));
   }
   GLST_TRY(dalloc_n(h, &h->atom_cell, N));
   GLST_TRY(dalloc_n(h, &h->atom_slot, N));
@@ -717,7 +736,6 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
         h->sat_nb = pow2_floor(std::min<uint32_t>(t.sat_nb, (uint32_t)std::max<size_t>(1, budget / per_node)));
       if (t.lr_waves) h->lr_waves = t.lr_waves;
       h->lr_variant = t.lr_variant;
-      if (t.sf_max_npt) h->sf_max_npt = t.sf_max_npt;
     }
     GLST_TRY(build_chunks(h, /*in_arena=*/true));
     const size_t kpad = ((size_t)h->stage_kmax + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
@@ -736,16 +754,17 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   if (!h->host_chunks.empty()) {
     CUDA_TRY(cudaMemcpyAsync(h->chunks, h->host_chunks.data(), h->host_chunks.size() * sizeof(dev::LrChunk),
                              cudaMemcpyHostToDevice, h->side));
-    CUDA_TRY(cudaMemcpyAsync(h->sf_units, h->host_units.data(), h->host_units.size() * sizeof(dev::SfUnit),
+    CUDA_TRY(cudaMemcpyAsync(h->tiles, h->host_tiles.data(), h->host_tiles.size() * sizeof(dev::DirTile),
                              cudaMemcpyHostToDevice, h->side));
   }
   h->host_chunks.clear();
-  h->host_units.clear();
+  h->host_tiles.clear();
   if (K) {
     CUDA_TRY(cudaMemcpyAsync(h->node64, n64.data(), K * sizeof(double4), cudaMemcpyHostToDevice, h->side));
     CUDA_TRY(cudaMemcpyAsync(h->node_radii, radii.data(), K * sizeof(uint32_t), cudaMemcpyHostToDevice, h->side));
     CUDA_TRY(cudaMemcpyAsync(h->dirs, dirs.data(), dirs.size() * sizeof(float4), cudaMemcpyHostToDevice, h->side));
     CUDA_TRY(cudaMemcpyAsync(h->kappa, kap.data(), kap.size() * sizeof(float), cudaMemcpyHostToDevice, h->side));
+    CUDA_TRY(cudaMemcpyAsync(h->cheb, cheb.data(), cheb.size() * sizeof(float), cudaMemcpyHostToDevice, h->side));
   }
   if (shard > 0) CUDA_TRY(cudaMemsetAsync(h->sr, 0, (size_t)h->sr_rows * N * sizeof(double4), h->side));
   GLST_TRY(set_kernel_attributes(h->device, 0));
@@ -784,17 +803,22 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
   return GLST_OK;
 }
 
-// Far-field phases of one node stage: structure-factor units [u0, u1),
+// Far-field phases of one node stage: direction tiles [u0, u1),
 // shell sums over nodes [kb, ke), long-range chunks [c0, c1).  S and R hold
 // the stage's nodes (local index = node - rg.kb).
+static dev::SfArgs sf_args(const glst_handle *h, const glst_handle::FarRange &rg) {
+  return dev::SfArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
+                     reinterpret_cast<const float4 *>(h->cheb), h->S, h->R, h->cheb_scale, h->plan.ncell,
+                     rg.u1 - rg.u0, h->max_rad, rg.kb};
+}
+
 static glst_status sf_stage(glst_handle *h, const glst_handle::FarRange &rg, cudaStream_t st) {
   if (rg.u1 <= rg.u0 || !h->plan.natom) return GLST_OK;
-  const uint32_t cg = (h->plan.ncell + dev::kSfCellsPerCta - 1) / dev::kSfCellsPerCta;
-  for (uint32_t r0 = 0; r0 < cg; r0 += 65535u) {  // gridDim.y is at most 65,535
-    dim3 grid(rg.u1 - rg.u0, std::min<uint32_t>(cg - r0, 65535u));
-    dev::k_structure_factors<<<grid, dev::kSfThreads, 0, st>>>(h->pk, h->cell_count, h->cell_point, h->grid,
-                                                                h->sf_units + rg.u0, h->dirs, h->kappa, rg.kb,
-                                                                r0 * dev::kSfCellsPerCta, h->S, h->R);
+  const uint32_t nt = rg.u1 - rg.u0, quads = (nt + dev::kSfWarps - 1) / dev::kSfWarps;
+  const uint32_t per_launch = 0x7fffffffu / quads;  // cells (gridDim.x is at most 2^31 - 1)
+  for (uint32_t c0 = 0; c0 < h->plan.ncell; c0 += per_launch) {
+    const uint32_t nc = std::min(per_launch, h->plan.ncell - c0);
+    dev::k_structure_factors<<<quads * nc, dev::kSfThreads, dev::sf_smem_bytes(h->max_rad), st>>>(sf_args(h, rg), c0);
     CUDA_TRY(cudaGetLastError());
   }
   return GLST_OK;
@@ -1224,7 +1248,7 @@ glst_status glst_get_info(const glst_handle *h, glst_info *info) {
   info->node_stages = (uint32_t)h->ranges.size();
   info->shell_sums_form = h->gsat ? 1u : 0u;
   info->gather_variant = h->lr_variant;
-  info->sf_max_npt = h->sf_max_npt;
+  info->sf_max_npt = 12;
   return GLST_OK;
 }
 
@@ -1321,22 +1345,10 @@ glst_status glst_autotune(glst_handle *h, const double *rx, const double *ry, co
       if (ms < best) best = ms, best_v = v;
     }
     h->lr_variant = best_v;
-    // structure factors: radial nodes per thread, at most (units' shape)
-    uint32_t best_npt = h->sf_max_npt;
-    best = 1e30f;
-    for (uint32_t npt : {12u, 8u, 6u}) {
-      h->sf_max_npt = npt;
-      GLST_TRY(build_chunks(h));
-      float ms = 0.f;
-      GLST_TRY(timed(phase_sf, &ms));
-      if (ms < best) best = ms, best_npt = npt;
-    }
-    h->sf_max_npt = best_npt;
-    GLST_TRY(build_chunks(h));
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[tune_key(h->plan, h->K)] = Tuning{h->sat_nb, h->lr_waves, h->lr_variant, h->sf_max_npt};
+    g_tune[tune_key(h->plan, h->K)] = Tuning{h->sat_nb, h->lr_waves, h->lr_variant};
   }
   if (sat_nb) *sat_nb = h->sat_nb;
   if (lr_waves) *lr_waves = h->lr_waves;
@@ -1545,7 +1557,7 @@ struct glst_batch {
   // of another).
   struct WlGroup {
     uint32_t ph_off[kPhases] = {}, ph_n[kPhases] = {}, ph_grid[kPhases] = {};
-    size_t shell_smem = 0;              // dynamic shared memory of the shell-sum launch
+    size_t shell_smem = 0, sf_smem = 0; // dynamic shared memory of the shell-sum and structure-factor launches
     cudaStream_t side = nullptr;        // near field beside the far field
     cudaEvent_t fork = nullptr, join = nullptr;
   };
@@ -1599,7 +1611,6 @@ static bool worklist_ok(const glst_handle *h) {
   if (h->nshards != 1 || h->ranges.size() > 1 || h->gsat) return false;
   if (h->lr_variant != 0) return false;  // the work-list gather is the default variant
   if (h->K && h->sat_nb < 2) return false;
-  if ((h->plan.ncell + dev::kSfCellsPerCta - 1) / dev::kSfCellsPerCta > 65535u) return false;
   return true;
 }
 
@@ -1640,6 +1651,8 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
   int nsm = 148, smem_optin = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device));
   CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device));
+  CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)dev::sf_smem_bytes(dev::kSfRadChunk)));
   CUDA_TRY(cudaFuncSetAttribute(dev::k_shell_sums_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin));
   CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(dev::kSortCap * sizeof(uint32_t))));
@@ -1668,9 +1681,10 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     });
     each(glst_batch::kSf, [&](uint32_t w, glst_handle *h) {
       if (!h->K || !h->plan.natom) return;
-      const uint32_t rows = (h->plan.ncell + dev::kSfCellsPerCta - 1) / dev::kSfCellsPerCta;
-      for (uint32_t r = 0; r < rows; r++)
-        for (uint32_t u = 0; u < h->n_sf_units; u++) items.push_back({w, u, r, 0});
+      const uint32_t quads = (h->n_tiles + dev::kSfWarps - 1) / dev::kSfWarps;
+      gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad));
+      for (uint32_t c = 0; c < h->plan.ncell; c++)
+        for (uint32_t u = 0; u < quads; u++) items.push_back({w, u, c, 0});
     });
     each(glst_batch::kShell, [&](uint32_t w, glst_handle *h) {
       if (!h->K || !h->plan.natom) return;
@@ -1715,7 +1729,7 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     GLST_TRY(grid(glst_batch::kScan, (const void *)dev::k_scan_multi, 1024, 0));
     GLST_TRY(grid(glst_batch::kScatter, (const void *)dev::k_scatter_multi, 256, 0));
     GLST_TRY(grid(glst_batch::kSort, (const void *)dev::k_sort_pack_multi, 256, dev::kSortCap * sizeof(uint32_t)));
-    GLST_TRY(grid(glst_batch::kSf, (const void *)dev::k_structure_factors_multi, dev::kSfThreads, 0));
+    GLST_TRY(grid(glst_batch::kSf, (const void *)dev::k_structure_factors_multi, dev::kSfThreads, gr.sf_smem));
     GLST_TRY(grid(glst_batch::kShell, (const void *)dev::k_shell_sums_multi, dev::kSatThreads, gr.shell_smem));
     GLST_TRY(grid(glst_batch::kLr, (const void *)dev::k_long_range_multi, dev::kLrThreads, 0));
     GLST_TRY(grid(glst_batch::kSr, (const void *)dev::k_short_range_multi, dev::kSrThreads, 0));
@@ -1758,7 +1772,8 @@ static glst_status worklist_descriptors(glst_batch *b, const double *const in[4]
     d.atom_cell = h->atom_cell; d.atom_slot = h->atom_slot; d.perm = h->perm;
     d.sorted_idx = h->sorted_idx; d.cell_count = h->cell_count; d.cell_point = h->cell_point;
     d.pk = h->pk; d.pd = h->pd; d.dirs = h->dirs; d.kappa = h->kappa;
-    d.chunks = h->chunks; d.sf_units = h->sf_units;
+    d.chunks = h->chunks;
+    if (h->K && !h->ranges.empty()) d.sf = sf_args(h, h->ranges[0]);
     d.S = h->S; d.R = h->R; d.part = h->part; d.sr = h->sr; d.sr_rows = h->sr_rows;
     d.cfx = h->cfx; d.cfy = h->cfy; d.cfz = h->cfz; d.cen = h->cen;
     // input-order outputs straight into the batch's arrays (or the
@@ -1789,7 +1804,7 @@ static glst_status worklist_launch(glst_batch *b, glst_batch::WlGroup &gr, cudaS
   GLST_TRY(go(glst_batch::kScan, dev::k_scan_multi, 1024, 0, st));
   GLST_TRY(go(glst_batch::kScatter, dev::k_scatter_multi, 256, 0, st));
   GLST_TRY(go(glst_batch::kSort, dev::k_sort_pack_multi, 256, dev::kSortCap * sizeof(uint32_t), st));
-  GLST_TRY(go(glst_batch::kSf, dev::k_structure_factors_multi, dev::kSfThreads, 0, st));
+  GLST_TRY(go(glst_batch::kSf, dev::k_structure_factors_multi, dev::kSfThreads, gr.sf_smem, st));
   // near field forked after the structure factors, as in a single solve
   CUDA_TRY(cudaEventRecord(gr.fork, st));
   CUDA_TRY(cudaStreamWaitEvent(gr.side, gr.fork, 0));
@@ -2079,7 +2094,7 @@ uint64_t estimate_bytes(const Plan &p, int nsm) {
     const uint64_t chunks = std::max<uint64_t>((8 * slots + C - 1) / C, stage_k / kMaxChunkNodes + 1) +
                             p.groups.size() + 1;
     const uint64_t stage_kpad = (stage_k + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
-    b += K * (32 + 4 + 16 + 4) + C * stage_kpad * (8 + 8) + chunks * N * 32;
+    b += K * (32 + 4 + 16 + 4) + (uint64_t)max_nr * p.groups.size() * dev::kChebMaxP * 4 + C * stage_kpad * (8 + 8) + chunks * N * 32;
     // global-memory shell-sum tables (grids whose per-node table exceeds the
     // shared memory of a CTA): 64 MB or one block, and the twiddles
     if ((C + 9 + p.n[0] + p.n[1] + p.n[2]) * 16 > (200ull << 10))

@@ -315,42 +315,103 @@ __device__ __forceinline__ void fma_sincos_signed2(float2 th, float q, float2 *s
 // ----------------------------------------------------------------------------
 // Structure factors.  S_c(k) = sum_{j in c} q_j e^{-i k.r_j}
 //                            = e^{-i k.c} sum_j q_j e^{-i k.d_j},  d_j = r_j - c.
-// Nodes are k = kappa_r s (group -> direction -> radial), so per atom and
-// direction u = s.d_j is formed once and each node's phase is one multiply.
-// A CTA takes one work unit -- up to 128 / nb directions of one group, nb
-// threads per direction, each thread NPT consecutive radial nodes -- and
-// kSfCellsPerCta consecutive cells.  Per (atom, node): one multiply, a sine
-// and cosine (SFU, or the FMA-pipe polynomial for the last slot pairs), two
-// FMAs, in paired FP32 instructions where two slots go together.  FP32 over a
-// tile of <= kSfAtomTile atoms (|k.d| <~ 25 rad), then FP64 over the tiles of
-// a denser cell.  S is stored cell-relative in FP32; its twiddle e^{-ik.c}
-// is applied by the shell-sum kernel as it loads S.
-constexpr int kSfThreads = 128;
-constexpr int kSfMaxNpt = 12;     // radial nodes per thread, at most
-constexpr int kSfCellsPerCta = 2;
+// Nodes are k = kappa_r s (group -> direction -> radial).  On a direction's
+// ray every phase is kappa_r u with one u = s.d_j, |u| <= U (U: the cell's
+// circumscribed sphere and a margin), and
+//   e^{-i kappa u} = sum_p (2 - [p = 0]) (-i)^p J_p(kappa U) T_p(u / U)
+// (Jacobi-Anger) falls off faster than geometrically beyond p = kappa U (18,
+// 8 and 4 rad in water10k's groups): P = 36, 24 and 16 terms carry all 33,
+// 27 and 19 radial nodes to below the rounding of an FP32 phase.  So a
+// direction takes P real moments sum_j q_j T_p(x_j), one FMA each per atom,
+// and one P x n_rad product per cell -- where one sine and cosine per (atom,
+// node) kept the SFU and FMA pipes full (water10k 1.11 ms).
+//
+// The moments are formed in the product basis T_{Bg} T_b (b < B, p = Bg + b):
+// B + P/B recurrence steps and P accumulations per atom instead of P and P.
+// The host expands the Jacobi-Anger series in that basis in FP64
+// (cheb_product_basis); B is even, so even b feed the real part of S and odd
+// b the imaginary part, and a pair (b, b + 1) is one FFMA2 both when it is
+// accumulated and when it is multiplied out.
+//
+// One warp per (32 directions, cell), lane = direction, moments in
+// registers, atoms broadcast from shared memory: no CTA barriers, and groups
+// of few directions waste lanes of one warp only.  FP32 over a tile of <=
+// kSfAtomTile atoms, then FP64 over the tiles of a denser cell.  S is stored
+// cell-relative in FP32; its twiddle e^{-ik.c} is applied by the shell sums
+// as they load S.  Atoms beyond U (outside the box by more than the margin,
+// or not a number) and tiles of too few atoms for the product (16 atoms cost
+// as much as P terms) take one sine and cosine per node instead.
+// Measured: water10k 1.112 -> 0.341 ms, 1,000 waters on 4^3 cells 0.144 ->
+// 0.056 ms, 168 atoms per cell 0.313 -> 0.094 ms; forces 3.3e-8 -> 1.5e-8 off
+// the FP64 path.
+constexpr int kSfWarps = 4;
+constexpr int kSfThreads = 32 * kSfWarps;
 constexpr int kSfAtomTile = 128;
+constexpr int kSfRadChunk = 64;   // radial nodes staged at a time, at most
+constexpr int kChebMaxP = 64;     // series terms, at most (even to 48, then multiples of 4)
+__host__ __device__ constexpr int cheb_b(int P) { return P > 24 ? 8 : 4; }
+__host__ __device__ constexpr int cheb_row(int P) { return (P + 3) / 4 * 4; }  // table row, in floats
 
-struct SfUnit {
+// Up to 32 directions of one group.
+struct DirTile {
   uint32_t node_begin;   // local internal index of (first direction, r = 0)
   uint32_t dir_begin;    // global direction index of the first direction
-  uint32_t n_dir;        // directions in the unit (<= kSfThreads / nb)
+  uint32_t n_dir;        // directions in the tile (<= 32)
   uint32_t n_rad;        // radial nodes per direction in this group
-  uint32_t nb;           // threads per direction
-  uint32_t npt;          // radial nodes per thread (nb * npt >= n_rad)
+  uint32_t P;            // series terms, even (0: one sincos per node)
+  uint32_t tab;          // offset of the group's n_rad x cheb_row(P) table
   uint32_t kappa_begin;  // offset of this group's radial table
   uint32_t pad;
 };
 
-// Slot pairs on the FMA pipe.  Per slot a polynomial costs ~21 FP32
-// operations and a SFU slot 4 FP32 operations plus 2 MUFU operations, each of
-// which occupies the SFU for 8 cycles of a warp.  Measured on water10k
-// (npt 11 / 9 / 10 in its three groups): SF 1.47 ms with no pairs, 1.31 ms
-// with (npt - 1) / 4 (2/2/2), 1.25 ms with (npt - 3) / 4 (2/1/1), 1.28 ms
-// with one pair everywhere, 1.29 ms with (npt - 3) / 3 (2/2/2 + ...).
-// Re-measured with S stored cell-relative in FP32 (no FP64 epilogue): 1.10 ms
-// with (npt - 3) / 4, 1.16 with (npt - 5) / 4, 1.17 with npt / 4, 1.19 with
-// (npt - 1) / 4, 1.30 with (npt + 1) / 4.
-__host__ __device__ constexpr int sf_poly_pairs(int npt) { return (npt - 3) / 4; }
+// Per-handle constants of the series: 1 / U and the largest |d|^2 it takes.
+struct ChebScale {
+  float inv_u, u2;
+};
+
+// Arguments of the structure factors.  Tiles index nodes by the handle's
+// local node; S holds the nodes from node_off on (a node range of the handle:
+// the whole of it, or one stage).
+struct SfArgs {
+  const float4 *pk;
+  const uint32_t *cell_count, *cell_point;
+  const DirTile *tiles;
+  const float4 *dirs;
+  const float *kappa;
+  const float4 *tab;   // product-basis series, cheb_row(P) floats per radial node
+  float2 *S, *lo_buf;  // lo_buf: scratch of S's size
+  ChebScale cs;
+  uint32_t ncell, n_tiles, max_rad, node_off;
+};
+
+// Rows of the staged results are an odd number of float2 apart (bank spread).
+__host__ __device__ constexpr uint32_t sf_row(uint32_t rc) { return rc | 1u; }
+
+__host__ __device__ inline size_t sf_smem_bytes(uint32_t max_rad) {
+  const uint32_t rc = max_rad < (uint32_t)kSfRadChunk ? max_rad : (uint32_t)kSfRadChunk;
+  return (size_t)kSfWarps * (32 * sizeof(float4) + 32 * sf_row(rc) * sizeof(float2));
+}
+
+// The general form, one sine and cosine per (atom, node), added to the staged
+// results: the tile's atoms beyond the series' range (all: every atom).
+__device__ __noinline__ void sf_direct(const float4 *__restrict__ pk, uint32_t na, bool all, float u2, float4 s,
+                                       const float *__restrict__ kappa, uint32_t rc, float2 *__restrict__ row) {
+  for (uint32_t r = 0; r < rc; r++) {
+    const float kap = kappa[r];
+    float fr = 0.f, fi = 0.f;
+    for (uint32_t j = 0; j < na; j++) {
+      const float4 p = pk[j];
+      if (!all && fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z)) <= u2) continue;
+      const float u = fmaf(s.x, p.x, fmaf(s.y, p.y, s.z * p.z));
+      float sn, cs, qs;
+      fma_sincos_signed(kap * u, p.w, &sn, &cs, &qs);
+      fr = fmaf(qs, cs, fr);
+      fi = fmaf(qs, sn, fi);
+    }
+    const float2 o = row[r];
+    row[r] = make_float2(o.x + fr, o.y - fi);
+  }
+}
 
 // A cell of several tiles adds them in FP64: the running sum is kept between
 // tiles as an unevaluated pair of floats, the leading part in S and the
@@ -358,158 +419,174 @@ __host__ __device__ constexpr int sf_poly_pairs(int npt) { return (npt - 3) / 4;
 // the structure factors are done); the last tile stores the sum rounded once
 // to FP32.  Out of line, so that the registers of this rare path do not
 // count against the hot loop's.
-__device__ __noinline__ void sf_store_dense(const float2 *s_f, uint32_t nodes, uint32_t cell, uint32_t node0,
-                                            uint32_t ncell, bool add, bool last, float2 *__restrict__ S,
+__device__ __noinline__ void sf_store_dense(float2 f, size_t o, bool add, bool last, float2 *__restrict__ S,
                                             float2 *__restrict__ lo_buf) {
-  for (uint32_t m = threadIdx.x; m < nodes; m += kSfThreads) {
-    const size_t o = sr_index(cell, node0 + m, ncell);
-    const float2 f = s_f[m];
-    double vx = f.x, vy = f.y;
-    if (add) {
-      const float2 h = S[o], l = lo_buf[o];
-      vx += (double)h.x + (double)l.x;
-      vy += (double)h.y + (double)l.y;
+  double vx = f.x, vy = f.y;
+  if (add) {
+    const float2 h = S[o], l = lo_buf[o];
+    vx += (double)h.x + (double)l.x;
+    vy += (double)h.y + (double)l.y;
+  }
+  const float hx = static_cast<float>(vx), hy = static_cast<float>(vy);
+  S[o] = make_float2(hx, hy);
+  if (!last) lo_buf[o] = make_float2(static_cast<float>(vx - hx), static_cast<float>(vy - hy));
+}
+
+// Moments of one tile of atoms in N (pairs (b, b + 1) of the product basis).
+// The zeroth, the tile's charge, is the same for every direction and node, so
+// the rounding of an FP32 sum would act as a point charge at the cell centre
+// (1e-7 e per cell: water10k forces 2e-7 off FP64 against 3e-8): it is summed
+// in FP64.
+template <int P>
+__device__ __forceinline__ void sf_moments(const float4 *__restrict__ pk, uint32_t na, const ChebScale &cs, float4 s,
+                                           float4 *__restrict__ s_at, float2 (&N)[P / 2], bool &beyond) {
+  constexpr int B = cheb_b(P);
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int m = 0; m < P / 2; m++) N[m] = make_float2(0.f, 0.f);
+  double charge = 0.0;
+  for (uint32_t b0 = 0; b0 < na; b0 += 32) {
+    const uint32_t nb = min(32u, na - b0);
+    float4 p = lane < nb ? pk[b0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool in = fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z)) <= cs.u2;
+    beyond |= __any_sync(0xffffffffu, !in) != 0;
+    p = in ? make_float4(p.x * cs.inv_u, p.y * cs.inv_u, p.z * cs.inv_u, p.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+    charge += (double)p.w;
+    __syncwarp();
+    s_at[lane] = p;
+    __syncwarp();
+#pragma unroll 2
+    for (uint32_t j = 0; j < nb; j++) {
+      const float4 a = s_at[j];
+      const float x = fmaf(s.x, a.x, fmaf(s.y, a.y, s.z * a.z));
+      const float x2 = x + x;
+      float T[B + 1];
+      T[0] = 1.0f;
+      T[1] = x;
+#pragma unroll
+      for (int b = 2; b <= B; b++) T[b] = fmaf(x2, T[b - 1], -T[b - 2]);
+      const float tb2 = T[B] + T[B];
+      float g0 = a.w, g1 = a.w * T[B];
+#pragma unroll
+      for (int g = 0; g * B < P; g++) {
+        const float2 gg = bcast(g0);
+#pragma unroll
+        for (int b = 0; b < B && g * B + b < P; b += 2)
+          if (g == 0 && b == 0) N[0].y = fmaf(g0, x, N[0].y);
+          else N[(g * B + b) / 2] = __ffma2_rn(gg, make_float2(T[b], T[b + 1]), N[(g * B + b) / 2]);
+        const float g2 = fmaf(tb2, g1, -g0);
+        g0 = g1;
+        g1 = g2;
+      }
     }
-    const float hx = static_cast<float>(vx), hy = static_cast<float>(vy);
-    S[o] = make_float2(hx, hy);
-    if (!last) lo_buf[o] = make_float2(static_cast<float>(vx - hx), static_cast<float>(vy - hy));
   }
+  for (int o = 16; o > 0; o >>= 1) charge += __shfl_xor_sync(0xffffffffu, charge, o);
+  N[0].x = static_cast<float>(charge);
 }
 
-template <int NPT>
-__device__ __forceinline__ void sf_unit(const SfUnit &u, const float4 *__restrict__ pk,
-                                        const uint32_t *__restrict__ cell_count,
-                                        const uint32_t *__restrict__ cell_point, const Grid &g,
-                                        const float4 *__restrict__ dirs, const float *__restrict__ kappa,
-                                        uint32_t c0, uint32_t c1, uint32_t node_off, float2 *__restrict__ S,
-                                        float2 *__restrict__ lo_buf, float4 *s_at, float2 *s_f) {
-  // Slots are handled in pairs (FMUL2/FFMA2); an odd last slot alone.
-  constexpr int NP2 = NPT / 2;
-  constexpr bool ODD = (NPT & 1) != 0;
-  constexpr int POLY2 = sf_poly_pairs(NPT);  // pairs on the FMA pipe (the last ones)
-  const uint32_t d = threadIdx.x / u.nb;
-  const uint32_t b = threadIdx.x - d * u.nb;
-  const bool act = d < u.n_dir;
-  const uint32_t r0 = b * NPT;
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-  if (act) {
-    const float4 sd = dirs[u.dir_begin + d];
-    sx = sd.x; sy = sd.y; sz = sd.z;
-  }
-  float kap[NPT];
+template <int P>
+__device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const float4 *__restrict__ pk, uint32_t cnt,
+                                        uint32_t cell, float4 *s_at, float2 *s_f) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const float4 s = lane < u.n_dir ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t node0 = u.node_begin - a.node_off;
+  const float4 *rows = a.tab + u.tab / 4;
+  uint32_t a0 = 0;
+  do {
+    const uint32_t na = min((uint32_t)kSfAtomTile, cnt - a0);
+    // few atoms: a sine and cosine per node cost 16 issue slots of the SFU,
+    // the product P FMAs per node
+    const bool series = P > 0 && 16u * na > (uint32_t)P;
+    bool beyond = !series;
+    float2 N[P > 0 ? P / 2 : 1];
+    if constexpr (P > 0) {
+      if (series) sf_moments<P>(pk + a0, na, a.cs, s, s_at, N, beyond);
+    }
+    for (uint32_t r0 = 0; r0 < u.n_rad; r0 += kSfRadChunk) {
+      const uint32_t rc = min((uint32_t)kSfRadChunk, u.n_rad - r0);
+      float2 *row = s_f + lane * sf_row(rc);
+      __syncwarp();
+      if (series) {
+        if constexpr (P > 0) {
+#pragma unroll 2
+          for (uint32_t r = 0; r < rc; r++) {
+            const float4 *t = rows + (size_t)(r0 + r) * (cheb_row(P) / 4);
+            float2 f0 = make_float2(0.f, 0.f), f1 = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < NPT; i++) kap[i] = (act && r0 + i < u.n_rad) ? kappa[u.kappa_begin + r0 + i] : 0.f;
-  float2 kap2[NP2 > 0 ? NP2 : 1];
-#pragma unroll
-  for (int k = 0; k < NP2; k++) kap2[k] = make_float2(kap[2 * k], kap[2 * k + 1]);
-  const float kap_odd = kap[NPT - 1];
-  const uint32_t nodes = u.n_dir * u.n_rad;
-  for (uint32_t cell = c0; cell < c1; cell++) {
-    const uint32_t cnt = cell_count[cell];
-    const uint32_t start = cell_point[cell];
-    uint32_t a0 = 0;
-    do {
-      const uint32_t na = min((uint32_t)kSfAtomTile, cnt - a0);
-      __syncthreads();
-      // (the atoms read from the staged tile, one broadcast shared load per
-      // atom per thread; broadcast global loads instead measured slower,
-      // water10k 1.133 against 1.088 ms, bitwise-equal)
-      if (threadIdx.x < na) s_at[threadIdx.x] = pk[start + a0 + threadIdx.x];
-      __syncthreads();
-      // FR = sum q cos, FI = sum q sin (the sign of S's imaginary part is
-      // applied when the sums are stored)
-      float2 FR[NP2 > 0 ? NP2 : 1], FI[NP2 > 0 ? NP2 : 1];
-#pragma unroll
-      for (int k = 0; k < NP2; k++) { FR[k] = make_float2(0.f, 0.f); FI[k] = make_float2(0.f, 0.f); }
-      float fr_odd = 0.f, fi_odd = 0.f;
-#pragma unroll 1
-      for (uint32_t j = 0; j < na; j++) {
-        const float4 p = s_at[j];
-        const float uu = fmaf(sx, p.x, fmaf(sy, p.y, sz * p.z));
-        const float2 uu2 = bcast(uu);
-        const float2 q2 = bcast(p.w);
-#pragma unroll
-        for (int k = 0; k < NP2 - POLY2; k++) {
-          const float2 th = __fmul2_rn(kap2[k], uu2);
-          float sa, ca, sb, cb;
-          sfu_sincos(th.x, &sa, &ca);
-          sfu_sincos(th.y, &sb, &cb);
-          FR[k] = __ffma2_rn(q2, make_float2(ca, cb), FR[k]);
-          FI[k] = __ffma2_rn(q2, make_float2(sa, sb), FI[k]);
+            for (int m = 0; m < cheb_row(P) / 4; m++) {
+              const float4 c = __ldg(t + m);
+              f0 = __ffma2_rn(N[2 * m], make_float2(c.x, c.y), f0);
+              if (2 * m + 1 < P / 2) f1 = __ffma2_rn(N[2 * m + 1], make_float2(c.z, c.w), f1);
+            }
+            row[r] = __fadd2_rn(f0, f1);
+          }
         }
-#pragma unroll
-        for (int k = NP2 - POLY2; k < NP2; k++) {
-          float2 sn, cs, qs;
-          fma_sincos_signed2(__fmul2_rn(kap2[k], uu2), p.w, &sn, &cs, &qs);
-          FR[k] = __ffma2_rn(qs, cs, FR[k]);
-          FI[k] = __ffma2_rn(qs, sn, FI[k]);
-        }
-        if (ODD) {
-          float sn, cs;
-          sfu_sincos(kap_odd * uu, &sn, &cs);
-          fr_odd = fmaf(p.w, cs, fr_odd);
-          fi_odd = fmaf(p.w, sn, fi_odd);
-        }
-      }
-      // Tile sums to shared memory in the unit's node order, then one thread
-      // per node (coalesced) stores them.  S holds the cell-relative sums in
-      // FP32 (an FP32 tile sum; FP64 storage held no more information and
-      // doubled the bytes written here and read by the shell sums); the
-      // shell-sum kernel applies the twiddle e^{-ik.c} in FP64 from its
-      // per-axis tables as it loads S.
-      if (act) {
-#pragma unroll
-        for (int k = 0; k < NP2; k++) {
-          if (r0 + 2 * k < u.n_rad) s_f[d * u.n_rad + r0 + 2 * k] = make_float2(FR[k].x, -FI[k].x);
-          if (r0 + 2 * k + 1 < u.n_rad) s_f[d * u.n_rad + r0 + 2 * k + 1] = make_float2(FR[k].y, -FI[k].y);
-        }
-        if (ODD && r0 + NPT - 1 < u.n_rad) s_f[d * u.n_rad + r0 + NPT - 1] = make_float2(fr_odd, -fi_odd);
-      }
-      __syncthreads();
-      if (cnt <= kSfAtomTile) {
-        for (uint32_t m = threadIdx.x; m < nodes; m += kSfThreads)
-          S[sr_index(cell, u.node_begin + m - node_off, g.ncell)] = s_f[m];
       } else {
-        sf_store_dense(s_f, nodes, cell, u.node_begin - node_off, g.ncell, a0 > 0, a0 + kSfAtomTile >= cnt, S,
-                       lo_buf);
+        for (uint32_t r = 0; r < rc; r++) row[r] = make_float2(0.f, 0.f);
       }
-      a0 += kSfAtomTile;
-    } while (a0 < cnt);
-  }
+      if (beyond && na) sf_direct(pk + a0, na, !series, a.cs.u2, s, a.kappa + u.kappa_begin + r0, rc, row);
+      __syncwarp();
+      // Coalesced stores: a whole direction's radial nodes are contiguous, so
+      // with one chunk the tile's n_dir x n_rad nodes are one run; lanes are
+      // aligned to the node blocks of S.
+      if (rc == u.n_rad) {
+        const uint32_t j0 = node0 % kNodeBlock;
+        // m / rc by multiplication (m < 32 x 64), where rows are padded
+        const uint32_t inv = sf_row(rc) == rc ? 0u : 0xffffffffu / rc + 1u;
+        const uint32_t end = j0 + u.n_dir * rc;
+        size_t o = ((size_t)(node0 / kNodeBlock) * a.ncell + cell) * kNodeBlock + lane;
+        for (uint32_t k = lane; k < end; k += 32, o += (size_t)a.ncell * kNodeBlock) {
+          if (k < j0) continue;
+          const uint32_t m = k - j0;
+          const float2 f = s_f[m + __umulhi(m, inv)];
+          if (cnt <= kSfAtomTile) a.S[o] = f;
+          else sf_store_dense(f, o, a0 > 0, a0 + kSfAtomTile >= cnt, a.S, a.lo_buf);
+        }
+      } else {
+        for (uint32_t m = lane; m < u.n_dir * rc; m += 32) {
+          const uint32_t d = m / rc, r = m - d * rc;
+          const size_t o = sr_index(cell, node0 + d * u.n_rad + r0 + r, a.ncell);
+          const float2 f = s_f[d * sf_row(rc) + r];
+          if (cnt <= kSfAtomTile) a.S[o] = f;
+          else sf_store_dense(f, o, a0 > 0, a0 + kSfAtomTile >= cnt, a.S, a.lo_buf);
+        }
+      }
+    }
+    a0 += kSfAtomTile;
+  } while (a0 < cnt);
 }
 
-// Units index nodes by the handle's local node; S holds the nodes from
-// node_off on (a node range of the handle: the whole of it, or one stage).
-// Cells: kSfCellsPerCta per CTA row from cell_base on (grids of more than
-// 65,535 rows take several launches).  lo_buf: scratch of S's size.
-__device__ __forceinline__ void sf_block(const float4 *__restrict__ pk, const uint32_t *__restrict__ cell_count,
-                                         const uint32_t *__restrict__ cell_point, const Grid &g,
-                                         const SfUnit *__restrict__ units, const float4 *__restrict__ dirs,
-                                         const float *__restrict__ kappa, uint32_t node_off, uint32_t cell_base,
-                                         float2 *__restrict__ S, float2 *__restrict__ lo_buf, uint32_t bx,
-                                         uint32_t by) {
-  __shared__ float4 s_at[kSfAtomTile];
-  __shared__ float2 s_f[kSfThreads * kSfMaxNpt];
-  const SfUnit u = units[bx];
-  const uint32_t c0 = cell_base + by * kSfCellsPerCta;
-  const uint32_t c1 = min(g.ncell, c0 + kSfCellsPerCta);
+// Work item: kSfWarps consecutive tiles and a cell; warps are independent.
+__device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_t cell) {
+  extern __shared__ float4 s_sf[];
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t ti = quad * kSfWarps + warp;
+  if (ti >= a.n_tiles) return;
+  const uint32_t rc = min(a.max_rad, (uint32_t)kSfRadChunk);
+  float4 *s_at = s_sf + warp * 32;
+  float2 *s_f = reinterpret_cast<float2 *>(s_sf + kSfWarps * 32) + (size_t)warp * 32 * sf_row(rc);
+  const DirTile u = a.tiles[ti];
+  const uint32_t cnt = a.cell_count[cell];
+  const float4 *atoms = a.pk + a.cell_point[cell];
 #define GLST_SF_CASE(n) \
-  case n: sf_unit<n>(u, pk, cell_count, cell_point, g, dirs, kappa, c0, c1, node_off, S, lo_buf, s_at, s_f); break;
-  switch (u.npt) {
-    GLST_SF_CASE(1) GLST_SF_CASE(2) GLST_SF_CASE(3) GLST_SF_CASE(4) GLST_SF_CASE(5) GLST_SF_CASE(6)
-    GLST_SF_CASE(7) GLST_SF_CASE(8) GLST_SF_CASE(9) GLST_SF_CASE(10) GLST_SF_CASE(11) GLST_SF_CASE(12)
+  case n: sf_tile<n>(a, u, atoms, cnt, cell, s_at, s_f); break;
+  switch (u.P) {
+    GLST_SF_CASE(0) GLST_SF_CASE(4) GLST_SF_CASE(6) GLST_SF_CASE(8) GLST_SF_CASE(10)
+    GLST_SF_CASE(12) GLST_SF_CASE(14) GLST_SF_CASE(16) GLST_SF_CASE(18) GLST_SF_CASE(20)
+    GLST_SF_CASE(22) GLST_SF_CASE(24) GLST_SF_CASE(26) GLST_SF_CASE(28) GLST_SF_CASE(30)
+    GLST_SF_CASE(32) GLST_SF_CASE(34) GLST_SF_CASE(36) GLST_SF_CASE(38) GLST_SF_CASE(40)
+    GLST_SF_CASE(42) GLST_SF_CASE(44) GLST_SF_CASE(46) GLST_SF_CASE(48) GLST_SF_CASE(52)
+    GLST_SF_CASE(56) GLST_SF_CASE(60) GLST_SF_CASE(64)
     default: break;
   }
 #undef GLST_SF_CASE
 }
 
-__global__ void __launch_bounds__(kSfThreads, 8)
-k_structure_factors(const float4 *__restrict__ pk, const uint32_t *__restrict__ cell_count,
-                    const uint32_t *__restrict__ cell_point, Grid g, const SfUnit *__restrict__ units,
-                    const float4 *__restrict__ dirs, const float *__restrict__ kappa, uint32_t node_off,
-                    uint32_t cell_base, float2 *__restrict__ S, float2 *__restrict__ lo_buf) {
-  sf_block(pk, cell_count, cell_point, g, units, dirs, kappa, node_off, cell_base, S, lo_buf, blockIdx.x,
-           blockIdx.y);
+__global__ void __launch_bounds__(kSfThreads, 4)
+k_structure_factors(const __grid_constant__ SfArgs a, uint32_t cell_base) {
+  const uint32_t quads = (a.n_tiles + kSfWarps - 1) / kSfWarps;
+  const uint32_t c = blockIdx.x / quads;
+  sf_block(a, blockIdx.x - c * quads, cell_base + c);
 }
 
 // ----------------------------------------------------------------------------

@@ -68,6 +68,16 @@ Plan make_plan(uint32_t natom, double tol, const double box[3], double rcut,
                int ct_float, TDesignStore &store);
 double rcut_from_ncell(const double box[3], const uint32_t ncell[3]);
 
+// Chebyshev (Jacobi-Anger) series of the phases of one direction,
+//   e^{-i z x} = sum_p c_p(z) (-i or 1)^{p odd} T_p(x),  |x| <= 1:
+// number of terms (even; above 48 a multiple of 4; 0 when more than
+// max_terms would be needed) with which every z in [0, z_max] is exact to below FP32 rounding,
+// the signed coefficients, and their conversion to the basis T_{Bg} T_b,
+// p = Bg + b, b < B (in place).
+unsigned series_terms(double z_max, unsigned max_terms);
+void phase_series(double z, unsigned P, double *c);
+void product_basis(unsigned P, unsigned B, double *c);
+
 // Exposed for tests of the numerics set-up.
 double erfc_inverse(double y, double tol);
 std::vector<double> gauss_legendre_roots(unsigned n);

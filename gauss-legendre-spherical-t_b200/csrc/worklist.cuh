@@ -25,7 +25,7 @@ struct SysDesc {
   const float4 *dirs;
   const float *kappa;
   const LrChunk *chunks;
-  const SfUnit *sf_units;
+  SfArgs sf;    // structure-factor arguments
   float2 *S, *R;
   double4 *part, *sr;
   double *cfx, *cfy, *cfz, *cen, *ofx, *ofy, *ofz, *oen, *block_energy, *energy;
@@ -85,16 +85,20 @@ __global__ void __launch_bounds__(256) k_sort_pack_multi(const SysDesc *__restri
   }
 }
 
-// item (a, b) = (structure-factor unit, cell row).  Seven CTAs per SM (72
-// registers): the descriptor's pointers take registers the one-system kernel
-// reads from its parameters, and at eight CTAs (64 registers) they spilled.
-__global__ void __launch_bounds__(kSfThreads, 7) k_structure_factors_multi(const SysDesc *__restrict__ sys,
+// item (a, b) = (quad of direction tiles, cell).  The arguments are copied to
+// shared memory and the body is called out of line: inlined into the item
+// loop its moments were spilled to local memory.
+__device__ __noinline__ void sf_item(const SfArgs &a, uint32_t quad, uint32_t cell) { sf_block(a, quad, cell); }
+
+__global__ void __launch_bounds__(kSfThreads, 4) k_structure_factors_multi(const SysDesc *__restrict__ sys,
                                                                           const WorkItem *__restrict__ items,
                                                                           uint32_t n) {
+  __shared__ SfArgs s_args;
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
-    const SysDesc &d = sys[w.sys];
-    sf_block(d.pk, d.cell_count, d.cell_point, d.g, d.sf_units, d.dirs, d.kappa, 0, 0, d.S, d.R, w.a, w.b);
+    if (threadIdx.x == 0) s_args = sys[w.sys].sf;
+    __syncthreads();
+    sf_item(s_args, w.a, w.b);
     __syncthreads();
   }
 }
