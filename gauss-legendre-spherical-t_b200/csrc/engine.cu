@@ -100,6 +100,8 @@ static std::shared_ptr<TDesignStore> get_store() {
 }
 
 // ---------------------------------------------------------------- handle
+static constexpr uint32_t kLrWaves = 4;  // waves of gather warps, untuned
+
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
@@ -110,11 +112,9 @@ struct glst_handle {
   int device = 0;
   dev::Grid grid{};
   uint32_t K = 0;
-  uint32_t nsplit = 1;  // long-range chunks (rows of part)
   uint32_t shard = 0, nshards = 1;  // node split across devices (1 = whole system)
   uint32_t k_begin = 0;             // first node (internal order) of this shard
-  uint32_t lr_waves = 8;            // long-range CTAs ~ lr_waves x resident slots
-  uint32_t lr_variant = 0;          // gather's FMA-pipe sin/cos share (kLrPolyMasks)
+  uint32_t lr_waves = kLrWaves;     // gather warps ~ lr_waves x resident slots
   size_t part_cap = 0;              // rows the part buffer holds
   size_t sat_per_node = 0;          // shell-sum shared bytes per node
   size_t sat_budget = 0;            // shell-sum shared bytes per CTA, at most
@@ -122,8 +122,6 @@ struct glst_handle {
   uint32_t sr_rows = dev::kSrRowsPlanes;  // near-field partial-sum rows
   size_t smem_sm = 0;  // shared memory per SM, less four CTAs' system reserve
   std::vector<uint32_t> g_node_base, g_dir_base, g_kappa_base;  // per group, internal order
-  std::vector<uint32_t> g_quad_base;  // per group, first radial-scale quad in kquads
-  dev::LrKappaQuads kquads{};         // the gather's radial scales (parameter space)
   uint32_t sat_nb = 1, sat_stride = 0;
   bool sat_xyz = true;  // shell-sum cell-coordinate table in shared memory
   uint32_t combine_blocks = 1;
@@ -147,16 +145,16 @@ struct glst_handle {
   uint32_t *node_radii = nullptr;
   float4 *dirs = nullptr;       // unit directions, FP32
   float *kappa = nullptr;       // radial scales per group, FP32
-  dev::LrChunk *chunks = nullptr;
   dev::DirTile *tiles = nullptr;    // runs of up to 32 directions of one group
-  float *cheb = nullptr;            // per group, n_radial x P: Chebyshev series of the phases (product basis)
+  float *cheb = nullptr;            // per group, n_radial x P: Chebyshev series of the phases
+                                    // (structure factors: product basis; gather: plain)
   dev::ChebScale cheb_scale{};
-  std::vector<uint32_t> g_cheb_P, g_cheb_tab;  // per group: series terms, offset of its table
+  std::vector<uint32_t> g_sf_P, g_sf_tab, g_lr_P, g_lr_tab;  // per group: series terms, offset of the table
+  uint32_t sf_tab4 = 0;             // float4s of the largest structure-factor table
   uint32_t max_rad = 1;             // radial nodes per direction, at most
-  size_t chunk_cap = 0, tile_cap = 0;         // entries the tables hold
-  bool chunks_owned = false, tiles_owned = false, part_owned = false;  // own cudaMalloc (else arena)
-  std::vector<dev::LrChunk> host_chunks;      // set-up: uploaded after the arena is committed
-  std::vector<dev::DirTile> host_tiles;
+  size_t tile_cap = 0;              // entries the table holds
+  bool tiles_owned = false, part_owned = false;  // own cudaMalloc (else arena)
+  std::vector<dev::DirTile> host_tiles;       // set-up: uploaded after the arena is committed
   uint32_t n_tiles = 0;
   // far field
   float2 *S = nullptr;
@@ -178,8 +176,10 @@ struct glst_handle {
   // hold one stage's nodes; a large system needs a fraction of the C x K
   // operand the whole node set would take.
   struct FarRange {
-    uint32_t kb, ke, c0, c1;  // nodes and long-range chunks of one stage
+    uint32_t kb, ke;          // nodes of one stage
     uint32_t u0, u1;          // direction tiles of the same nodes
+    uint32_t tpc;             // tiles per long-range chunk
+    uint32_t rows() const { return (u1 - u0 + tpc - 1) / tpc; }  // long-range chunks
   };
   std::vector<FarRange> ranges;
   uint32_t stage_kmax = 0;    // nodes of the largest stage (S and R hold this many)
@@ -269,14 +269,12 @@ static void release(glst_handle *h, bool device_idle = false) {
   for (auto &b : h->bufs) cudaFreeAsync(b.p, h->side);
   h->bufs.clear();
   h->pending.clear();
-  if (h->chunks_owned && h->chunks) cudaFree(h->chunks);
   if (h->tiles_owned && h->tiles) cudaFree(h->tiles);
   if (h->part_owned && h->part) cudaFree(h->part);
-  h->chunks = nullptr;
   h->tiles = nullptr;
   h->part = nullptr;
-  h->chunks_owned = h->tiles_owned = h->part_owned = false;
-  h->chunk_cap = h->tile_cap = h->part_cap = 0;
+  h->tiles_owned = h->part_owned = false;
+  h->tile_cap = h->part_cap = 0;
   h->bytes = 0;
   if (h->side) cudaStreamDestroy(h->side);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -291,7 +289,6 @@ static void release(glst_handle *h, bool device_idle = false) {
 // bucket) for every later handle of that shape in this process.
 struct Tuning {
   uint32_t sat_nb = 0, lr_waves = 0;  // 0 = default
-  uint32_t lr_variant = 0;
 };
 static std::mutex g_tune_mu;
 static std::map<std::tuple<uint32_t, uint32_t, uint32_t>, Tuning> g_tune;
@@ -320,14 +317,16 @@ static uint64_t stage_budget() {
   return b;
 }
 
-// Nodes per gather chunk, at most (a CTA's work is 128 atoms x its chunk's
-// nodes; water10k's chunks hold ~1,800 nodes) and at least: every chunk
-// writes a partial row of 32 bytes per atom that the combine reads back, so
-// 256 nodes or more keep that traffic at <= 0.25 byte per (atom, node) pair
-// (the 3,000-atom, 4^3-cell system had 33-node chunks: 28 MB of partial
-// rows, 2 bytes per pair, against 10 MB of S and R).
-static constexpr size_t kMaxChunkNodes = 2048;
-static constexpr size_t kMinChunkNodes = 256;
+// Direction tiles per gather chunk (a warp's work: a cell and a chunk).  Every
+// chunk writes a partial row of 32 bytes per atom that the combine reads back
+// and stages the cell's atoms, so at least two tiles, and no
+// more chunks than fill the GPU with `waves` waves of warps; at most 16 tiles, so that the last wave stays
+// short on large grids.
+static uint32_t tiles_per_chunk(size_t n_tiles, size_t ncell, uint32_t waves, int nsm) {
+  const size_t slots = (size_t)nsm * 12;
+  const size_t chunks = std::max<size_t>(1, ((size_t)waves * slots + ncell - 1) / ncell);
+  return (uint32_t)std::max<size_t>(2, std::min<size_t>(16, n_tiles / chunks));
+}
 
 // Near-field rows (kernels.cuh): nine when three rows' CTAs (one per cell
 // and x plane) would be fewer than six per SM (up to 6^3 cells on B200:
@@ -343,160 +342,116 @@ static uint32_t pow2_floor(uint32_t v) {
   return p;
 }
 
-// Node stages and long-range chunks.  First this handle's node range: all
-// nodes, or -- when the system is split over several devices -- a contiguous
-// run of whole directions holding about K / nshards nodes (the reference
-// splits its node list into contiguous per-GPU ranges,
-// src/glst_force.cu:276-293).  Then stages: contiguous runs of whole
-// directions of about equal node count, as many as the S + R budget needs.
-// Then, per stage, long-range chunks (whole directions of one group) sized so
-// that the gather's grid is about lr_waves waves of resident CTAs, and the
-// structure-factor units.
-static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
+// Node stages, direction tiles and long-range chunks.  The nodes are cut into
+// tiles of up to 32 directions of one group, one warp each of the structure
+// factors and the gather.  First this handle's tiles: all of them, or -- when
+// the system is split over several devices -- a contiguous run holding about
+// K / nshards nodes (the reference splits its node list into contiguous
+// per-GPU ranges, src/glst_force.cu:276-293).  Then stages: contiguous runs
+// of tiles of about equal node count, as many as the S + R budget needs.
+// Then, per stage, long-range chunks: runs of tiles_per_chunk tiles.  (FP32
+// sums stay within a tile, everything across tiles is FP64, so neither the
+// shards nor the chunks change a result beyond FP64 rounding.)
+static glst_status build_tiles(glst_handle *h, bool in_arena = false) {
   const Plan &p = h->plan;
   const size_t C = p.ncell, Kall = p.has_far ? p.K() : 0, N = p.natom;
-  const size_t slots = (size_t)h->nsm * 16;
-  const size_t want_chunks = std::max<size_t>(1, ((size_t)h->lr_waves * slots + C - 1) / C);
-  struct Dir {
-    uint32_t gi, j;  // group, direction within the group
-    uint32_t k;      // first node (internal order) of the direction
+  struct Tile {
+    uint32_t gi, j, n;  // group, first direction within the group, directions
+    uint32_t k, ke;     // nodes (internal order)
   };
-  std::vector<Dir> dirs_all;
-  for (size_t gi = 0; gi < (Kall ? p.groups.size() : 0); gi++)
-    for (uint32_t j = 0; j < p.groups[gi].n_dir; j++)
-      dirs_all.push_back({(uint32_t)gi, j, h->g_node_base[gi] + j * p.groups[gi].n_radial});
-  auto dir_nodes = [&](const Dir &d) { return p.groups[d.gi].n_radial; };
-  // The whole system's stage count and chunk size.  A shard cuts its chunks
-  // at the whole system's chunk size, so that its chunks are exactly the
-  // whole system's chunks of its node range (the shards' sum then groups
-  // every FP32 partial sum as the unsharded solve).
+  std::vector<Tile> all;
+  for (size_t gi = 0; gi < (Kall ? p.groups.size() : 0); gi++) {
+    const auto &g = p.groups[gi];
+    for (uint32_t j = 0; j < g.n_dir; j += 32) {
+      const uint32_t n = std::min(32u, g.n_dir - j), k = h->g_node_base[gi] + j * g.n_radial;
+      all.push_back({(uint32_t)gi, j, n, k, k + n * g.n_radial});
+    }
+  }
   const uint64_t kpad_sys = (Kall + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
   const uint64_t nst_sys = std::max<uint64_t>(1, (C * kpad_sys * 16 + stage_budget() - 1) / stage_budget());
-  auto chunk_nodes = [&](size_t stage_nodes) {
-    return std::max<size_t>(kMinChunkNodes, std::min<size_t>(kMaxChunkNodes, stage_nodes / want_chunks));
-  };
-  // this handle's directions [d0, d1)
-  size_t d0 = 0, d1 = dirs_all.size();
+  // the whole system's chunk size; a shard takes whole chunks of it
+  const uint32_t tpc_sys = tiles_per_chunk(all.size() / nst_sys, C, h->lr_waves, h->nsm);
+  // this handle's tiles [d0, d1)
+  size_t d0 = 0, d1 = all.size();
   if (h->nshards > 1 && Kall) {
-    // shard by provisional chunks of the whole system's chunk size, each
-    // assigned to the shard its middle node falls in
-    const size_t target = chunk_nodes(Kall / nst_sys);
     bool any = false;
-    size_t i = 0;
-    while (i < dirs_all.size()) {
-      const uint32_t gi = dirs_all[i].gi;
-      const uint32_t dpc = (uint32_t)std::max<size_t>(1, target / p.groups[gi].n_radial);
-      size_t e = i;
-      while (e < dirs_all.size() && dirs_all[e].gi == gi && e - i < dpc) e++;
-      const uint64_t nodes = (uint64_t)(e - i) * p.groups[gi].n_radial;
-      const uint64_t mid = (uint64_t)dirs_all[i].k + nodes / 2;
+    for (size_t i = 0; i < all.size(); i += tpc_sys) {
+      const size_t e = std::min(all.size(), i + tpc_sys);
+      const uint64_t mid = ((uint64_t)all[i].k + all[e - 1].ke) / 2;
       if (mid * h->nshards / Kall == h->shard) {
         if (!any) d0 = i;
         d1 = e;
         any = true;
       }
-      i = e;
     }
     if (!any) d0 = d1 = 0;
   }
-  const uint32_t kb = d0 < d1 ? dirs_all[d0].k : 0;
-  const uint32_t ke = d0 < d1 ? dirs_all[d1 - 1].k + dir_nodes(dirs_all[d1 - 1]) : 0;
+  const uint32_t kb = d0 < d1 ? all[d0].k : 0;
   h->k_begin = kb;
-  h->K = ke - kb;
+  h->K = (d0 < d1 ? all[d1 - 1].ke : 0) - kb;
   const uint64_t K = h->K;
   // stages
   const uint64_t kpad_all = (K + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
   uint64_t nst = std::max<uint64_t>(1, (C * kpad_all * 16 + stage_budget() - 1) / stage_budget());
   nst = std::min<uint64_t>(nst, std::max<size_t>(1, d1 - d0));
-  std::vector<std::pair<size_t, size_t>> stage_dirs;  // [first, last) direction of each stage
-  {
-    // a stage ends on a tile boundary of its group (no partial tile inside a
-    // group's run but at its end), or at the end of a group
-    size_t i = d0;
-    for (uint64_t st = 0; st < nst && i < d1; st++) {
-      const uint64_t target_end = kb + K * (st + 1) / nst;  // node where this stage should end
-      size_t e = i + 1;
-      while (e < d1 && dirs_all[e].k < target_end) e++;
-      while (e < d1 && dirs_all[e].gi == dirs_all[e - 1].gi && dirs_all[e].j % 32 != 0) e++;
-      if (st + 1 == nst) e = d1;
-      stage_dirs.push_back({i, e});
-      i = e;
-    }
-  }
-  // chunks and units per stage
-  std::vector<dev::LrChunk> chunks;
   std::vector<dev::DirTile> tiles;
   h->ranges.clear();
   h->stage_kmax = 0;
   h->part_rows = 1;
-  for (const auto &sd : stage_dirs) {
+  size_t i = d0;
+  for (uint64_t st = 0; st < nst && i < d1; st++) {
+    const uint64_t target_end = kb + K * (st + 1) / nst;  // node where this stage should end
+    size_t e = i + 1;
+    while (e < d1 && (st + 1 == nst || all[e].k < target_end)) e++;
     glst_handle::FarRange rg{};
-    rg.kb = dirs_all[sd.first].k - kb;
-    rg.ke = dirs_all[sd.second - 1].k + dir_nodes(dirs_all[sd.second - 1]) - kb;
-    // ... and at most kMaxChunkNodes nodes, so that on large systems (few
-    // chunks fill the GPU) the last wave of gather CTAs stays short; at least
-    // kMinChunkNodes (partial-row traffic on small systems)
-    const size_t target_nodes = chunk_nodes(h->nshards > 1 ? Kall / nst_sys : rg.ke - rg.kb);
-    rg.c0 = (uint32_t)chunks.size();
+    rg.kb = all[i].k - kb;
+    rg.ke = all[e - 1].ke - kb;
     rg.u0 = (uint32_t)tiles.size();
-    size_t i = sd.first;
-    while (i < sd.second) {
-      // this group's run of directions inside the stage
-      const uint32_t gi = dirs_all[i].gi;
-      const auto &g = p.groups[gi];
-      size_t e = i;
-      while (e < sd.second && dirs_all[e].gi == gi) e++;
-      const uint32_t n_dir = (uint32_t)(e - i), j_first = dirs_all[i].j;
-      const uint32_t dpc = (uint32_t)std::max<size_t>(1, target_nodes / g.n_radial);
-      for (uint32_t j0 = 0; j0 < n_dir; j0 += dpc) {
-        dev::LrChunk c{};
-        c.n_dir = std::min(dpc, n_dir - j0);
-        c.n_rad = g.n_radial;
-        c.node_begin = dirs_all[i].k + j0 * g.n_radial - kb;
-        c.dir_begin = h->g_dir_base[gi] + j_first + j0;
-        c.kappa_begin = h->g_kappa_base[gi];
-        c.pad[0] = h->g_quad_base[gi];
-        chunks.push_back(c);
-      }
-      // Direction tiles: the group's whole run cut into runs of 32
-      // directions, one warp of the structure factors each.
-      for (uint32_t j0 = 0; j0 < n_dir; j0 += 32) {
-        dev::DirTile u{};
-        u.node_begin = dirs_all[i].k + j0 * g.n_radial - kb;
-        u.dir_begin = h->g_dir_base[gi] + j_first + j0;
-        u.n_dir = std::min(32u, n_dir - j0);
-        u.n_rad = g.n_radial;
-        u.P = h->g_cheb_P[gi];
-        u.tab = h->g_cheb_tab[gi];
-        u.kappa_begin = h->g_kappa_base[gi];
+    rg.tpc = h->nshards > 1 ? tpc_sys : tiles_per_chunk(e - i, C, h->lr_waves, h->nsm);
+    // a group's tiles are padded to whole quads (a structure-factor CTA's
+    // warps share one group's table)
+    const size_t first = i;
+    auto pad_quad = [&]() {
+      while ((tiles.size() - rg.u0) % dev::kSfWarps) {
+        dev::DirTile u = tiles.back();
+        u.n_dir = 0;
         tiles.push_back(u);
       }
-      i = e;
+    };
+    for (; i < e; i++) {
+      const uint32_t gi = all[i].gi;
+      if (i > first && gi != all[i - 1].gi) pad_quad();
+      dev::DirTile u{};
+      u.node_begin = all[i].k - kb;
+      u.dir_begin = h->g_dir_base[gi] + all[i].j;
+      u.n_dir = all[i].n;
+      u.n_rad = p.groups[gi].n_radial;
+      u.P = h->g_sf_P[gi];
+      u.tab = h->g_sf_tab[gi];
+      u.kappa_begin = h->g_kappa_base[gi];
+      u.lr_P = h->g_lr_P[gi];
+      u.lr_tab = h->g_lr_tab[gi];
+      tiles.push_back(u);
     }
-    rg.c1 = (uint32_t)chunks.size();
+    pad_quad();
     rg.u1 = (uint32_t)tiles.size();
-    if (rg.c1 - rg.c0 > 65535) return fail(GLST_ERR_SIZE, "too many long-range chunks in a node stage");
     h->stage_kmax = std::max(h->stage_kmax, rg.ke - rg.kb);
-    h->part_rows = std::max(h->part_rows, rg.c1 - rg.c0);
+    h->part_rows = std::max(h->part_rows, rg.rows());
     h->ranges.push_back(rg);
   }
   // rows a later stage writes beyond what stage 0 writes start at zero
-  h->part_zero_from = h->ranges.empty() ? h->part_rows : h->ranges[0].c1 - h->ranges[0].c0;
-  h->nsplit = (uint32_t)chunks.size();
+  h->part_zero_from = h->ranges.empty() ? h->part_rows : h->ranges[0].rows();
   h->n_tiles = (uint32_t)tiles.size();
   const size_t part_rows = h->part_rows;
   if (in_arena) {
-    // first build (set-up): carve the tables and partial rows out of the
+    // first build (set-up): carve the table and partial rows out of the
     // handle's single allocation; uploaded once it is committed.  Separate
     // small cudaMalloc calls here took 25-270 ms while a server's other
     // requests kept the GPU busy.
-    GLST_TRY(dalloc_n(h, &h->chunks, std::max<size_t>(1, chunks.size())));
     GLST_TRY(dalloc_n(h, &h->tiles, std::max<size_t>(1, tiles.size())));
     GLST_TRY(dalloc_n(h, &h->part, part_rows * std::max<size_t>(1, N)));
-    h->chunk_cap = std::max<size_t>(1, chunks.size());
     h->tile_cap = std::max<size_t>(1, tiles.size());
     h->part_cap = part_rows;
-    h->host_chunks = std::move(chunks);
     h->host_tiles = std::move(tiles);
     return GLST_OK;
   }
@@ -516,16 +471,12 @@ static glst_status build_chunks(glst_handle *h, bool in_arena = false) {
     h->bytes += need * elem;
     return GLST_OK;
   };
-  GLST_TRY(regrow(reinterpret_cast<void **>(&h->chunks), h->chunks_owned, h->chunk_cap,
-                  std::max<size_t>(1, chunks.size()), sizeof(dev::LrChunk)));
   GLST_TRY(regrow(reinterpret_cast<void **>(&h->tiles), h->tiles_owned, h->tile_cap,
                   std::max<size_t>(1, tiles.size()), sizeof(dev::DirTile)));
   size_t part_cap_elems = h->part_cap * std::max<size_t>(1, N);
   GLST_TRY(regrow(reinterpret_cast<void **>(&h->part), h->part_owned, part_cap_elems,
                   part_rows * std::max<size_t>(1, N), sizeof(double4)));
   h->part_cap = part_cap_elems / std::max<size_t>(1, N);
-  if (!chunks.empty())
-    CUDA_TRY(cudaMemcpy(h->chunks, chunks.data(), chunks.size() * sizeof(dev::LrChunk), cudaMemcpyHostToDevice));
   if (!tiles.empty())
     CUDA_TRY(cudaMemcpy(h->tiles, tiles.data(), tiles.size() * sizeof(dev::DirTile), cudaMemcpyHostToDevice));
   return GLST_OK;
@@ -542,7 +493,9 @@ static glst_status set_kernel_attributes(int device, size_t shell_smem) {
   int &d = done[device];
   if (!(d & 1)) {
     CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)dev::sf_smem_bytes(dev::kSfRadChunk)));
+                                  (int)dev::sf_smem_bytes(dev::kSfRadChunk, dev::kLrMaxRad * dev::kChebMaxP / 4)));
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)dev::lr_smem_bytes(dev::kSfRadChunk)));
     CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(dev::kSortCap * sizeof(uint32_t))));
     d |= 1;
@@ -598,7 +551,6 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   std::vector<uint32_t> radii(K);
   std::vector<float4> dirs;
   std::vector<float> kap;
-  std::vector<uint32_t> quad_base;  // per group, the first of its radial-scale quads
   // Chebyshev series of the phases on |u| <= U, U the radius of the cell's
   // circumscribed sphere and 2 % (atoms slightly outside the box stay within)
   // Coordinates are scaled by 1 / U in FP32, so U is the reciprocal of an
@@ -606,11 +558,13 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   const float cheb_inv = (float)(1.0 / (1.02 * 0.5 * std::sqrt(3.0) * p.cell_dim));
   const double cheb_u = 1.0 / (double)cheb_inv;
   h->cheb_scale = dev::ChebScale{cheb_inv, (float)(cheb_u * cheb_u)};
-  h->g_cheb_P.clear();
-  h->g_cheb_tab.clear();
+  h->g_sf_P.clear();
+  h->g_sf_tab.clear();
+  h->g_lr_P.clear();
+  h->g_lr_tab.clear();
   h->max_rad = 1;
+  h->sf_tab4 = 0;
   std::vector<float> cheb;
-  dev::LrKappaQuads kq{};
   uint32_t nquad = 0;
   {
     uint32_t ref_base = 0, ibase = 0;
@@ -619,28 +573,37 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
       kappa_base.push_back((uint32_t)kap.size());
       h->max_rad = std::max(h->max_rad, g.n_radial);
       {
-        const uint32_t P = glst::series_terms(*std::max_element(g.kappa.begin(), g.kappa.end()) * cheb_u, dev::kChebMaxP);
-        h->g_cheb_P.push_back(P);
-        h->g_cheb_tab.push_back((uint32_t)cheb.size());
-        std::vector<double> c(P);
-        for (unsigned r = 0; P && r < g.n_radial; r++) {
-          glst::phase_series(g.kappa[r] * cheb_u, P, c.data());
-          glst::product_basis(P, dev::cheb_b((int)P), c.data());
-          for (double v : c) cheb.push_back((float)v);
-          cheb.resize(cheb.size() + dev::cheb_row((int)P) - P, 0.f);
+        // series of the structure factors (product basis), then of the gather
+        std::vector<double> z, w, c;
+        for (unsigned r = 0; r < g.n_radial; r++) {
+          z.push_back(g.kappa[r] * cheb_u);
+          w.push_back(p.w[ref_base + (size_t)r * g.n_dir]);
+        }
+        const uint32_t sf_P = glst::series_terms(z, nullptr, dev::kChebMaxP);
+        const uint32_t lr_P = glst::series_terms(z, w.data(), dev::kChebMaxP);
+        h->g_sf_P.push_back(sf_P);
+        h->sf_tab4 = std::max<uint32_t>(h->sf_tab4, g.n_radial * (dev::cheb_row((int)sf_P) / 4));
+        h->g_sf_tab.push_back((uint32_t)cheb.size());
+        for (unsigned r = 0; sf_P && r < g.n_radial; r++) {
+          c.assign(dev::cheb_row((int)sf_P), 0.0);
+          glst::phase_series(z[r], sf_P, c.data());
+          glst::product_basis(sf_P, dev::cheb_b((int)sf_P), c.data());
+          cheb.insert(cheb.end(), c.begin(), c.end());
+        }
+        h->g_lr_P.push_back(lr_P);
+        h->g_lr_tab.push_back((uint32_t)cheb.size());
+        for (unsigned r = 0; lr_P && r < g.n_radial; r++) {
+          c.assign(dev::cheb_row((int)lr_P), 0.0);
+          glst::phase_series(z[r], lr_P, c.data());
+          cheb.insert(cheb.end(), c.begin(), c.end());
         }
       }
       dir_base.push_back((uint32_t)dirs.size());
       node_base.push_back(ibase);
       for (unsigned r = 0; r < g.n_radial; r++) kap.push_back((float)g.kappa[r]);
-      quad_base.push_back(nquad);
-      for (unsigned r0 = 0; r0 < g.n_radial; r0 += 4, nquad++) {
-        if (nquad >= (uint32_t)dev::kLrKappaQuads)
-          return fail(GLST_ERR_SIZE, "more than %d radial-scale quads", dev::kLrKappaQuads);
-        float v[4];
-        for (unsigned i = 0; i < 4; i++) v[i] = r0 + i < g.n_radial ? (float)g.kappa[r0 + i] : 0.f;
-        kq.q[nquad] = make_float4(v[0], v[1], v[2], v[3]);
-      }
+      nquad += (g.n_radial + 3) / 4;
+      if (nquad > dev::kLrMaxQuads)
+        return fail(GLST_ERR_SIZE, "more than %u radial-scale quads", dev::kLrMaxQuads);
       for (unsigned j = 0; j < g.n_dir; j++)
         dirs.push_back(make_float4((float)g.dirs[3 * j], (float)g.dirs[3 * j + 1], (float)g.dirs[3 * j + 2], 0.f));
       for (unsigned j = 0; j < g.n_dir; j++) {
@@ -657,7 +620,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
       }
       ref_base += g.n_radial * g.n_dir;
       ibase += g.n_radial * g.n_dir;
-      if (g.n_radial > (unsigned)dev::kLrfTileNodes)
+      if (g.n_radial > dev::kLrMaxRad)
         return fail(GLST_ERR_SIZE, "%u radial nodes exceed the tile of the long-range kernel", g.n_radial);
     }
     GLST_TRY(dalloc_n(h, &h->node64, K));
@@ -728,16 +691,13 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     h->g_node_base = node_base;
     h->g_dir_base = dir_base;
     h->g_kappa_base = kappa_base;
-    h->g_quad_base = quad_base;
-    h->kquads = kq;
     {
       const Tuning t = tuned(p, h->K);
       if (t.sat_nb && !h->gsat)
         h->sat_nb = pow2_floor(std::min<uint32_t>(t.sat_nb, (uint32_t)std::max<size_t>(1, budget / per_node)));
       if (t.lr_waves) h->lr_waves = t.lr_waves;
-      h->lr_variant = t.lr_variant;
     }
-    GLST_TRY(build_chunks(h, /*in_arena=*/true));
+    GLST_TRY(build_tiles(h, /*in_arena=*/true));
     const size_t kpad = ((size_t)h->stage_kmax + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
     GLST_TRY(dalloc_n(h, &h->S, C * kpad));
     GLST_TRY(dalloc_n(h, &h->R, C * kpad));
@@ -751,13 +711,10 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     }
   }
   GLST_TRY(commit_allocs(h));
-  if (!h->host_chunks.empty()) {
-    CUDA_TRY(cudaMemcpyAsync(h->chunks, h->host_chunks.data(), h->host_chunks.size() * sizeof(dev::LrChunk),
-                             cudaMemcpyHostToDevice, h->side));
+  if (!h->host_tiles.empty()) {
     CUDA_TRY(cudaMemcpyAsync(h->tiles, h->host_tiles.data(), h->host_tiles.size() * sizeof(dev::DirTile),
                              cudaMemcpyHostToDevice, h->side));
   }
-  h->host_chunks.clear();
   h->host_tiles.clear();
   if (K) {
     CUDA_TRY(cudaMemcpyAsync(h->node64, n64.data(), K * sizeof(double4), cudaMemcpyHostToDevice, h->side));
@@ -804,21 +761,22 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
 }
 
 // Far-field phases of one node stage: direction tiles [u0, u1),
-// shell sums over nodes [kb, ke), long-range chunks [c0, c1).  S and R hold
+// shell sums over nodes [kb, ke), the gather over the same tiles.  S and R hold
 // the stage's nodes (local index = node - rg.kb).
 static dev::SfArgs sf_args(const glst_handle *h, const glst_handle::FarRange &rg) {
   return dev::SfArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
                      reinterpret_cast<const float4 *>(h->cheb), h->S, h->R, h->cheb_scale, h->plan.ncell,
-                     rg.u1 - rg.u0, h->max_rad, rg.kb};
+                     rg.u1 - rg.u0, h->max_rad, rg.kb, h->sf_tab4};
 }
 
 static glst_status sf_stage(glst_handle *h, const glst_handle::FarRange &rg, cudaStream_t st) {
   if (rg.u1 <= rg.u0 || !h->plan.natom) return GLST_OK;
-  const uint32_t nt = rg.u1 - rg.u0, quads = (nt + dev::kSfWarps - 1) / dev::kSfWarps;
-  const uint32_t per_launch = 0x7fffffffu / quads;  // cells (gridDim.x is at most 2^31 - 1)
+  const uint32_t quads = (rg.u1 - rg.u0) / dev::kSfWarps;
+  const uint32_t per_launch = 0x7fffffffu / quads / dev::kSfCells * dev::kSfCells;  // cells (gridDim.x < 2^31)
   for (uint32_t c0 = 0; c0 < h->plan.ncell; c0 += per_launch) {
     const uint32_t nc = std::min(per_launch, h->plan.ncell - c0);
-    dev::k_structure_factors<<<quads * nc, dev::kSfThreads, dev::sf_smem_bytes(h->max_rad), st>>>(sf_args(h, rg), c0);
+    dev::k_structure_factors<<<quads * ((nc + dev::kSfCells - 1) / dev::kSfCells), dev::kSfThreads,
+                                dev::sf_smem_bytes(h->max_rad, h->sf_tab4), st>>>(sf_args(h, rg), c0);
     CUDA_TRY(cudaGetLastError());
   }
   return GLST_OK;
@@ -870,23 +828,20 @@ static glst_status shell_stage(glst_handle *h, const glst_handle::FarRange &rg, 
   return GLST_OK;
 }
 
+static dev::LrArgs lr_args(const glst_handle *h, size_t stage) {
+  const auto &rg = h->ranges[stage];
+  return dev::LrArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
+                     reinterpret_cast<const float4 *>(h->cheb), h->R, h->part, h->cheb_scale, h->plan.ncell,
+                     rg.u1 - rg.u0, rg.tpc, h->max_rad, rg.kb, h->plan.natom,
+                     stage > 0 ? 1 : 0};  // stage 0 writes its rows, later stages add into the same rows
+}
+
 static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
   const auto &rg = h->ranges[stage];
-  if (rg.c1 <= rg.c0 || !h->plan.natom) return GLST_OK;
-  dim3 grid((h->plan.natom + dev::kLrThreads - 1) / dev::kLrThreads, rg.c1 - rg.c0);
-  // stage 0 writes its rows, later stages add into the same rows
-#define GLST_LR(v)                                                                                            \
-  case v:                                                                                                     \
-    dev::k_long_range_flat<v><<<grid, dev::kLrThreads, 0, st>>>(h->pk, h->cell_point, h->plan.ncell,          \
-                                                                h->chunks + rg.c0, h->dirs, h->kappa, h->R,   \
-                                                                rg.kb, h->plan.natom, stage > 0 ? 1 : 0,      \
-                                                                h->part, h->kquads);                          \
-    break;
-  switch (h->lr_variant) {
-    GLST_LR(0) GLST_LR(1) GLST_LR(2) GLST_LR(3)
-    default: return fail(GLST_ERR_INVALID_ARG, "bad gather variant");
-  }
-#undef GLST_LR
+  if (rg.u1 <= rg.u0 || !h->plan.natom) return GLST_OK;
+  const uint64_t ctas = ((uint64_t)rg.rows() * h->plan.ncell + dev::kLrWarps - 1) / dev::kLrWarps;
+  if (ctas > 0x7fffffffu) return fail(GLST_ERR_SIZE, "too many cells for the gather's grid");
+  dev::k_long_range<<<(uint32_t)ctas, dev::kLrThreads, dev::lr_smem_bytes(h->max_rad), st>>>(lr_args(h, stage), rg.rows());
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }
@@ -1247,7 +1202,7 @@ glst_status glst_get_info(const glst_handle *h, glst_info *info) {
   info->kernels_per_compute = h->plan.natom ? 4u + (h->shard == 0 ? 1u : 0u) + far + 2u : 2u;
   info->node_stages = (uint32_t)h->ranges.size();
   info->shell_sums_form = h->gsat ? 1u : 0u;
-  info->gather_variant = h->lr_variant;
+  info->gather_variant = 0;
   info->sf_max_npt = 12;
   return GLST_OK;
 }
@@ -1328,27 +1283,17 @@ glst_status glst_autotune(glst_handle *h, const double *rx, const double *ry, co
     best = 1e30f;
     for (uint32_t w : {2u, 4u, 8u, 16u, 32u}) {
       h->lr_waves = w;
-      GLST_TRY(build_chunks(h));
+      GLST_TRY(build_tiles(h));
       float ms = 0.f;
       GLST_TRY(timed(phase_lr, &ms));
       if (ms < best) best = ms, best_w = w;
     }
     h->lr_waves = best_w;
-    GLST_TRY(build_chunks(h));
-    // long-range gather: FMA-pipe sine/cosine share (compiled variants)
-    uint32_t best_v = h->lr_variant;
-    best = 1e30f;
-    for (uint32_t v = 0; v < (uint32_t)dev::kLrVariants; v++) {
-      h->lr_variant = v;
-      float ms = 0.f;
-      GLST_TRY(timed(phase_lr, &ms));
-      if (ms < best) best = ms, best_v = v;
-    }
-    h->lr_variant = best_v;
+    GLST_TRY(build_tiles(h));
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[tune_key(h->plan, h->K)] = Tuning{h->sat_nb, h->lr_waves, h->lr_variant};
+    g_tune[tune_key(h->plan, h->K)] = Tuning{h->sat_nb, h->lr_waves};
   }
   if (sat_nb) *sat_nb = h->sat_nb;
   if (lr_waves) *lr_waves = h->lr_waves;
@@ -1557,7 +1502,7 @@ struct glst_batch {
   // of another).
   struct WlGroup {
     uint32_t ph_off[kPhases] = {}, ph_n[kPhases] = {}, ph_grid[kPhases] = {};
-    size_t shell_smem = 0, sf_smem = 0; // dynamic shared memory of the shell-sum and structure-factor launches
+    size_t shell_smem = 0, sf_smem = 0, lr_smem = 0;  // dynamic shared memory of the far-field launches
     cudaStream_t side = nullptr;        // near field beside the far field
     cudaEvent_t fork = nullptr, join = nullptr;
   };
@@ -1609,7 +1554,6 @@ static void batch_release(glst_batch *b) {
 // shell sums in shared memory with several nodes per CTA (or no far field).
 static bool worklist_ok(const glst_handle *h) {
   if (h->nshards != 1 || h->ranges.size() > 1 || h->gsat) return false;
-  if (h->lr_variant != 0) return false;  // the work-list gather is the default variant
   if (h->K && h->sat_nb < 2) return false;
   return true;
 }
@@ -1652,7 +1596,9 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
   CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device));
   CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device));
   CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)dev::sf_smem_bytes(dev::kSfRadChunk)));
+                                (int)dev::sf_smem_bytes(dev::kSfRadChunk, dev::kLrMaxRad * dev::kChebMaxP / 4)));
+  CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)dev::lr_smem_bytes(dev::kSfRadChunk)));
   CUDA_TRY(cudaFuncSetAttribute(dev::k_shell_sums_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin));
   CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(dev::kSortCap * sizeof(uint32_t))));
@@ -1681,9 +1627,9 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     });
     each(glst_batch::kSf, [&](uint32_t w, glst_handle *h) {
       if (!h->K || !h->plan.natom) return;
-      const uint32_t quads = (h->n_tiles + dev::kSfWarps - 1) / dev::kSfWarps;
-      gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad));
-      for (uint32_t c = 0; c < h->plan.ncell; c++)
+      const uint32_t quads = h->n_tiles / dev::kSfWarps;
+      gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad, h->sf_tab4));
+      for (uint32_t c = 0; c < h->plan.ncell; c += dev::kSfCells)
         for (uint32_t u = 0; u < quads; u++) items.push_back({w, u, c, 0});
     });
     each(glst_batch::kShell, [&](uint32_t w, glst_handle *h) {
@@ -1692,9 +1638,9 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     });
     each(glst_batch::kLr, [&](uint32_t w, glst_handle *h) {
       if (!h->K || !h->plan.natom) return;
-      const uint32_t ab = (h->plan.natom + dev::kLrThreads - 1) / dev::kLrThreads;
-      for (uint32_t c = 0; c < h->nsplit; c++)
-        for (uint32_t a = 0; a < ab; a++) items.push_back({w, a, c, 0});
+      gr.lr_smem = std::max(gr.lr_smem, dev::lr_smem_bytes(h->max_rad));
+      for (uint32_t r = 0; r < h->part_rows; r++)
+        for (uint32_t c = 0; c < h->plan.ncell; c += dev::kLrWarps) items.push_back({w, c, r, 0});
     });
     each(glst_batch::kSr, [&](uint32_t w, glst_handle *h) {
       if (!h->plan.natom) return;
@@ -1716,7 +1662,7 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     }
     auto grid = [&](int ph, const void *fn, int threads, size_t smem) -> glst_status {
       uint32_t g = gr.ph_n[ph];
-      if (persistent) {
+      if (persistent && ph != glst_batch::kSf) {
         int per_sm = 0;
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
         g = std::min<uint32_t>(g, (uint32_t)std::max(1, per_sm) * nsm);
@@ -1731,7 +1677,7 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     GLST_TRY(grid(glst_batch::kSort, (const void *)dev::k_sort_pack_multi, 256, dev::kSortCap * sizeof(uint32_t)));
     GLST_TRY(grid(glst_batch::kSf, (const void *)dev::k_structure_factors_multi, dev::kSfThreads, gr.sf_smem));
     GLST_TRY(grid(glst_batch::kShell, (const void *)dev::k_shell_sums_multi, dev::kSatThreads, gr.shell_smem));
-    GLST_TRY(grid(glst_batch::kLr, (const void *)dev::k_long_range_multi, dev::kLrThreads, 0));
+    GLST_TRY(grid(glst_batch::kLr, (const void *)dev::k_long_range_multi, dev::kLrThreads, gr.lr_smem));
     GLST_TRY(grid(glst_batch::kSr, (const void *)dev::k_short_range_multi, dev::kSrThreads, 0));
     GLST_TRY(grid(glst_batch::kCombine, (const void *)dev::k_combine_multi, dev::kCombineThreads, 0));
     GLST_TRY(grid(glst_batch::kEnergy, (const void *)dev::k_energy_multi, 256, 0));
@@ -1771,10 +1717,12 @@ static glst_status worklist_descriptors(glst_batch *b, const double *const in[4]
     d.rx = in[0] + o; d.ry = in[1] + o; d.rz = in[2] + o; d.qc = in[3] + o;
     d.atom_cell = h->atom_cell; d.atom_slot = h->atom_slot; d.perm = h->perm;
     d.sorted_idx = h->sorted_idx; d.cell_count = h->cell_count; d.cell_point = h->cell_point;
-    d.pk = h->pk; d.pd = h->pd; d.dirs = h->dirs; d.kappa = h->kappa;
-    d.chunks = h->chunks;
-    if (h->K && !h->ranges.empty()) d.sf = sf_args(h, h->ranges[0]);
-    d.S = h->S; d.R = h->R; d.part = h->part; d.sr = h->sr; d.sr_rows = h->sr_rows;
+    d.pk = h->pk; d.pd = h->pd;
+    if (h->K && !h->ranges.empty()) {
+      d.sf = sf_args(h, h->ranges[0]);
+      d.lr = lr_args(h, 0);
+    }
+    d.part = h->part; d.sr = h->sr; d.sr_rows = h->sr_rows;
     d.cfx = h->cfx; d.cfy = h->cfy; d.cfz = h->cfz; d.cen = h->cen;
     // input-order outputs straight into the batch's arrays (or the
     // handle's own when the caller passes none)
@@ -1811,7 +1759,7 @@ static glst_status worklist_launch(glst_batch *b, glst_batch::WlGroup &gr, cudaS
   GLST_TRY(go(glst_batch::kSr, dev::k_short_range_multi, dev::kSrThreads, 0, gr.side));
   CUDA_TRY(cudaEventRecord(gr.join, gr.side));
   GLST_TRY(go(glst_batch::kShell, dev::k_shell_sums_multi, dev::kSatThreads, gr.shell_smem, st));
-  GLST_TRY(go(glst_batch::kLr, dev::k_long_range_multi, dev::kLrThreads, 0, st));
+  GLST_TRY(go(glst_batch::kLr, dev::k_long_range_multi, dev::kLrThreads, gr.lr_smem, st));
   CUDA_TRY(cudaStreamWaitEvent(st, gr.join, 0));
   GLST_TRY(go(glst_batch::kCombine, dev::k_combine_multi, dev::kCombineThreads, 0, st));
   GLST_TRY(go(glst_batch::kEnergy, dev::k_energy_multi, 256, 0, st));
@@ -2080,21 +2028,26 @@ uint64_t estimate_bytes(const Plan &p, int nsm) {
   const uint64_t N = p.natom, C = p.ncell, K = p.has_far ? p.K() : 0;
   uint64_t b = N * (4 * 4 + 16 + 32 + 32 * (uint64_t)sr_rows_for(C, nsm) + 8 * 8 + 32) + C * 8 + 4096;
   if (K) {
-    const uint64_t slots = (uint64_t)nsm * 16;
     const uint64_t kpad = (K + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
     const uint64_t nst = std::max<uint64_t>(1, (C * kpad * 16 + stage_budget() - 1) / stage_budget());
-    // the largest stage: ~K / stages, plus up to one structure-factor unit of
-    // directions (stages end on unit boundaries)
+    // the largest stage: ~K / stages, plus up to one tile of directions
+    // (stages end on tile boundaries)
     uint32_t max_nr = 1;
     for (const auto &g : p.groups) max_nr = std::max(max_nr, g.n_radial);
     const uint64_t stage_k =
-        nst == 1 ? kpad : std::min<uint64_t>(kpad, (K + nst - 1) / nst + (uint64_t)dev::kSfThreads * max_nr);
-    // gather chunks of a stage (partial rows): enough to fill the GPU, at
-    // most kMaxChunkNodes nodes each, one more per group boundary
-    const uint64_t chunks = std::max<uint64_t>((8 * slots + C - 1) / C, stage_k / kMaxChunkNodes + 1) +
-                            p.groups.size() + 1;
+        nst == 1 ? kpad : std::min<uint64_t>(kpad, (K + nst - 1) / nst + 32ull * max_nr);
+    // direction tiles (a stage holds no more than all), and a stage's gather
+    // chunks (partial rows)
+    uint64_t n_tiles = 0;
+    for (const auto &g : p.groups) n_tiles += (g.n_dir + 127) / 128 * 4;
+    uint64_t chunks = 1;
+    for (uint64_t t = std::max<uint64_t>(1, n_tiles / nst); t <= n_tiles / nst + 8; t++) {
+      const uint64_t tpc = tiles_per_chunk(t, C, kLrWaves, nsm);
+      chunks = std::max(chunks, (t + tpc - 1) / tpc + 1);
+    }
     const uint64_t stage_kpad = (stage_k + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
-    b += K * (32 + 4 + 16 + 4) + (uint64_t)max_nr * p.groups.size() * dev::kChebMaxP * 4 + C * stage_kpad * (8 + 8) + chunks * N * 32;
+    b += K * (32 + 4 + 16 + 4) + (uint64_t)max_nr * p.groups.size() * dev::kChebMaxP * 8 +
+         (n_tiles + 8 * nst) * sizeof(dev::DirTile) + C * stage_kpad * (8 + 8) + chunks * N * 32;
     // global-memory shell-sum tables (grids whose per-node table exceeds the
     // shared memory of a CTA): 64 MB or one block, and the twiddles
     if ((C + 9 + p.n[0] + p.n[1] + p.n[2]) * 16 > (200ull << 10))

@@ -288,29 +288,9 @@ __device__ __forceinline__ void fma_sincos_signed(float th, float q, float *s, f
   *qs = __int_as_float(__float_as_int(q) ^ (__float_as_int(t) << 31));
 }
 
-// The same polynomial on two angles at once with the paired FP32
-// instructions of sm_100 (FFMA2/FMUL2/FADD2: two IEEE FP32 operations per
-// instruction, each lane bit-identical to the scalar form above).
+// Operand pairs of the paired FP32 instructions (FFMA2/FADD2: two IEEE FP32
+// operations per instruction).
 __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
-
-__device__ __forceinline__ void fma_sincos_signed2(float2 th, float q, float2 *s, float2 *c, float2 *qs) {
-  const float2 t = __ffma2_rn(th, bcast(kInvPi), bcast(kRoundMagic));
-  const float2 n = __fadd2_rn(t, bcast(-kRoundMagic));
-  float2 r = __ffma2_rn(n, bcast(-kPiHi), th);
-  r = __ffma2_rn(n, bcast(-kPiLo), r);
-  const float2 r2 = __fmul2_rn(r, r);
-  float2 p = __ffma2_rn(bcast(kSin4), r2, bcast(kSin3));
-  p = __ffma2_rn(p, r2, bcast(kSin2));
-  p = __ffma2_rn(p, r2, bcast(kSin1));
-  *s = __ffma2_rn(__fmul2_rn(p, r2), r, r);
-  float2 cc = __ffma2_rn(bcast(kCos4), r2, bcast(kCos3));
-  cc = __ffma2_rn(cc, r2, bcast(kCos2));
-  cc = __ffma2_rn(cc, r2, bcast(kCos1));
-  *c = __ffma2_rn(cc, r2, bcast(kCos0));
-  const int qi = __float_as_int(q);
-  *qs = make_float2(__int_as_float(qi ^ (__float_as_int(t.x) << 31)),
-                    __int_as_float(qi ^ (__float_as_int(t.y) << 31)));
-}
 
 // ----------------------------------------------------------------------------
 // Structure factors.  S_c(k) = sum_{j in c} q_j e^{-i k.r_j}
@@ -333,26 +313,30 @@ __device__ __forceinline__ void fma_sincos_signed2(float2 th, float q, float2 *s
 // b the imaginary part, and a pair (b, b + 1) is one FFMA2 both when it is
 // accumulated and when it is multiplied out.
 //
-// One warp per (32 directions, cell), lane = direction, moments in
-// registers, atoms broadcast from shared memory: no CTA barriers, and groups
-// of few directions waste lanes of one warp only.  FP32 over a tile of <=
+// A CTA's four warps take 32 directions of one group each, lane = direction,
+// moments in registers, atoms broadcast from shared memory, for kSfCells
+// cells; the group's table is copied to shared memory once (read through L1
+// as broadcasts it took five wavefronts per 16 bytes, and half of L1's time).
+// After that the warps are independent.  FP32 over a tile of <=
 // kSfAtomTile atoms, then FP64 over the tiles of a denser cell.  S is stored
 // cell-relative in FP32; its twiddle e^{-ik.c} is applied by the shell sums
 // as they load S.  Atoms beyond U (outside the box by more than the margin,
 // or not a number) and tiles of too few atoms for the product (16 atoms cost
 // as much as P terms) take one sine and cosine per node instead.
-// Measured: water10k 1.112 -> 0.341 ms, 1,000 waters on 4^3 cells 0.144 ->
+// Measured: water10k 1.112 -> 0.297 ms, 1,000 waters on 4^3 cells 0.144 ->
 // 0.056 ms, 168 atoms per cell 0.313 -> 0.094 ms; forces 3.3e-8 -> 1.5e-8 off
 // the FP64 path.
 constexpr int kSfWarps = 4;
 constexpr int kSfThreads = 32 * kSfWarps;
 constexpr int kSfAtomTile = 128;
+constexpr int kSfCells = 1;       // cells per CTA (4: 5 % slower on water10k, 40 % on 1,000 waters)
 constexpr int kSfRadChunk = 64;   // radial nodes staged at a time, at most
 constexpr int kChebMaxP = 64;     // series terms, at most (even to 48, then multiples of 4)
 __host__ __device__ constexpr int cheb_b(int P) { return P > 24 ? 8 : 4; }
 __host__ __device__ constexpr int cheb_row(int P) { return (P + 3) / 4 * 4; }  // table row, in floats
 
-// Up to 32 directions of one group.
+// Up to 32 directions of one group (none: padding, so that a group's tiles are
+// whole quads).
 struct DirTile {
   uint32_t node_begin;   // local internal index of (first direction, r = 0)
   uint32_t dir_begin;    // global direction index of the first direction
@@ -361,7 +345,7 @@ struct DirTile {
   uint32_t P;            // series terms, even (0: one sincos per node)
   uint32_t tab;          // offset of the group's n_rad x cheb_row(P) table
   uint32_t kappa_begin;  // offset of this group's radial table
-  uint32_t pad;
+  uint32_t lr_P, lr_tab; // the gather's series terms and table
 };
 
 // Per-handle constants of the series: 1 / U and the largest |d|^2 it takes.
@@ -382,14 +366,15 @@ struct SfArgs {
   float2 *S, *lo_buf;  // lo_buf: scratch of S's size
   ChebScale cs;
   uint32_t ncell, n_tiles, max_rad, node_off;
+  uint32_t tab4;       // float4s of the largest group's table
 };
 
 // Rows of the staged results are an odd number of float2 apart (bank spread).
 __host__ __device__ constexpr uint32_t sf_row(uint32_t rc) { return rc | 1u; }
 
-__host__ __device__ inline size_t sf_smem_bytes(uint32_t max_rad) {
+__host__ __device__ inline size_t sf_smem_bytes(uint32_t max_rad, uint32_t tab4) {
   const uint32_t rc = max_rad < (uint32_t)kSfRadChunk ? max_rad : (uint32_t)kSfRadChunk;
-  return (size_t)kSfWarps * (32 * sizeof(float4) + 32 * sf_row(rc) * sizeof(float2));
+  return tab4 * sizeof(float4) + (size_t)kSfWarps * (32 * sizeof(float4) + 32 * sf_row(rc) * sizeof(float2));
 }
 
 // The general form, one sine and cosine per (atom, node), added to the staged
@@ -445,9 +430,12 @@ __device__ __forceinline__ void sf_moments(const float4 *__restrict__ pk, uint32
 #pragma unroll
   for (int m = 0; m < P / 2; m++) N[m] = make_float2(0.f, 0.f);
   double charge = 0.0;
+  float4 ahead = lane < na ? pk[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t b0 = 0; b0 < na; b0 += 32) {
     const uint32_t nb = min(32u, na - b0);
-    float4 p = lane < nb ? pk[b0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 p = ahead;
+    if (b0 + 32 + lane < na) ahead = pk[b0 + 32 + lane];
+    else ahead = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool in = fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z)) <= cs.u2;
     beyond |= __any_sync(0xffffffffu, !in) != 0;
     p = in ? make_float4(p.x * cs.inv_u, p.y * cs.inv_u, p.z * cs.inv_u, p.w) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -455,7 +443,7 @@ __device__ __forceinline__ void sf_moments(const float4 *__restrict__ pk, uint32
     __syncwarp();
     s_at[lane] = p;
     __syncwarp();
-#pragma unroll 2
+#pragma unroll 4
     for (uint32_t j = 0; j < nb; j++) {
       const float4 a = s_at[j];
       const float x = fmaf(s.x, a.x, fmaf(s.y, a.y, s.z * a.z));
@@ -486,11 +474,10 @@ __device__ __forceinline__ void sf_moments(const float4 *__restrict__ pk, uint32
 
 template <int P>
 __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const float4 *__restrict__ pk, uint32_t cnt,
-                                        uint32_t cell, float4 *s_at, float2 *s_f) {
+                                        uint32_t cell, const float4 *rows, float4 *s_at, float2 *s_f) {
   const uint32_t lane = threadIdx.x & 31u;
   const float4 s = lane < u.n_dir ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t node0 = u.node_begin - a.node_off;
-  const float4 *rows = a.tab + u.tab / 4;
   uint32_t a0 = 0;
   do {
     const uint32_t na = min((uint32_t)kSfAtomTile, cnt - a0);
@@ -514,7 +501,7 @@ __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const
             float2 f0 = make_float2(0.f, 0.f), f1 = make_float2(0.f, 0.f);
 #pragma unroll
             for (int m = 0; m < cheb_row(P) / 4; m++) {
-              const float4 c = __ldg(t + m);
+              const float4 c = t[m];
               f0 = __ffma2_rn(N[2 * m], make_float2(c.x, c.y), f0);
               if (2 * m + 1 < P / 2) f1 = __ffma2_rn(N[2 * m + 1], make_float2(c.z, c.w), f1);
             }
@@ -556,20 +543,25 @@ __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const
   } while (a0 < cnt);
 }
 
-// Work item: kSfWarps consecutive tiles and a cell; warps are independent.
-__device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_t cell) {
+// Work item: kSfWarps consecutive tiles (of one group) and kSfCells cells
+// from `cell0` on.
+__device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_t cell0) {
   extern __shared__ float4 s_sf[];
   const uint32_t warp = threadIdx.x >> 5;
-  const uint32_t ti = quad * kSfWarps + warp;
-  if (ti >= a.n_tiles) return;
+  const DirTile u = a.tiles[quad * kSfWarps + warp];  // (a group's tiles are padded to whole quads)
+  const uint32_t tab4 = u.n_rad * (uint32_t)(cheb_row((int)u.P) / 4);
+  for (uint32_t i = threadIdx.x; i < tab4; i += kSfThreads) s_sf[i] = a.tab[u.tab / 4 + i];
+  __syncthreads();
+  if (u.n_dir == 0) return;
   const uint32_t rc = min(a.max_rad, (uint32_t)kSfRadChunk);
-  float4 *s_at = s_sf + warp * 32;
-  float2 *s_f = reinterpret_cast<float2 *>(s_sf + kSfWarps * 32) + (size_t)warp * 32 * sf_row(rc);
-  const DirTile u = a.tiles[ti];
-  const uint32_t cnt = a.cell_count[cell];
-  const float4 *atoms = a.pk + a.cell_point[cell];
-#define GLST_SF_CASE(n) \
-  case n: sf_tile<n>(a, u, atoms, cnt, cell, s_at, s_f); break;
+  float4 *s_at = s_sf + a.tab4 + warp * 32;
+  float2 *s_f = reinterpret_cast<float2 *>(s_sf + a.tab4 + kSfWarps * 32) + (size_t)warp * 32 * sf_row(rc);
+  const uint32_t cell1 = min(a.ncell, cell0 + kSfCells);
+#define GLST_SF_CASE(n)                                                                            \
+  case n:                                                                                          \
+    for (uint32_t cell = cell0; cell < cell1; cell++)                                              \
+      sf_tile<n>(a, u, a.pk + a.cell_point[cell], a.cell_count[cell], cell, s_sf, s_at, s_f);      \
+    break;
   switch (u.P) {
     GLST_SF_CASE(0) GLST_SF_CASE(4) GLST_SF_CASE(6) GLST_SF_CASE(8) GLST_SF_CASE(10)
     GLST_SF_CASE(12) GLST_SF_CASE(14) GLST_SF_CASE(16) GLST_SF_CASE(18) GLST_SF_CASE(20)
@@ -584,9 +576,9 @@ __device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_
 
 __global__ void __launch_bounds__(kSfThreads, 4)
 k_structure_factors(const __grid_constant__ SfArgs a, uint32_t cell_base) {
-  const uint32_t quads = (a.n_tiles + kSfWarps - 1) / kSfWarps;
+  const uint32_t quads = a.n_tiles / kSfWarps;
   const uint32_t c = blockIdx.x / quads;
-  sf_block(a, blockIdx.x - c * quads, cell_base + c);
+  sf_block(a, blockIdx.x - c * quads, cell_base + c * kSfCells);
 }
 
 // ----------------------------------------------------------------------------
@@ -977,292 +969,330 @@ __global__ void k_gsat_shell(Grid g, GsatArgs a) {
 
 // ----------------------------------------------------------------------------
 // Long-range gather (src/glst_force.cu:983-1135 restated):
-//   en_i = q_i Re sum_k e^{ik.d_i} R'_c(k),   f_i = q_i sum_k Im(...) k
-// Nodes are held in the order group -> direction -> radial, k = kappa_r s_j,
-// so per atom and direction u = s_j . d_i is formed once and each node costs
-// one multiply, one SFU sin/cos pair and four FMAs:
-//   e += c R'x - s R'y,   g += kappa_r (c R'y + s R'x),   f += g s_j.
-// FP32 inside a tile, FP64 across tiles.
-constexpr int kLrThreads = 128;
-
-struct LrChunk {
-  uint32_t node_begin;   // internal index of (first direction, r = 0)
-  uint32_t dir_begin;    // global direction index of the first direction
-  uint32_t n_dir;        // directions in the chunk
-  uint32_t n_rad;        // radial nodes per direction in this group
-  uint32_t kappa_begin;  // offset of this group's radial table
-  uint32_t pad[3];
-};
-
-// A CTA takes 128 consecutive cell-ordered atoms whatever their cells (so
-// every warp is full -- one CTA per cell left ~10-15 % of the lanes of last
-// warps idle, measured 2.06 vs 1.63 ms on water10k), and stages the R' tiles
-// of the up to kLrfCells cells those atoms belong to; lanes read their own
-// cell's tile.  Atoms of sparser ranges (more cells) are handled in several
-// passes over windows of kLrfCells cells.
+//   en_i = q_i Re sum_k e^{ik.d_i} R'_c(k),   f_i = q_i sum_k Im(...) k.
+// Per direction s_j the sum over its radial nodes is a function of u = s_j.d_i
+// alone, and with the series of the structure factors a short one:
+//   e(x) = Re sum_r e^{i kappa_r U x} R'_r = sum_p c_p T_p(x),   x = u / U,
+//   c_p = sum_r (2 - [p = 0]) Re(i^p R'_r) J_p(kappa_r U),
+//   sum_r kappa_r Im(e^{i kappa_r u} R'_r) = -e'(x) / U.
+// The weights in R' (a Gaussian in kappa) let fewer terms do than the
+// structure factors need: P = 30, 18 and 14 in water10k's groups.  So a
+// (cell, direction) takes one n_rad x P product, and an (atom, direction) two
+// short series instead of a sine, a cosine and six FMAs per node (water10k
+// 1.40 ms, at the SFU's bound).
 //
-// Radial nodes go in pairs (r, r+1) -- a direction with an odd count gets a
-// zero node -- stored as float4 (R'x_r, R'x_r+1, R'y_r, R'y_r+1) so that the
-// paired FP32 instructions (FMUL2/FFMA2) do two nodes at once:
-//   EA += c R'x,  EB += s R'y,  G += kappa (c R'y + s R'x),   e = EA - EB.
-// One pair in kLrPolyStride takes its sine and cosine from the FMA-pipe
-// polynomial, interleaved with the SFU pairs of its group (the FMA pipe
-// already carries ~7 FP32 operations per node, so only a small share pays):
-// water10k 1.57 ms with none, 1.51 ms with 1 in 7, 1.53 with 1 in 5, 1.66
-// with 1 in 3; a separate polynomial loop after the SFU loop (20-40 %)
-// measured 1.63-1.87 ms.  The radial scales load as float4 quads (two
-// pairs), so groups are even: 14 pairs with 2 on the polynomial, 1.462 ms
-// against 1.482 ms with one scale load per pair (groups of 6 / 8 / 12 / 16
-// pairs with 1 / 1 / 2 / 2 on the polynomial: 1.503 / 1.483 / 1.476 / 1.498).
-// The cell slots of a tile are kLrfSlotPad float4 apart beyond the tile so
-// that the up to four addresses a warp reads fall in different shared-memory
-// banks (32.9 M bank conflicts per launch without the pad, 0.25 M with).
-// Two adjacent atoms per thread (256 atoms per CTA, one R' load serving both
-// when they share a cell: 0.75 shared loads per (atom, node pair) instead of
-// 1.5) gave bitwise-equal results but ran 14 % slower (water10k 1.67 vs
-// 1.465 ms; 96 registers, 5 CTAs per SM): the MUFU latency the 32 resident
-// warps hide outweighs the MIO-queue relief.  Staging the tiles with
-// asynchronous copies (cp.async, no prefetch registers: 64 registers without
-// spills) was bitwise-equal and slower too: 1.570 ms at 8 CTAs per SM, 1.584
-// at 9, 1.599 at 10 -- the copies add to the MIO queue, and more resident
-// warps do not help a gather bound by that queue.  Reading each lane's R'
-// pair straight from global memory (two L1-cached loads per node pair, no
-// staging, barriers or window passes) was bitwise-equal and far slower:
-// 2.75 against 1.44 ms.
-constexpr int kLrfCells = 4;           // cells staged per pass
-constexpr int kLrfTilePairs = 128;     // node pairs per cell tile
-constexpr int kLrfTileNodes = 2 * kLrfTilePairs;
-constexpr int kLrfSlotPad = 2;
-constexpr int kLrfSlot = kLrfTilePairs + kLrfSlotPad;
-constexpr int kLrfPerThread = (kLrfCells * kLrfTilePairs) / kLrThreads;
-constexpr int kLrGroup = 14;      // node pairs per group (even: radial scales load as quads)
-static_assert(kLrGroup % 2 == 0, "groups are whole radial-scale quads");
-// Which pairs of a group take the FMA-pipe polynomial: bit q of the mask.
-// The variants are compiled in and chosen per plan by the autotuner
-// (glst_autotune); variant 0, three pairs in fourteen at 1, 5, 10, is the
-// default.  With the radial scales in the parameter space (a lighter MIO
-// queue) three pairs beat two: water10k 1.397 ms at {1, 5, 10}, 1.406 at
-// {0, 5, 10}, against 1.436 at {6, 13} (the earlier default); {2, 7, 12}
-// 1.407, {4, 9, 13} 1.410, {0, 4, 9} 1.409, {1, 6, 11} 1.419, {0, 7} 1.420,
-// four pairs {2, 6, 10, 13} 1.429, {0, 4, 8, 12} 1.428.
-constexpr uint32_t kLrPolyMasks[4] = {(1u << 1) | (1u << 5) | (1u << 10), 0u, (1u << 6) | (1u << 13),
-                                      (1u << 1) | (1u << 5) | (1u << 9) | (1u << 13)};
-constexpr int kLrVariants = 4;
+// Lane = direction, atoms broadcast from shared memory: both series'
+// coefficients stay in registers as (e, e') pairs for paired FP32
+// instructions, and the inner loop loads nothing but the atom.  In the
+// product basis T_{Bg} T_b the inner sums over b need B - 1 Chebyshev values
+// and the outer sum over g another P / B.  The 32 directions are then summed
+// across the warp for eight atoms at a time: 31 shuffles leave one of the 8 x
+// 4 sums in each lane.  FP32 over the 32 directions, FP64 across direction
+// tiles and warps.  Atoms beyond the series' range and tiles of too few atoms
+// for the product take a sine and cosine per node (lr_direct).
+//
+// Warps are independent: each takes a cell and a chunk of direction tiles,
+// with no CTA barriers (four warps on one cell's chunk waited for each other
+// a third of the time).  A tile's R' is copied to shared memory
+// asynchronously while the previous tile's series are evaluated -- the buffer
+// is free once its coefficients are formed.
+// Measured: water10k 1.458 -> 0.485 ms, 3,000 atoms on 4^3 cells 0.141 ->
+// 0.076 ms, 168 atoms per cell 0.279 -> 0.148 ms, a million atoms 55 -> 17 ms;
+// forces 1.5e-8 -> 0.9e-8 off the FP64 path.
+constexpr int kLrWarps = 4;
+constexpr int kLrThreads = 32 * kLrWarps;
+constexpr int kLrAtomTile = 128;
+constexpr int kLrBatch = 8;       // atoms reduced across the warp together
+constexpr uint32_t kLrMaxRad = 256;    // radial nodes per direction, at most (set-up checks)
+constexpr uint32_t kLrMaxQuads = 128;  // radial nodes of all groups, in fours, at most (set-up checks)
 
-__device__ __forceinline__ uint32_t cell_of_atom(const uint32_t *__restrict__ cell_point, uint32_t ncell,
-                                                 uint32_t p) {
-  // last cell whose first atom is <= p (cells may be empty: the last such)
-  uint32_t lo = 0, hi = ncell - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (cell_point[mid] <= p) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-// The radial scales of every group as quads (kappa_4t .. kappa_4t+3 of a
-// group, 0 beyond its last), passed in the gather's parameter space; a
-// chunk's quads start at quad_begin.
-constexpr int kLrKappaQuads = 128;
-struct LrKappaQuads {
-  float4 q[kLrKappaQuads];
+struct LrArgs {
+  const float4 *pk;
+  const uint32_t *cell_count, *cell_point;
+  const DirTile *tiles;
+  const float4 *dirs;
+  const float *kappa;
+  const float4 *tab;   // Chebyshev series, cheb_row(P) floats per radial node
+  const float2 *R;
+  double4 *part;       // one row of natom per chunk of tiles
+  ChebScale cs;
+  uint32_t ncell, n_tiles, tiles_per_chunk, max_rad, node_off, natom;
+  int accumulate;      // a later node stage adds into the same rows
 };
 
-template <uint32_t kPolyMask, bool kParamKappa>
-__device__ __forceinline__ void lr_block(const float4 *__restrict__ pk, const uint32_t *__restrict__ cell_point,
-                                         uint32_t ncell, const LrChunk *__restrict__ chunks,
-                                         const float4 *__restrict__ dirs, const float *__restrict__ kappa,
-                                         const float2 *__restrict__ R, uint32_t node_off, uint32_t natom,
-                                         int accumulate, double4 *__restrict__ part, uint32_t bx, uint32_t by,
-                                         const LrKappaQuads *kpq = nullptr) {
-  __shared__ float4 s_n[2][kLrfCells * kLrfSlot];
-  __shared__ float4 s_kappa4[kParamKappa ? 1 : kLrfTilePairs / 2];
-  __shared__ uint32_t s_cells[kLrThreads];  // each thread's cell, then the distinct cells in order
-  __shared__ uint32_t s_heads[kLrThreads / 32];
-  const uint32_t a0 = bx * kLrThreads;
-  const uint32_t p = a0 + threadIdx.x;
-  const bool active = p < natom;
-  const LrChunk ch = chunks[by];
-  const uint32_t nr = ch.n_rad;
-  const uint32_t npr = (nr + 1) >> 1;                                   // pairs per direction
-  const uint32_t dirs_per_tile = max(1u, (uint32_t)kLrfTilePairs / npr);  // npr <= kLrfTilePairs (host check)
-  const uint32_t ntiles = (ch.n_dir + dirs_per_tile - 1) / dirs_per_tile;
-  // radial scales of pairs (2t, 2t+1): kappa_{4t .. 4t+3}, 0 beyond the last
-  if constexpr (!kParamKappa) {
-    for (uint32_t t = threadIdx.x; 2 * t < npr; t += kLrThreads) {
-      float kq[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) kq[i] = 4 * t + i < nr ? kappa[ch.kappa_begin + 4 * t + i] : 0.f;
-      s_kappa4[t] = make_float4(kq[0], kq[1], kq[2], kq[3]);
+__host__ __device__ inline size_t lr_smem_bytes(uint32_t max_rad) {
+  const uint32_t rc = max_rad < (uint32_t)kSfRadChunk ? max_rad : (uint32_t)kSfRadChunk;
+  return (size_t)kLrWarps * (kLrAtomTile * (sizeof(float4) + 4 * sizeof(double)) + 32 * sf_row(rc) * sizeof(float2));
+}
+
+// The general form for a warp's 32 directions: the tile's atoms beyond the
+// series' range (all: every atom), one sine and cosine per (atom, node).
+__device__ __noinline__ void lr_direct(const LrArgs &a, const DirTile &u, const float4 *__restrict__ atoms,
+                                       uint32_t na, bool all, uint32_t cell, double *__restrict__ acc) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool act = lane < u.n_dir;
+  const float4 s = act ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t node0 = u.node_begin - a.node_off + (act ? lane : 0) * u.n_rad;
+  for (uint32_t j = 0; j < na; j++) {
+    const float4 p = atoms[j];
+    if (!all && fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z)) <= a.cs.u2) continue;
+    const float x = fmaf(s.x, p.x, fmaf(s.y, p.y, s.z * p.z));
+    float e = 0.f, g = 0.f;
+    for (uint32_t r = 0; r < u.n_rad; r++) {
+      const float kap = a.kappa[u.kappa_begin + r];
+      const float2 v = a.R[sr_index(cell, node0 + r, a.ncell)];
+      float sn, cs, sg;
+      fma_sincos_signed(kap * x, 1.0f, &sn, &cs, &sg);
+      e = fmaf(sg, fmaf(cs, v.x, -sn * v.y), e);
+      g = fmaf(kap * sg, fmaf(cs, v.y, sn * v.x), g);
     }
-  }
-  const float4 *kq4 = kParamKappa ? kpq->q + ch.pad[0] : s_kappa4;
-  // The distinct cells of the CTA's atoms, in order, and each atom's rank
-  // among them: windows of kLrfCells occupied cells.  (Windows of
-  // consecutive cell indices made blocks that span empty and sparse cells --
-  // the reference's grid of rcut-edged cells leaves the outer layer nearly
-  // empty when the box is a little over a multiple of rcut -- take up to six
-  // passes over every node tile with most warps idle: 13,500 atoms on 6^3
-  // cells, 14 of them empty, 0.834 ms against 0.853 ms for 18,000 atoms.)
-  const uint32_t my_cell = active ? cell_of_atom(cell_point, ncell, p) : 0xffffffffu;
-  const float4 pa = active ? pk[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-  s_cells[threadIdx.x] = my_cell;
-  __syncthreads();
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const bool head = active && (threadIdx.x == 0 || s_cells[threadIdx.x - 1] != my_cell);
-  const uint32_t hmask = __ballot_sync(0xffffffffu, head);
-  if (lane == 0) s_heads[warp] = __popc(hmask);
-  __syncthreads();  // every thread has read its predecessor's cell
-  uint32_t before = 0, ncells = 0;
+    if (!act) e = g = 0.f;
+    float f[4] = {e, g * s.x, g * s.y, g * s.z};
 #pragma unroll
-  for (int w = 0; w < kLrThreads / 32; w++) {
-    const uint32_t h = s_heads[w];
-    before += (w < (int)warp) ? h : 0u;
-    ncells += h;
-  }
-  // rank = heads at or before this thread, less one (active threads only)
-  const uint32_t rank = before + __popc(hmask & (0xffffffffu >> (31u - lane))) - 1u;
-  if (head) s_cells[rank] = my_cell;
-  __syncthreads();
-  double ex = 0.0, ey = 0.0, ez = 0.0, ee = 0.0;
-  for (uint32_t w0 = 0; w0 < ncells; w0 += kLrfCells) {
-    const uint32_t nc = min((uint32_t)kLrfCells, ncells - w0);
-    const bool mine = active && rank >= w0 && rank < w0 + nc;
-    const uint32_t slot = mine ? rank - w0 : 0;
-    const bool warp_live = __any_sync(0xffffffffu, mine);
-    float4 pre[kLrfPerThread];
-    // prefetch one tile of every cell of this window into registers
-    auto prefetch = [&](uint32_t d0) {
-      const uint32_t nd = min(dirs_per_tile, ch.n_dir - d0);
-#pragma unroll
-      for (int k = 0; k < kLrfPerThread; k++) {
-        const uint32_t t = threadIdx.x + k * kLrThreads;
-        const uint32_t c = t / kLrfTilePairs, i = t % kLrfTilePairs;
-        const uint32_t dd = i / npr, r = 2 * (i - dd * npr);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < nc && dd < nd) {
-          const uint32_t node = ch.node_begin + (d0 + dd) * nr + r - node_off;
-          const uint32_t cell = s_cells[w0 + c];
-          const float2 x0 = R[sr_index(cell, node, ncell)];
-          const float2 x1 = (r + 1 < nr) ? R[sr_index(cell, node + 1, ncell)] : make_float2(0.f, 0.f);
-          v = make_float4(x0.x, x1.x, x0.y, x1.y);
-        }
-        pre[k] = v;
-      }
-    };
-    __syncthreads();  // previous window done with s_n
-    prefetch(0);
-    for (uint32_t tile = 0; tile < ntiles; tile++) {
-      const uint32_t d0 = tile * dirs_per_tile;
-      const uint32_t nd = min(dirs_per_tile, ch.n_dir - d0);
-      float4 *buf = s_n[tile & 1];
-#pragma unroll
-      for (int k = 0; k < kLrfPerThread; k++) {
-        const uint32_t t = threadIdx.x + k * kLrThreads;
-        buf[(t / kLrfTilePairs) * kLrfSlot + t % kLrfTilePairs] = pre[k];
-      }
-      __syncthreads();
-      if (tile + 1 < ntiles) prefetch(d0 + dirs_per_tile);
-      if (warp_live) {
-        float tx = 0.f, ty = 0.f, tz = 0.f, te = 0.f;
-        const float4 *cb = buf + slot * kLrfSlot;
-        for (uint32_t d = 0; d < nd; d++) {
-          const float4 sj = dirs[ch.dir_begin + d0 + d];
-          const float u = fmaf(sj.x, pa.x, fmaf(sj.y, pa.y, sj.z * pa.z));
-          const float2 u2 = bcast(u);
-          float2 EA = make_float2(0.f, 0.f), EB = make_float2(0.f, 0.f), G = make_float2(0.f, 0.f);
-          const float4 *nn = cb + d * npr;
-          // Groups of kLrGroup pairs: pair q with bit q of kPolyMask takes
-          // its sine and cosine from the FMA-pipe polynomial, interleaved
-          // with the SFU pairs of its group; the remaining pairs use the SFU.  The radial scales of two pairs come
-          // in one 16-byte load (the R' pair and the scales were two shared
-          // loads per node pair in the MIO queue beside four MUFU operations).
-          auto sfu_pair = [&](const float4 &v, float2 kp) {
-            const float2 th = __fmul2_rn(kp, u2);
-            float s0, c0, s1, c1;
-            sfu_sincos(th.x, &s0, &c0);
-            sfu_sincos(th.y, &s1, &c1);
-            const float2 C = make_float2(c0, c1), Sn = make_float2(s0, s1);
-            const float2 RX = make_float2(v.x, v.y), RY = make_float2(v.z, v.w);
-            EA = __ffma2_rn(C, RX, EA);
-            EB = __ffma2_rn(Sn, RY, EB);
-            G = __ffma2_rn(kp, __ffma2_rn(C, RY, __fmul2_rn(Sn, RX)), G);
-          };
-          uint32_t k = 0;  // even throughout
-          for (; k + kLrGroup <= npr; k += kLrGroup) {
-            float4 kq;
-#pragma unroll
-            for (int q = 0; q < kLrGroup; q++) {
-              if ((q & 1) == 0) kq = kq4[(k + q) >> 1];
-              const float2 kp = (q & 1) ? make_float2(kq.z, kq.w) : make_float2(kq.x, kq.y);
-              const float4 v = nn[k + q];
-              if ((kPolyMask >> q) & 1u) {
-                const float2 th = __fmul2_rn(kp, u2);
-                float2 C, Sn, sg;
-                fma_sincos_signed2(th, 1.0f, &Sn, &C, &sg);  // sg = (+-1, +-1)
-                const float2 RX = __fmul2_rn(make_float2(v.x, v.y), sg);
-                const float2 RY = __fmul2_rn(make_float2(v.z, v.w), sg);
-                EA = __ffma2_rn(C, RX, EA);
-                EB = __ffma2_rn(Sn, RY, EB);
-                G = __ffma2_rn(kp, __ffma2_rn(C, RY, __fmul2_rn(Sn, RX)), G);
-              } else {
-                sfu_pair(v, kp);
-              }
-            }
-          }
-          // The last, partial group of a direction stays on the SFU: its
-          // polynomial pairs, either guarded in a second unrolled copy of the
-          // group (water10k 1.491 ms) or one pair per step with a uniform
-          // test of the mask (1.511 ms), were slower than none (1.397 ms) --
-          // only interleaved with the SFU pairs of a full group does the
-          // polynomial's dependent chain hide.
-          for (; k + 2 <= npr; k += 2) {
-            const float4 kq = kq4[k >> 1];
-            sfu_pair(nn[k], make_float2(kq.x, kq.y));
-            sfu_pair(nn[k + 1], make_float2(kq.z, kq.w));
-          }
-          if (k < npr) {
-            const float4 kq = kq4[k >> 1];
-            sfu_pair(nn[k], make_float2(kq.x, kq.y));
-          }
-          const float e = (EA.x + EA.y) - (EB.x + EB.y), gsum = G.x + G.y;
-          te += e;
-          tx = fmaf(gsum, sj.x, tx);
-          ty = fmaf(gsum, sj.y, ty);
-          tz = fmaf(gsum, sj.z, tz);
-        }
-        if (mine) {
-          ee += te;
-          ex += tx;
-          ey += ty;
-          ez += tz;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (active) {
-    const double q = static_cast<double>(pa.w);
-    double4 *dst = part + (size_t)by * natom + p;
-    double4 v = make_double4(q * ex, q * ey, q * ez, q * ee);
-    if (accumulate) {  // a later node stage adds into the same rows
-      const double4 o = *dst;
-      v = make_double4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
-    }
-    *dst = v;
+    for (int c = 0; c < 4; c++)
+      for (int o = 16; o > 0; o >>= 1) f[c] += __shfl_xor_sync(0xffffffffu, f[c], o);
+    if (lane < 4) acc[4 * j + lane] += (double)(lane == 0 ? f[0] : lane == 1 ? f[1] : lane == 2 ? f[2] : f[3]);
   }
 }
 
-template <int kVariant>
-__global__ void __launch_bounds__(kLrThreads, 8)
-k_long_range_flat(const float4 *__restrict__ pk, const uint32_t *__restrict__ cell_point, uint32_t ncell,
-                  const LrChunk *__restrict__ chunks, const float4 *__restrict__ dirs,
-                  const float *__restrict__ kappa, const float2 *__restrict__ R, uint32_t node_off,
-                  uint32_t natom, int accumulate, double4 *__restrict__ part,
-                  const __grid_constant__ LrKappaQuads kpq) {
-  lr_block<kLrPolyMasks[kVariant], true>(pk, cell_point, ncell, chunks, dirs, kappa, R, node_off, natom,
-                                         accumulate, part, blockIdx.x, blockIdx.y, &kpq);
+// Sum two atoms' values over lanes that differ in `bit`: lanes with the bit
+// clear keep the first atom's, the others the second's.
+template <int NV>
+__device__ __forceinline__ void lr_merge(const float *a, const float *b, int bit, float *out) {
+  const bool up = (threadIdx.x & bit) != 0;
+#pragma unroll
+  for (int c = 0; c < NV; c++) {
+    const float keep = up ? b[c] : a[c], give = up ? a[c] : b[c];
+    out[c] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+  }
+}
+
+// One direction's two series at a scaled atom: (e, e').
+template <int P>
+__device__ __forceinline__ float2 lr_series(const float2 (&AB)[P], float4 s, float4 at) {
+  constexpr int B = cheb_b(P);
+  const float x = fmaf(s.x, at.x, fmaf(s.y, at.y, s.z * at.z));
+  const float x2 = x + x;
+  float T[B + 1];
+  T[0] = 1.0f;
+  T[1] = x;
+#pragma unroll
+  for (int b = 2; b <= B; b++) T[b] = fmaf(x2, T[b - 1], -T[b - 2]);
+  const float tb2 = T[B] + T[B];
+  float g0 = 1.0f, g1 = T[B];
+  float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int g = 0; g * B < P; g++) {
+    float2 in = AB[g * B];
+#pragma unroll
+    for (int b = 1; b < B && g * B + b < P; b++) in = __ffma2_rn(AB[g * B + b], bcast(T[b]), in);
+    sum = g == 0 ? in : __ffma2_rn(in, bcast(g0), sum);
+    const float g2 = fmaf(tb2, g1, -g0);
+    g0 = g1;
+    g1 = g2;
+  }
+  return sum;
+}
+
+// R' of a tile whose radial nodes fit one chunk, to shared memory, without
+// waiting: the tile's nodes are one run, lanes aligned to R's node blocks.
+__device__ __forceinline__ void lr_fetch(const LrArgs &a, const DirTile &u, uint32_t cell, float2 *s_r) {
+  const uint32_t lane = threadIdx.x & 31u, rc = u.n_rad;
+  if (rc <= (uint32_t)kSfRadChunk) {
+    const uint32_t node0 = u.node_begin - a.node_off, j0 = node0 % kNodeBlock;
+    const uint32_t inv = sf_row(rc) == rc ? 0u : 0xffffffffu / rc + 1u;
+    const uint32_t end = j0 + u.n_dir * rc;
+    const float2 *src = a.R + ((size_t)(node0 / kNodeBlock) * a.ncell + cell) * kNodeBlock + lane;
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(s_r));
+    for (uint32_t k = lane; k < end; k += 32, src += (size_t)a.ncell * kNodeBlock)
+      if (k >= j0) {
+        const uint32_t m = k - j0 + __umulhi(k - j0, inv);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * m), "l"(src) : "memory");
+      }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// One tile's series at the warp's na atoms, added to acc.  `next`: the tile
+// whose R' is fetched meanwhile (if any).
+template <int P>
+__device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const DirTile *next, uint32_t na,
+                                        uint32_t cell, const float4 *__restrict__ s_at, double *__restrict__ acc,
+                                        float2 *s_r) {
+  constexpr int B = cheb_b(P);
+  const uint32_t lane = threadIdx.x & 31u;
+  float2 c2[P / 2];  // (c_p, c_{p+1})
+#pragma unroll
+  for (int m = 0; m < P / 2; m++) c2[m] = make_float2(0.f, 0.f);
+  for (uint32_t r0 = 0; r0 < u.n_rad; r0 += kSfRadChunk) {
+    const uint32_t rc = min((uint32_t)kSfRadChunk, u.n_rad - r0);
+    if (rc < u.n_rad) {
+      const uint32_t node0 = u.node_begin - a.node_off;
+      __syncwarp();
+      for (uint32_t m = lane; m < u.n_dir * rc; m += 32) {
+        const uint32_t d = m / rc, r = m - d * rc;
+        s_r[d * sf_row(rc) + r] = a.R[sr_index(cell, node0 + d * u.n_rad + r0 + r, a.ncell)];
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    const float2 *row = s_r + (lane < u.n_dir ? lane : 0) * sf_row(rc);
+    const float4 *t = a.tab + u.lr_tab / 4 + (size_t)r0 * (cheb_row(P) / 4);
+#pragma unroll 2
+    for (uint32_t r = 0; r < rc; r++, t += cheb_row(P) / 4) {
+      const float2 v = row[r];
+#pragma unroll
+      for (int m = 0; m < cheb_row(P) / 4; m++) {
+        const float4 c = __ldg(t + m);
+        c2[2 * m] = __ffma2_rn(v, make_float2(c.x, c.y), c2[2 * m]);
+        if (2 * m + 1 < P / 2) c2[2 * m + 1] = __ffma2_rn(v, make_float2(c.z, c.w), c2[2 * m + 1]);
+      }
+    }
+  }
+  __syncwarp();  // every lane has read its row
+  if (next) lr_fetch(a, *next, cell, s_r);
+  // (c_p, c'_p): the derivative's series by c'_{p-1} = c'_{p+1} + 2 p c_p,
+  // then both in the product basis (T_{Bg+b} = 2 T_{Bg} T_b - T_{Bg-b})
+  float2 AB[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) AB[p].x = (p & 1) ? c2[p / 2].y : c2[p / 2].x;
+  AB[P - 1].y = 0.f;
+#pragma unroll
+  for (int p = P - 1; p > 0; p--) AB[p - 1].y = fmaf(2.0f * p, AB[p].x, p + 1 < P ? AB[p + 1].y : 0.f);
+  AB[0].y *= 0.5f;
+#pragma unroll
+  for (int p = P - 1; p > B; p--) {
+    const int g = p / B, b = p % B;
+    if (b == 0) continue;
+    AB[B * g - b] = __ffma2_rn(AB[p], bcast(-1.0f), AB[B * g - b]);
+    AB[p] = __fadd2_rn(AB[p], AB[p]);
+  }
+  // inactive lanes contribute nothing
+  const float live = lane < u.n_dir ? 1.0f : 0.0f;
+  const float4 s = lane < u.n_dir ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  // g = -e' / U
+  const float3 sg = make_float3(-a.cs.inv_u * s.x, -a.cs.inv_u * s.y, -a.cs.inv_u * s.z);
+  const uint32_t slot = 4u * (((lane >> 4) & 1u) + 2u * ((lane >> 3) & 1u) + 4u * ((lane >> 2) & 1u)) + (lane & 3u);
+  for (uint32_t j0 = 0; j0 < na; j0 += kLrBatch) {
+    float q4[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      float m2[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        float v[2][4];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const float2 eg = lr_series<P>(AB, s, s_at[j0 + 4 * h + 2 * i + k]);
+          v[k][0] = live * eg.x;
+          v[k][1] = eg.y * sg.x;
+          v[k][2] = eg.y * sg.y;
+          v[k][3] = eg.y * sg.z;
+        }
+        lr_merge<4>(v[0], v[1], 16, m2[i]);
+      }
+      lr_merge<4>(m2[0], m2[1], 8, q4[h]);
+    }
+    float e4[4], e2[2], e1[1];
+    lr_merge<4>(q4[0], q4[1], 4, e4);
+    lr_merge<2>(e4, e4 + 2, 2, e2);
+    lr_merge<1>(e2, e2 + 1, 1, e1);
+    acc[4 * j0 + slot] += (double)e1[0];
+  }
+}
+
+// Work item of a warp: a cell and a chunk of direction tiles.
+__device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t chunk) {
+  extern __shared__ float4 s_lr[];
+  const uint32_t cnt = a.cell_count[cell];
+  if (cnt == 0) return;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t start = a.cell_point[cell];
+  const uint32_t t0 = chunk * a.tiles_per_chunk, t1 = min(a.n_tiles, t0 + a.tiles_per_chunk);
+  const uint32_t rc = min(a.max_rad, (uint32_t)kSfRadChunk);
+  float4 *s_at = s_lr + warp * kLrAtomTile;
+  double *acc = reinterpret_cast<double *>(s_lr + kLrWarps * kLrAtomTile) + warp * (kLrAtomTile * 4);
+  float2 *s_r = reinterpret_cast<float2 *>(reinterpret_cast<double *>(s_lr + kLrWarps * kLrAtomTile) +
+                                           kLrWarps * kLrAtomTile * 4) + (size_t)warp * 32 * sf_row(rc);
+  for (uint32_t a0 = 0; a0 < cnt; a0 += kLrAtomTile) {
+    const uint32_t na = min((uint32_t)kLrAtomTile, cnt - a0), pad = (na + kLrBatch - 1) & ~(uint32_t)(kLrBatch - 1);
+    // the first series tile
+    auto is_series = [&](const DirTile &u) { return u.n_dir > 0 && u.lr_P > 0 && 16u * na > u.lr_P; };
+    uint32_t t = t0;
+    while (t < t1 && !is_series(a.tiles[t])) t++;
+    DirTile u;
+    if (t < t1) {
+      u = a.tiles[t];
+      lr_fetch(a, u, cell, s_r);
+    }
+    bool beyond = false;
+    for (uint32_t i = lane; i < 4 * pad; i += 32) acc[i] = 0.0;
+    for (uint32_t b0 = 0; b0 < pad; b0 += 32) {
+      const uint32_t i = b0 + lane;
+      const float4 p = i < na ? a.pk[start + a0 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool in = fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z)) <= a.cs.u2;
+      // (an atom beyond the range: its series sums are dropped below)
+      s_at[i] = in ? make_float4(p.x * a.cs.inv_u, p.y * a.cs.inv_u, p.z * a.cs.inv_u, 0.f)
+                   : make_float4(0.f, 0.f, 0.f, 1.f);
+      beyond |= __any_sync(0xffffffffu, !in) != 0;
+    }
+    __syncwarp();
+    while (t < t1) {
+      uint32_t tn = t + 1;
+      while (tn < t1 && !is_series(a.tiles[tn])) tn++;
+      DirTile un;
+      if (tn < t1) un = a.tiles[tn];
+      const DirTile *next = tn < t1 ? &un : nullptr;
+#define GLST_LR_CASE(n) \
+  case n: lr_tile<n>(a, u, next, na, cell, s_at, acc, s_r); break;
+      switch (u.lr_P) {
+      GLST_LR_CASE(4) GLST_LR_CASE(6) GLST_LR_CASE(8) GLST_LR_CASE(10) GLST_LR_CASE(12)
+      GLST_LR_CASE(14) GLST_LR_CASE(16) GLST_LR_CASE(18) GLST_LR_CASE(20) GLST_LR_CASE(22)
+      GLST_LR_CASE(24) GLST_LR_CASE(26) GLST_LR_CASE(28) GLST_LR_CASE(30) GLST_LR_CASE(32)
+      GLST_LR_CASE(34) GLST_LR_CASE(36) GLST_LR_CASE(38) GLST_LR_CASE(40) GLST_LR_CASE(42)
+      GLST_LR_CASE(44) GLST_LR_CASE(46) GLST_LR_CASE(48) GLST_LR_CASE(52) GLST_LR_CASE(56)
+      GLST_LR_CASE(60) GLST_LR_CASE(64)
+        default: break;
+      }
+#undef GLST_LR_CASE
+      t = tn;
+      u = un;
+    }
+    __syncwarp();
+    if (beyond) {  // drop their series sums; lr_direct gives theirs
+      for (uint32_t i = lane; i < na; i += 32)
+        if (s_at[i].w != 0.f) acc[4 * i] = acc[4 * i + 1] = acc[4 * i + 2] = acc[4 * i + 3] = 0.0;
+      __syncwarp();
+    }
+    for (uint32_t td = t0; td < t1; td++) {
+      const DirTile d = a.tiles[td];
+      if (d.n_dir == 0) continue;
+      const bool series = is_series(d);
+      if (!series || beyond) lr_direct(a, d, a.pk + start + a0, na, !series, cell, acc);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < na; i += 32) {
+      const double q = static_cast<double>(a.pk[start + a0 + i].w);
+      double4 *dst = a.part + (size_t)chunk * a.natom + start + a0 + i;
+      double4 o = make_double4(q * acc[4 * i + 1], q * acc[4 * i + 2], q * acc[4 * i + 3], q * acc[4 * i]);
+      if (a.accumulate) {
+        const double4 d = *dst;
+        o = make_double4(d.x + o.x, d.y + o.y, d.z + o.z, d.w + o.w);
+      }
+      *dst = o;
+    }
+    __syncwarp();
+  }
+}
+
+// Items chunk by chunk, so that the first (largest) groups' work starts first
+// and a CTA's warps share a chunk's tables.
+__global__ void __launch_bounds__(kLrThreads, 3)
+k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
+  const uint64_t item = (uint64_t)blockIdx.x * kLrWarps + (threadIdx.x >> 5);
+  const uint32_t chunk = (uint32_t)(item / a.ncell);
+  if (chunk >= n_chunks) return;
+  lr_warp(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
 }
 
 // ----------------------------------------------------------------------------

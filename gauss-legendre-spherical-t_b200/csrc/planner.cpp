@@ -521,19 +521,31 @@ static void bessel_j(double z, unsigned n, double *j) {
   for (unsigned p = 0; p < n; p++) j[p] /= sum;
 }
 
-unsigned series_terms(double z_max, unsigned max_terms) {
-  std::vector<double> j(max_terms + 24);
-  bessel_j(z_max, static_cast<unsigned>(j.size()), j.data());
-  // the omitted terms, bounded by 2 sum_{p >= P} |J_p(z_max)|, stay below
-  // 2e-7: |J_p| grows with z below its first maximum at z > p, so smaller z
-  // omit less.  FP32 rounding of a phase of z_max rad is larger (6e-8 z_max),
-  // and only the largest radial node's phase at the edge of the range omits
-  // this much (4e-8 of the structure factors' RMS at z_max = 18).
+unsigned series_terms(const std::vector<double> &z, const double *w, unsigned max_terms) {
+  // The omitted terms at |x| = 1, 2 sum_{p >= P} |J_p(z)|.  Without weights:
+  // of the largest z (J_p grows with z below its first maximum at z > p), at
+  // most 2e-7; FP32 rounding of a phase of z rad is larger (6e-8 z), and only
+  // the largest z at the edge of the range omits this much (4e-8 of the
+  // structure factors' RMS at z = 18).  With weights: the mean over w z (the
+  // derivative's weights, which favour large z more than the sum's own), at
+  // most 1e-8.
+  const unsigned n = max_terms + 24;
+  const double z_max = z.empty() ? 0.0 : *std::max_element(z.begin(), z.end());
+  std::vector<double> j(n), omit(n, 0.0);
+  double norm = 0.0;
+  for (size_t r = 0; r < z.size(); r++) {
+    const double wz = w ? std::abs(w[r]) * z[r] : (z[r] == z_max ? 1.0 : 0.0);
+    if (!(wz > 0.0)) continue;
+    bessel_j(z[r], n, j.data());
+    for (unsigned p = 0; p < n; p++) omit[p] += 2.0 * wz * std::abs(j[p]);
+    norm += wz;
+  }
+  const double limit = (w ? 1e-8 : 2e-7) * norm;
   double tail = 0.0;
-  unsigned P = static_cast<unsigned>(j.size());
-  while (P > 1 && tail + 2.0 * std::abs(j[P - 1]) <= 2e-7) tail += 2.0 * std::abs(j[--P]);
+  unsigned P = n;
+  while (P > 1 && tail + omit[P - 1] <= limit) tail += omit[--P];
   P = std::max(4u, P <= 48 ? (P + 1) / 2 * 2 : (P + 3) / 4 * 4);
-  return P <= max_terms && z_max < P ? P : 0;
+  return P <= max_terms && z_max < n - 16 ? P : 0;
 }
 
 void phase_series(double z, unsigned P, double *c) {

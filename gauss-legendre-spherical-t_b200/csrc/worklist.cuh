@@ -22,11 +22,8 @@ struct SysDesc {
   uint32_t *atom_cell, *atom_slot, *perm, *sorted_idx, *cell_count, *cell_point;
   float4 *pk;
   double4 *pd;
-  const float4 *dirs;
-  const float *kappa;
-  const LrChunk *chunks;
   SfArgs sf;    // structure-factor arguments
-  float2 *S, *R;
+  LrArgs lr;    // gather arguments
   double4 *part, *sr;
   double *cfx, *cfy, *cfz, *cen, *ofx, *ofy, *ofz, *oen, *block_energy, *energy;
 };
@@ -85,22 +82,14 @@ __global__ void __launch_bounds__(256) k_sort_pack_multi(const SysDesc *__restri
   }
 }
 
-// item (a, b) = (quad of direction tiles, cell).  The arguments are copied to
-// shared memory and the body is called out of line: inlined into the item
-// loop its moments were spilled to local memory.
-__device__ __noinline__ void sf_item(const SfArgs &a, uint32_t quad, uint32_t cell) { sf_block(a, quad, cell); }
-
+// item (a, b) = (quad of direction tiles, first of kSfCells cells); always one
+// CTA per item (inside a loop over items the moments went to local memory)
 __global__ void __launch_bounds__(kSfThreads, 4) k_structure_factors_multi(const SysDesc *__restrict__ sys,
                                                                           const WorkItem *__restrict__ items,
                                                                           uint32_t n) {
-  __shared__ SfArgs s_args;
-  for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const WorkItem w = items[it];
-    if (threadIdx.x == 0) s_args = sys[w.sys].sf;
-    __syncthreads();
-    sf_item(s_args, w.a, w.b);
-    __syncthreads();
-  }
+  const WorkItem w = items[blockIdx.x];
+  const SfArgs a = sys[w.sys].sf;
+  sf_block(a, w.a, w.b);
 }
 
 // item a = block of nb nodes; dynamic shared memory: the largest system's
@@ -116,17 +105,20 @@ __global__ void __launch_bounds__(kSatThreads, 3) k_shell_sums_multi(const SysDe
   }
 }
 
-// item (a, b) = (block of kLrThreads atoms, long-range chunk); seven CTAs per
-// SM, as the structure factors; the default polynomial share (the work
-// list takes only systems with the default launch variants)
-__global__ void __launch_bounds__(kLrThreads, 7) k_long_range_multi(const SysDesc *__restrict__ sys,
+// item (a, b) = (first of kLrWarps cells, long-range chunk); out of line, as
+// the structure factors
+__device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_warp(a, cell, chunk); }
+
+__global__ void __launch_bounds__(kLrThreads, 3) k_long_range_multi(const SysDesc *__restrict__ sys,
                                                                     const WorkItem *__restrict__ items,
                                                                     uint32_t n) {
+  __shared__ LrArgs s_args;
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
-    const SysDesc &d = sys[w.sys];
-    lr_block<kLrPolyMasks[0], false>(d.pk, d.cell_point, d.g.ncell, d.chunks, d.dirs, d.kappa, d.R, 0, d.natom, 0,
-                              d.part, w.a, w.b);
+    if (threadIdx.x == 0) s_args = sys[w.sys].lr;
+    __syncthreads();
+    const uint32_t cell = w.a + (threadIdx.x >> 5);
+    if (cell < s_args.ncell) lr_item(s_args, cell, w.b);
     __syncthreads();
   }
 }

@@ -80,9 +80,7 @@ typedef struct glst_info {
                                nodes per CTA; 1: the grid's per-node table
                                does not fit in shared memory, tables in global
                                memory (any grid size) */
-  uint32_t gather_variant;  /* share of the gather's sines/cosines on the FMA
-                               pipe: 0 = 2 in 14 node pairs (default), 1 =
-                               none, 2 = 1 in 14, 3 = 3 in 14 (glst_autotune) */
+  uint32_t gather_variant;  /* always 0 (kept for the structure's layout) */
   uint32_t sf_max_npt;      /* always 12 (kept for the structure's layout) */
 } glst_info;
 
@@ -211,12 +209,10 @@ glst_status glst_plan(uint32_t natom, double tol, double box_x, double box_y,
                       uint32_t *group);
 
 /* Autotuner: times, on these inputs (device FP64 arrays, as glst_compute),
- * the shell-sum kernel for 1..32 nodes per CTA, the long-range gather for
- * 2..32 waves of chunk CTAs and for each of its compiled FMA-pipe sine/cosine
- * shares; keeps the fastest for this handle, and remembers them for every later
+ * the shell-sum kernel for 1..32 nodes per CTA and the long-range gather for
+ * 2..32 waves of warps; keeps the fastest for this handle, and remembers them for every later
  * handle of the same shape (cells, nodes, atom-count bucket) in this process.
- * Returns the first two choices (glst_get_info reports the others).  Waits for
- * the stream; outputs must be recomputed afterwards.  Handles whose far field
+ * Returns the two choices.  Waits for the stream; outputs must be recomputed afterwards.  Handles whose far field
  * runs in one node stage only.  No reference counterpart. */
 glst_status glst_autotune(glst_handle *h, const double *d_rx,
                           const double *d_ry, const double *d_rz,
