@@ -886,11 +886,17 @@ static glst_status phase_lr(glst_handle *h, cudaStream_t st) {
   return (h->K && single_stage(h)) ? lr_stage(h, 0, st) : GLST_OK;
 }
 
+static uint32_t sr_blocks(uint32_t ncell, uint32_t warps_per_cell) {
+  return (uint32_t)(((uint64_t)ncell * warps_per_cell + dev::kSrWarps - 1) / dev::kSrWarps);
+}
+
 static glst_status phase_sr(glst_handle *h, cudaStream_t st) {
   if (!h->plan.natom || h->shard > 0) return GLST_OK;  // shard 0 owns the near field
-  dim3 grid(h->plan.ncell, h->sr_rows);
+  const uint32_t width = dev::sr_width(h->plan.natom, h->sr_rows);
+  const uint32_t wpc = dev::sr_warps_per_cell(h->plan.natom, h->plan.ncell, width);
+  dim3 grid(sr_blocks(h->plan.ncell, wpc), h->sr_rows);
   dev::k_short_range<<<grid, dev::kSrThreads, 0, st>>>(h->pd, h->cell_count, h->cell_point, h->grid,
-                                                       h->plan.natom, h->sr, h->sr_rows);
+                                                       h->plan.natom, h->sr, h->sr_rows, wpc, width);
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }
@@ -1645,7 +1651,10 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     each(glst_batch::kSr, [&](uint32_t w, glst_handle *h) {
       if (!h->plan.natom) return;
       for (uint32_t pl = 0; pl < h->sr_rows; pl++)
-        for (uint32_t c = 0; c < h->plan.ncell; c++) items.push_back({w, c, pl, 0});
+        for (uint32_t c = 0; c < sr_blocks(h->plan.ncell, dev::sr_warps_per_cell(h->plan.natom, h->plan.ncell,
+                                                                              dev::sr_width(h->plan.natom, h->sr_rows)));
+             c++)
+          items.push_back({w, c, pl, 0});
     });
     each(glst_batch::kCombine, [&](uint32_t w, glst_handle *h) {
       if (h->plan.natom)

@@ -1298,126 +1298,169 @@ k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
 // ----------------------------------------------------------------------------
 // Near field (src/glst_force.cu:1170-1544 restated): bare q_i q_j / r over
 // the own cell (self skipped) and the up to 26 neighbour cells inside the
-// grid (open boundary).  FP64 throughout.  CTA = (cell, row of neighbour
-// cells, below); thread = atom; each row writes its own partial row of
-// per-atom sums, summed by k_combine in a fixed order.  Smaller CTAs (64 or 96 threads, which
-// fit in the registers the shell-sum blocks leave free) measured slower on
-// water10k: 3.132 / 3.136 ms per solve against 3.122 ms.
+// grid (open boundary).  FP64 throughout, bound by the FP64 pipe: 18
+// operations per pair, the reciprocal square root a hardware approximation
+// and one third-order step (below) instead of the library's general one.
+//
+// The three neighbour cells along z are consecutive cells, so their atoms are
+// one run: nine runs, (dx, dy), cover the neighbourhood.  One warp per (32
+// atoms of a cell, row of runs), the runs' atoms staged 32 at a time in the
+// warp's own shared memory, the next 32 loaded meanwhile -- no CTA barriers,
+// and full batches where cells hold few atoms.  Cells of at most 16 or 8 atoms
+// split each batch over two or four groups of lanes, and so do systems too
+// small to fill the GPU with one lane per (atom, row) (sr_width).  A row is one run or the
+// three of an x plane, and writes its own partial row of per-atom sums, summed
+// by k_combine in a fixed order.
+// Measured (one thread per atom and CTA barriers between cells before):
+// water10k 0.291 -> 0.220 ms, 168 atoms per cell 0.400 -> 0.285 ms, 26^3 cells
+// of 6 atoms 0.485 -> 0.101 ms, 3,000 atoms on 4^3 cells 0.067 -> 0.052 ms, a
+// million atoms 4.44 -> 4.03 ms.
 constexpr int kSrThreads = 128;
-// One CTA per (cell, row of neighbour cells) writes one row of per-atom
-// partial sums: 3 rows (the x planes, 9 cells each) or 9 rows (x, y lines,
-// 3 cells each).  Rows are numbered in x-major order of the 27 neighbours;
-// the row holding the cell itself starts with it.  Nine rows shorten each
-// thread's serial run of pairs threefold and triple the CTAs, for grids too
-// small to fill the GPU with three (3,000 atoms on 4^3 cells: 0.076 ->
-// 0.033 ms; 9,000 atoms on 5^3: 0.162 -> 0.092 ms; 18,000 on 6^3: 0.244 ->
-// 0.117 ms); water10k's 7^3 grid already has 1,029 CTAs, and there nine
-// rows measured 0.2 % slower per solve beside the far field.
-// In the nine-row form each thread also runs two chains of accumulators
-// (pairs j and j+1) instead of one, so the FP64 pipe has more independent
-// work (3,000 atoms: near field 0.033 -> 0.025 ms, solve 0.141 -> 0.133 ms;
-// 9,000 atoms: solve 0.239 -> 0.223 ms).  The three-row form keeps one
-// chain: on water10k two chains made the near field 18 % faster alone but
-// the solve 0.2 % slower beside the far field.
+constexpr int kSrWarps = kSrThreads / 32;
 constexpr int kSrRowsPlanes = 3;
 constexpr int kSrRowsLines = 9;
 constexpr int kSrRowsMax = kSrRowsLines;
 
-template <bool kTwoChains>
-__device__ __forceinline__ void sr_block(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
-                                         const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
-                                         double4 *__restrict__ sr, uint32_t rows, uint32_t cell, uint32_t by) {
-  __shared__ double4 s_at[kSrThreads];
-  const int n = 27 / static_cast<int>(rows);  // neighbour cells per row
-  const int t0 = static_cast<int>(by) * n;    // x-major index of the row's first neighbour
-  const int dx = t0 / 9 - 1;                  // constant along a row
-  const bool own_row = static_cast<int>(by) == 13 / n;
+// 1 / sqrt(x): y0 with relative error d (the hardware's, below 2^-20), then
+// with h = 1 - x y0^2 the series (1 - h)^{-1/2} = 1 + h / 2 + 3 h^2 / 8 to
+// second order; the rest, 5 h^3 / 16, is below 1e-17.  Zero, infinite and
+// not-a-number results of the approximation stand.
+__device__ __forceinline__ double sr_rsqrt(double x) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+  const double h = fma(-(x * y0), y0, 1.0);
+  const double y = fma(y0 * h, fma(0.375, h, 0.5), y0);
+  return (unsigned)(__double2hiint(y0) - 0x00100000) >= 0x7fe00000u ? y0 : y;
+}
+
+struct SrSum {
+  double x, y, z, e;
+};
+
+// One staged batch: lanes take atoms sub, sub + groups, ..., four at a time in
+// four independent chains (a pair is a dozen dependent FP64 operations, and
+// their latency, not their number, bounds a warp that does one pair after
+// another).  The batch is padded with uncharged far-away atoms.
+constexpr int kSrChains = 4;
+template <bool kOwn>
+__device__ __forceinline__ void sr_batch(const double4 *s_at, uint32_t n, uint32_t sub, uint32_t groups,
+                                         const double4 &me, uint32_t self, SrSum (&f)[kSrChains]) {
+#pragma unroll 1
+  for (uint32_t j0 = sub; j0 < n; j0 += kSrChains * groups) {
+    double dx[kSrChains], dy[kSrChains], dz[kSrChains], ir[kSrChains], q[kSrChains];
+#pragma unroll
+    for (int u = 0; u < kSrChains; u++) {
+      const uint32_t j = j0 + u * groups;
+      const double4 o = s_at[j];
+      const bool same = kOwn && j == self;
+      dx[u] = me.x - o.x;
+      dy[u] = me.y - o.y;
+      dz[u] = me.z - o.z;
+      q[u] = same ? 0.0 : o.w;
+      const double r2 = fma(dx[u], dx[u], fma(dy[u], dy[u], dz[u] * dz[u]));
+      ir[u] = sr_rsqrt(same ? 1.0 : r2);
+    }
+#pragma unroll
+    for (int u = 0; u < kSrChains; u++) {
+      const double e = q[u] * ir[u];
+      const double fs = e * (ir[u] * ir[u]);
+      f[u].x = fma(fs, dx[u], f[u].x);
+      f[u].y = fma(fs, dy[u], f[u].y);
+      f[u].z = fma(fs, dz[u], f[u].z);
+      f[u].e += e;
+    }
+  }
+}
+
+// A warp's share of a cell: chunks chunk0, chunk0 + warps_per_cell, ... of its
+// atoms against row `row` of `rows`.
+__device__ __forceinline__ void sr_warp(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
+                                        const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
+                                        double4 *__restrict__ sr, uint32_t rows, uint32_t row, uint32_t cell,
+                                        uint32_t chunk0, uint32_t warps_per_cell, uint32_t max_width,
+                                        double4 *s_at) {
   const uint32_t cnt = cell_count[cell];
+  const uint32_t width = min(max_width, cnt > 16 ? 32u : cnt > 8 ? 16u : 8u), groups = 32u / width;
+  if (chunk0 * width >= cnt) return;
+  const uint32_t lane = threadIdx.x & 31u, sub = lane / width, li = lane & (width - 1u);
   const uint32_t start = cell_point[cell];
   const int ix = cell / (g.ny * g.nz), iy = (cell / g.nz) % g.ny, iz = cell % g.nz;
-  const int jx = ix + dx;
-  const bool plane_in = jx >= 0 && jx < (int)g.nx;
-  for (uint32_t a0 = 0; a0 < cnt; a0 += kSrThreads) {
-    const uint32_t ai = a0 + threadIdx.x;
-    const bool active = ai < cnt;
-    const double4 me = active ? pd[start + ai] : make_double4(0., 0., 0., 0.);
-    double fx = 0.0, fy = 0.0, fz = 0.0, en = 0.0;
-    // (own cell first in its row, as the reference's intra kernel)
-    for (int nbi = 0; nbi < n && plane_in; nbi++) {
-      const int t = t0 + (own_row ? (nbi + n / 2) % n : nbi);
-      const int dyc = (t / 3) % 3 - 1, dzc = t % 3 - 1;
-      const int jy = iy + dyc, jz = iz + dzc;
-      if (jy < 0 || jz < 0 || jy >= (int)g.ny || jz >= (int)g.nz) continue;
-      const bool own = dx == 0 && dyc == 0 && dzc == 0;
-      const uint32_t nb = (jx * g.ny + jy) * g.nz + jz;
-      const uint32_t bcnt = cell_count[nb];
-      const uint32_t bstart = cell_point[nb];
-      for (uint32_t b0 = 0; b0 < bcnt; b0 += kSrThreads) {
-        const uint32_t nbt = min((uint32_t)kSrThreads, bcnt - b0);
-        __syncthreads();
-        if (threadIdx.x < nbt) s_at[threadIdx.x] = pd[bstart + b0 + threadIdx.x];
-        __syncthreads();
-        if (!active) continue;
-        auto pair = [&](uint32_t j, double &ax, double &ay, double &az, double &an) {
-          if (own && b0 + j == ai) return;  // self
-          const double4 o4 = s_at[j];
-          const double dx = me.x - o4.x, dy = me.y - o4.y, dz = me.z - o4.z;
-          const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-          const double ir = rsqrt(r2);
-          const double e = me.w * o4.w * ir;
-          const double fs = e * ir * ir;
-          ax = fma(fs, dx, ax);
-          ay = fma(fs, dy, ay);
-          az = fma(fs, dz, az);
-          an += e;
-        };
-        if constexpr (kTwoChains) {
-          // branch-free pairs (the self pair selected to zero), so the two
-          // chains' instructions interleave
-          double gx = 0.0, gy = 0.0, gz = 0.0, gn = 0.0;
-          uint32_t j = 0;
-          for (; j + 1 < nbt; j += 2) {
-            const double4 o4 = s_at[j], p4 = s_at[j + 1];
-            const bool sa = own && b0 + j == ai, sb = own && b0 + j + 1 == ai;
-            const double dx = me.x - o4.x, dy = me.y - o4.y, dz = me.z - o4.z;
-            const double hx = me.x - p4.x, hy = me.y - p4.y, hz = me.z - p4.z;
-            const double r2 = sa ? 1.0 : fma(dx, dx, fma(dy, dy, dz * dz));
-            const double s2 = sb ? 1.0 : fma(hx, hx, fma(hy, hy, hz * hz));
-            const double ir = rsqrt(r2), is = rsqrt(s2);
-            const double e = sa ? 0.0 : me.w * o4.w * ir;
-            const double h = sb ? 0.0 : me.w * p4.w * is;
-            const double fs = e * ir * ir, hs = h * is * is;
-            fx = fma(fs, dx, fx);
-            gx = fma(hs, hx, gx);
-            fy = fma(fs, dy, fy);
-            gy = fma(hs, hy, gy);
-            fz = fma(fs, dz, fz);
-            gz = fma(hs, hz, gz);
-            en += e;
-            gn += h;
-          }
-          if (j < nbt) pair(j, fx, fy, fz, en);
-          fx += gx;
-          fy += gy;
-          fz += gz;
-          en += gn;
-        } else {
-          for (uint32_t j = 0; j < nbt; j++) pair(j, fx, fy, fz, en);
-        }
+  const uint32_t z0 = iz > 0 ? iz - 1 : 0, z1 = min(iz + 1, (int)g.nz - 1);
+  const uint32_t n_runs = kSrRowsLines / rows;
+  for (uint32_t a0 = chunk0 * width; a0 < cnt; a0 += warps_per_cell * width) {
+    const bool active = a0 + li < cnt;
+    const uint32_t i = start + a0 + li;
+    const double4 me = active ? pd[i] : make_double4(0., 0., 0., 0.);
+    const double4 none = make_double4(1e30, 1e30, 1e30, 0.);
+    SrSum f4[kSrChains] = {};
+    for (uint32_t q = 0; q < n_runs; q++) {
+      const int t = row * n_runs + q, dx = t / 3 - 1, dy = t % 3 - 1;
+      const int jx = ix + dx, jy = iy + dy;
+      if (jx < 0 || jy < 0 || jx >= (int)g.nx || jy >= (int)g.ny) continue;
+      const uint32_t c = (jx * g.ny + jy) * g.nz;
+      uint32_t b = cell_point[c + z0];
+      const uint32_t end = cell_point[c + z1] + cell_count[c + z1];
+      const bool own = dx == 0 && dy == 0;
+      double4 ahead = b + lane < end ? pd[b + lane] : none;
+      for (; b < end; b += 32) {
+        __syncwarp();
+        s_at[lane] = ahead;
+        __syncwarp();
+        ahead = b + 32 + lane < end ? pd[b + 32 + lane] : none;
+        const uint32_t n = min(32u, end - b);
+        if (own) sr_batch<true>(s_at, n, sub, groups, me, i - b, f4);
+        else sr_batch<false>(s_at, n, sub, groups, me, 0, f4);
       }
     }
-    if (active) sr[(size_t)by * natom + start + ai] = make_double4(fx, fy, fz, en);
+    SrSum f;
+    f.x = (f4[0].x + f4[1].x) + (f4[2].x + f4[3].x);
+    f.y = (f4[0].y + f4[1].y) + (f4[2].y + f4[3].y);
+    f.z = (f4[0].z + f4[1].z) + (f4[2].z + f4[3].z);
+    f.e = (f4[0].e + f4[1].e) + (f4[2].e + f4[3].e);
+    for (uint32_t o = width; o < 32; o <<= 1) {
+      f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
+      f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
+      f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
+      f.e += __shfl_xor_sync(0xffffffffu, f.e, o);
+    }
+    if (active && sub == 0) {
+      const double qi = me.w;
+      sr[(size_t)row * natom + i] = make_double4(qi * f.x, qi * f.y, qi * f.z, qi * f.e);
+    }
   }
+}
+
+// CTA: kSrWarps / warps_per_cell cells.
+__device__ __forceinline__ void sr_block(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
+                                         const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
+                                         double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell,
+                                         uint32_t max_width, uint32_t bx, uint32_t row) {
+  __shared__ double4 s_at[kSrWarps][32];
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t w = bx * kSrWarps + warp, cell = w / warps_per_cell;
+  if (cell >= g.ncell) return;
+  sr_warp(pd, cell_count, cell_point, g, natom, sr, rows, row, cell, w - cell * warps_per_cell, warps_per_cell,
+          max_width, s_at[warp]);
 }
 
 __global__ void __launch_bounds__(kSrThreads)
 k_short_range(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
               const uint32_t *__restrict__ cell_point, Grid g, uint32_t natom,
-              double4 *__restrict__ sr, uint32_t rows) {
-  if (rows == kSrRowsLines)
-    sr_block<true>(pd, cell_count, cell_point, g, natom, sr, rows, blockIdx.x, blockIdx.y);
-  else
-    sr_block<false>(pd, cell_count, cell_point, g, natom, sr, rows, blockIdx.x, blockIdx.y);
+              double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell, uint32_t max_width) {
+  sr_block(pd, cell_count, cell_point, g, natom, sr, rows, warps_per_cell, max_width, blockIdx.x, blockIdx.y);
+}
+
+// Lanes per chunk, at most: the widest chunks of which there are still 2,048
+// (about four warps for each of the GPU's schedulers), else 8 atoms wide.
+__host__ __device__ inline uint32_t sr_width(uint32_t natom, uint32_t rows) {
+  const uint64_t lanes = (uint64_t)natom * rows;
+  return lanes >= 2048u * 32u ? 32u : lanes >= 2048u * 16u ? 16u : 8u;
+}
+
+// Warps per cell for a mean number of atoms per cell.
+__host__ __device__ inline uint32_t sr_warps_per_cell(uint32_t natom, uint32_t ncell, uint32_t width) {
+  const uint32_t mean = natom / ncell;
+  return 4 * mean <= 3 * width ? 1u : 4 * mean <= 7 * width ? 2u : 4u;
 }
 
 // ----------------------------------------------------------------------------

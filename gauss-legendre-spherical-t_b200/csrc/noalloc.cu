@@ -186,7 +186,7 @@ extern "C" glst_status glst_near_field_noalloc(uint32_t natom, const double *d_r
     dev::k_sort_pack<<<(uint32_t)ncell, 256, dev::kSortCap * sizeof(uint32_t), st>>>(
         perm, cell_count, cell_point, g, atom_cell, natom, d_rx, d_ry, d_rz, d_qc, sorted, pk, pd);
     dev::k_short_range<<<dim3((uint32_t)ncell, dev::kSrRowsPlanes), dev::kSrThreads, 0, st>>>(
-        pd, cell_count, cell_point, g, natom, sr, dev::kSrRowsPlanes);
+        pd, cell_count, cell_point, g, natom, sr, dev::kSrRowsPlanes, dev::kSrWarps, dev::sr_width(natom, dev::kSrRowsPlanes));
     dev::k_combine<<<(natom + dev::kCombineAtoms - 1) / dev::kCombineAtoms, dev::kCombineThreads, 0, st>>>(
         sr, dev::kSrRowsPlanes, nullptr, 0, sorted, natom, 0, cell_out, cell_out + kMaxAtoms, cell_out + 2ull * kMaxAtoms,
         cell_out + 3ull * kMaxAtoms, d_fx, d_fy, d_fz, d_en, block_e);

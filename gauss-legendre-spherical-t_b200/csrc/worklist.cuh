@@ -123,17 +123,15 @@ __global__ void __launch_bounds__(kLrThreads, 3) k_long_range_multi(const SysDes
   }
 }
 
-// item (a, b) = (cell, row of neighbour cells)
+// item (a, b) = (block of cells, row of neighbour cells)
 __global__ void __launch_bounds__(kSrThreads) k_short_range_multi(const SysDesc *__restrict__ sys,
                                                                   const WorkItem *__restrict__ items,
                                                                   uint32_t n) {
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const SysDesc &d = sys[w.sys];
-    if (d.sr_rows == kSrRowsLines)
-      sr_block<true>(d.pd, d.cell_count, d.cell_point, d.g, d.natom, d.sr, d.sr_rows, w.a, w.b);
-    else
-      sr_block<false>(d.pd, d.cell_count, d.cell_point, d.g, d.natom, d.sr, d.sr_rows, w.a, w.b);
+    sr_block(d.pd, d.cell_count, d.cell_point, d.g, d.natom, d.sr, d.sr_rows, sr_warps_per_cell(d.natom, d.g.ncell, sr_width(d.natom, d.sr_rows)),
+             sr_width(d.natom, d.sr_rows), w.a, w.b);
     __syncthreads();
   }
 }
