@@ -751,7 +751,8 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
     const uint32_t nb = (N + 255) / 256;
     dev::k_scatter<<<nb, 256, 0, st>>>(h->atom_cell, h->atom_slot, h->cell_point, N, h->perm);
     CUDA_TRY(cudaGetLastError());
-    dev::k_sort_pack<<<C, 256, dev::kSortCap * sizeof(uint32_t), st>>>(
+    const uint32_t spc = dev::sort_cells(N, C);
+    dev::k_sort_pack<<<(C + spc - 1) / spc, 32 * dev::kSortCells, dev::kSortCap * sizeof(uint32_t), st>>>(
         h->perm, h->cell_count, h->cell_point, h->grid, h->atom_cell, N, rx, ry, rz, qc, h->sorted_idx, h->pk,
         h->pd);
     CUDA_TRY(cudaGetLastError());
@@ -766,16 +767,18 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
 static dev::SfArgs sf_args(const glst_handle *h, const glst_handle::FarRange &rg) {
   return dev::SfArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
                      reinterpret_cast<const float4 *>(h->cheb), h->S, h->R, h->cheb_scale, h->plan.ncell,
-                     rg.u1 - rg.u0, h->max_rad, rg.kb, h->sf_tab4};
+                     rg.u1 - rg.u0, h->max_rad, rg.kb, h->sf_tab4,
+                     dev::sf_cells(h->plan.natom, h->plan.ncell)};
 }
 
 static glst_status sf_stage(glst_handle *h, const glst_handle::FarRange &rg, cudaStream_t st) {
   if (rg.u1 <= rg.u0 || !h->plan.natom) return GLST_OK;
   const uint32_t quads = (rg.u1 - rg.u0) / dev::kSfWarps;
-  const uint32_t per_launch = 0x7fffffffu / quads / dev::kSfCells * dev::kSfCells;  // cells (gridDim.x < 2^31)
+  const uint32_t cells = sf_args(h, rg).cells;
+  const uint32_t per_launch = 0x7fffffffu / quads / cells * cells;  // cells (gridDim.x < 2^31)
   for (uint32_t c0 = 0; c0 < h->plan.ncell; c0 += per_launch) {
     const uint32_t nc = std::min(per_launch, h->plan.ncell - c0);
-    dev::k_structure_factors<<<quads * ((nc + dev::kSfCells - 1) / dev::kSfCells), dev::kSfThreads,
+    dev::k_structure_factors<<<quads * ((nc + cells - 1) / cells), dev::kSfThreads,
                                 dev::sf_smem_bytes(h->max_rad, h->sf_tab4), st>>>(sf_args(h, rg), c0);
     CUDA_TRY(cudaGetLastError());
   }
@@ -915,9 +918,7 @@ static glst_status phase_combine(glst_handle *h, cudaStream_t st, const OutDest 
   if (N) {
     dev::k_combine<<<h->combine_blocks, dev::kCombineThreads, 0, st>>>(
         h->sr, h->sr_rows, h->part, h->part_rows, h->sorted_idx, N, h->K ? 1 : 0, h->cfx, h->cfy, h->cfz, h->cen,
-        ofx, ofy, ofz, oen, h->block_energy);
-    CUDA_TRY(cudaGetLastError());
-    dev::k_energy_total<<<1, 256, 0, st>>>(h->block_energy, h->combine_blocks, energy);
+        ofx, ofy, ofz, oen, h->block_energy, h->flags + 1, energy);
     CUDA_TRY(cudaGetLastError());
   } else {
     CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double), st));
@@ -1198,14 +1199,14 @@ glst_status glst_get_info(const glst_handle *h, glst_info *info) {
   info->device_bytes = h->bytes;
   // assignment 4 (+0 without atoms), near field 1, far field per stage:
   // structure factors 1, shell sums 1 (global-memory form: twiddles 1 + 4
-  // per node batch), gather 1; combine 2
+  // per node batch), gather 1; combine 1
   uint32_t far = 0;
   if (h->K && h->plan.natom)
     for (const auto &rg : h->ranges) {
       const uint32_t nblk = (rg.ke - rg.kb + dev::kNodeBlock - 1) / dev::kNodeBlock;
       far += 2u + (h->gsat ? 1u + 4u * ((nblk + h->gsat_nblk - 1) / h->gsat_nblk) : 1u);
     }
-  info->kernels_per_compute = h->plan.natom ? 4u + (h->shard == 0 ? 1u : 0u) + far + 2u : 2u;
+  info->kernels_per_compute = h->plan.natom ? 4u + (h->shard == 0 ? 1u : 0u) + far + 1u : 1u;
   info->node_stages = (uint32_t)h->ranges.size();
   info->shell_sums_form = h->gsat ? 1u : 0u;
   info->gather_variant = 0;
@@ -1629,13 +1630,14 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     });
     each(glst_batch::kSort, [&](uint32_t w, glst_handle *h) {
       if (h->plan.natom)
-        for (uint32_t c = 0; c < h->plan.ncell; c++) items.push_back({w, c, 0, 0});
+        for (uint32_t c = 0, spc = dev::sort_cells(h->plan.natom, h->plan.ncell); c < (h->plan.ncell + spc - 1) / spc; c++)
+          items.push_back({w, c, 0, 0});
     });
     each(glst_batch::kSf, [&](uint32_t w, glst_handle *h) {
       if (!h->K || !h->plan.natom) return;
       const uint32_t quads = h->n_tiles / dev::kSfWarps;
       gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad, h->sf_tab4));
-      for (uint32_t c = 0; c < h->plan.ncell; c += dev::kSfCells)
+      for (uint32_t c = 0; c < h->plan.ncell; c += dev::sf_cells(h->plan.natom, h->plan.ncell))
         for (uint32_t u = 0; u < quads; u++) items.push_back({w, u, c, 0});
     });
     each(glst_batch::kShell, [&](uint32_t w, glst_handle *h) {
@@ -1660,7 +1662,9 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
       if (h->plan.natom)
         for (uint32_t a = 0; a < h->combine_blocks; a++) items.push_back({w, a, 0, 0});
     });
-    each(glst_batch::kEnergy, [&](uint32_t w, glst_handle *) { items.push_back({w, 0, 0, 0}); });
+    each(glst_batch::kEnergy, [&](uint32_t w, glst_handle *h) {
+      if (!h->plan.natom) items.push_back({w, 0, 0, 0});  // (the combine writes the others')
+    });
     // shell sums: the group's largest shared-memory need
     for (uint32_t w = w0; w < w0 + nw; w++) {
       const glst_handle *h = b->sys[b->wl[w]];
@@ -1741,6 +1745,7 @@ static glst_status worklist_descriptors(glst_batch *b, const double *const in[4]
     d.oen = out[3] ? out[3] + o : h->oen;
     d.block_energy = h->block_energy;
     d.energy = b->energies + i;
+    d.ticket = h->flags + 1;
   }
   if (!ds.empty()) CUDA_TRY(cudaMemcpy(b->d_desc, ds.data(), ds.size() * sizeof(dev::SysDesc), cudaMemcpyHostToDevice));
   return GLST_OK;

@@ -93,19 +93,20 @@ __global__ void k_bin(const double *__restrict__ rx, const double *__restrict__ 
   bin_block(rx, ry, rz, n, g, atom_cell, atom_slot, cell_count, blockIdx.x);
 }
 
-// K_scan: exclusive offsets of the cell counts (one CTA of 1024 threads,
-// chunked block scan).
+// K_scan: exclusive offsets of the cell counts (one CTA of 1024 threads, four
+// consecutive cells per thread and step: 26^3 cells in 5 steps instead of 18).
 __device__ __forceinline__ void scan_body(const uint32_t *__restrict__ cell_count, uint32_t ncell,
                                           uint32_t *__restrict__ cell_point) {
   __shared__ uint32_t warp_sums[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t base = 0; base < ncell; base += blockDim.x) {
-    const uint32_t c = base + threadIdx.x;
-    const uint32_t v = (c < ncell) ? cell_count[c] : 0u;
-    uint32_t x = v;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < ncell; base += 4 * blockDim.x) {
+    const uint32_t c = base + 4 * threadIdx.x;
+    uint32_t v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = (c + u < ncell) ? cell_count[c + u] : 0u;
+    const uint32_t mine = v[0] + v[1] + v[2] + v[3];
+    uint32_t x = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -113,22 +114,21 @@ __device__ __forceinline__ void scan_body(const uint32_t *__restrict__ cell_coun
     }
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      const unsigned nw = blockDim.x >> 5;
-      uint32_t s = (lane < nw) ? warp_sums[lane] : 0u;
+    uint32_t s = (lane < nw) ? warp_sums[lane] : 0u;  // every warp scans the warps' sums
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= (unsigned)o) s += y;
-      }
-      if (lane < nw) warp_sums[lane] = s;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= (unsigned)o) s += y;
     }
-    __syncthreads();
-    const uint32_t before = carry + (warp ? warp_sums[warp - 1] : 0u) + (x - v);
-    if (c < ncell) cell_point[c] = before;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = before + v;
-    __syncthreads();
+    const uint32_t before_warp = __shfl_sync(0xffffffffu, s, (warp + 31) & 31u);
+    uint32_t p = carry + (warp ? before_warp : 0u) + (x - mine);
+    carry += __shfl_sync(0xffffffffu, s, 31);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (c + u < ncell) cell_point[c + u] = p;
+      p += v[u];
+    }
+    __syncthreads();  // warp_sums is rewritten
   }
 }
 
@@ -153,11 +153,19 @@ __global__ void k_scatter(const uint32_t *__restrict__ atom_cell,
   scatter_block(atom_cell, atom_slot, cell_point, n, perm, blockIdx.x);
 }
 
-// K_sort_pack: one CTA per cell.  The atomics of k_bin leave the atoms of a
-// cell in arbitrary order; sorting each cell's indices ascending reproduces
-// the order of a stable sort by cell id (the reference's CUB radix sort,
-// src/glst_force.cu:510-517).  Then writes the packets.  Launched with
-// blockDim.x a multiple of 32 and kSortCap u32 of dynamic shared memory.
+// K_sort_pack.  The atomics of k_bin leave the atoms of a cell in arbitrary
+// order; sorting each cell's indices ascending reproduces the order of a
+// stable sort by cell id (the reference's CUB radix sort,
+// src/glst_force.cu:510-517).  Then writes the packets.  A CTA takes one cell
+// (bitonic sort), or on sparse grids kSortCells cells: one warp each for cells
+// of up to kSortWarpCap atoms, an atom's place being the number of smaller
+// indices, then the whole CTA for each larger one.  Launched with 32
+// kSortCells threads and kSortCap u32 of dynamic shared memory.
+constexpr uint32_t kSortCells = 8;
+constexpr uint32_t kSortWarpCap = 32;
+__host__ __device__ inline uint32_t sort_cells(uint32_t natom, uint32_t ncell) {  // cells per CTA
+  return natom / ncell <= 16 ? kSortCells : 1u;
+}
 __device__ __forceinline__ void pack_atom(uint32_t slot, uint32_t a, double cx, double cy, double cz,
                                           const double *__restrict__ rx, const double *__restrict__ ry,
                                           const double *__restrict__ rz, const double *__restrict__ qc,
@@ -178,7 +186,7 @@ __device__ __forceinline__ void sort_pack_block(const uint32_t *__restrict__ per
                                                 const double *__restrict__ rz, const double *__restrict__ qc,
                                                 uint32_t *__restrict__ sorted_idx, float4 *__restrict__ pk,
                                                 double4 *__restrict__ pd, uint32_t cell) {
-  extern __shared__ uint32_t s_idx[];
+  extern __shared__ uint32_t s_idx[];  // the whole CTA's
   const uint32_t cnt = cell_count[cell];
   const uint32_t start = cell_point[cell];
   if (cnt == 0) return;
@@ -238,6 +246,47 @@ __device__ __forceinline__ void sort_pack_block(const uint32_t *__restrict__ per
     pack_atom(start + i, s_idx[i], cx, cy, cz, rx, ry, rz, qc, sorted_idx, pk, pd);
 }
 
+__device__ __forceinline__ void sort_pack_cells(const uint32_t *__restrict__ perm,
+                                                const uint32_t *__restrict__ cell_count,
+                                                const uint32_t *__restrict__ cell_point, const Grid &g,
+                                                const uint32_t *__restrict__ atom_cell, uint32_t natom,
+                                                const double *__restrict__ rx, const double *__restrict__ ry,
+                                                const double *__restrict__ rz, const double *__restrict__ qc,
+                                                uint32_t *__restrict__ sorted_idx, float4 *__restrict__ pk,
+                                                double4 *__restrict__ pd, uint32_t bx) {
+  extern __shared__ uint32_t s_idx[];
+  if (sort_cells(natom, g.ncell) == 1) {
+    sort_pack_block(perm, cell_count, cell_point, g, atom_cell, natom, rx, ry, rz, qc, sorted_idx, pk, pd, bx);
+    return;
+  }
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t cell = bx * kSortCells + warp;
+  const uint32_t cnt = cell < g.ncell ? cell_count[cell] : 0u;
+  if (cnt > 0 && cnt <= kSortWarpCap) {
+    const uint32_t start = cell_point[cell];
+    uint32_t *mine = s_idx + warp * kSortWarpCap;
+    for (uint32_t i = lane; i < cnt; i += 32) mine[i] = perm[start + i];
+    __syncwarp();
+    const uint32_t ix = cell / (g.ny * g.nz), iy = (cell / g.nz) % g.ny, iz = cell % g.nz;
+    const double cx = cell_centre(ix, g.l), cy = cell_centre(iy, g.l), cz = cell_centre(iz, g.l);
+    for (uint32_t i = lane; i < cnt; i += 32) {
+      const uint32_t a = mine[i];
+      uint32_t rank = 0;
+#pragma unroll 8
+      for (uint32_t j = 0; j < cnt; j++) rank += mine[j] < a ? 1u : 0u;
+      pack_atom(start + rank, a, cx, cy, cz, rx, ry, rz, qc, sorted_idx, pk, pd);
+    }
+  }
+  if (!__syncthreads_or(cnt > kSortWarpCap)) return;
+  for (uint32_t w = 0; w < kSortCells; w++) {
+    const uint32_t c = bx * kSortCells + w;
+    if (c < g.ncell && cell_count[c] > kSortWarpCap) {
+      sort_pack_block(perm, cell_count, cell_point, g, atom_cell, natom, rx, ry, rz, qc, sorted_idx, pk, pd, c);
+      __syncthreads();
+    }
+  }
+}
+
 __global__ void k_sort_pack(const uint32_t *__restrict__ perm,
                             const uint32_t *__restrict__ cell_count,
                             const uint32_t *__restrict__ cell_point, Grid g,
@@ -246,7 +295,7 @@ __global__ void k_sort_pack(const uint32_t *__restrict__ perm,
                             const double *__restrict__ rz, const double *__restrict__ qc,
                             uint32_t *__restrict__ sorted_idx, float4 *__restrict__ pk,
                             double4 *__restrict__ pd) {
-  sort_pack_block(perm, cell_count, cell_point, g, atom_cell, natom, rx, ry, rz, qc, sorted_idx, pk, pd,
+  sort_pack_cells(perm, cell_count, cell_point, g, atom_cell, natom, rx, ry, rz, qc, sorted_idx, pk, pd,
                   blockIdx.x);
 }
 
@@ -314,8 +363,8 @@ __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
 // accumulated and when it is multiplied out.
 //
 // A CTA's four warps take 32 directions of one group each, lane = direction,
-// moments in registers, atoms broadcast from shared memory, for kSfCells
-// cells; the group's table is copied to shared memory once (read through L1
+// moments in registers, atoms broadcast from shared memory, for one cell
+// (sparse grids: eight); the group's table is copied to shared memory once (read through L1
 // as broadcasts it took five wavefronts per 16 bytes, and half of L1's time).
 // After that the warps are independent.  FP32 over a tile of <=
 // kSfAtomTile atoms, then FP64 over the tiles of a denser cell.  S is stored
@@ -329,7 +378,6 @@ __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
 constexpr int kSfWarps = 4;
 constexpr int kSfThreads = 32 * kSfWarps;
 constexpr int kSfAtomTile = 128;
-constexpr int kSfCells = 1;       // cells per CTA (4: 5 % slower on water10k, 40 % on 1,000 waters)
 constexpr int kSfRadChunk = 64;   // radial nodes staged at a time, at most
 constexpr int kChebMaxP = 64;     // series terms, at most (even to 48, then multiples of 4)
 __host__ __device__ constexpr int cheb_b(int P) { return P > 24 ? 8 : 4; }
@@ -367,7 +415,13 @@ struct SfArgs {
   ChebScale cs;
   uint32_t ncell, n_tiles, max_rad, node_off;
   uint32_t tab4;       // float4s of the largest group's table
+  uint32_t cells;      // cells per CTA
 };
+
+// Cells per structure-factor CTA: one (four cost 5 % on water10k, 40 % on 1,000
+// waters), but eight where a cell's few atoms take less than copying the table
+// (26^3 cells of 6 atoms: 0.32 ms with one, 0.24 with four).
+__host__ __device__ inline uint32_t sf_cells(uint32_t natom, uint32_t ncell) { return natom / ncell <= 16 ? 8u : 1u; }
 
 // Rows of the staged results are an odd number of float2 apart (bank spread).
 __host__ __device__ constexpr uint32_t sf_row(uint32_t rc) { return rc | 1u; }
@@ -543,8 +597,8 @@ __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const
   } while (a0 < cnt);
 }
 
-// Work item: kSfWarps consecutive tiles (of one group) and kSfCells cells
-// from `cell0` on.
+// Work item: kSfWarps consecutive tiles (of one group) and a.cells cells from
+// `cell0` on.
 __device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_t cell0) {
   extern __shared__ float4 s_sf[];
   const uint32_t warp = threadIdx.x >> 5;
@@ -556,7 +610,7 @@ __device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_
   const uint32_t rc = min(a.max_rad, (uint32_t)kSfRadChunk);
   float4 *s_at = s_sf + a.tab4 + warp * 32;
   float2 *s_f = reinterpret_cast<float2 *>(s_sf + a.tab4 + kSfWarps * 32) + (size_t)warp * 32 * sf_row(rc);
-  const uint32_t cell1 = min(a.ncell, cell0 + kSfCells);
+  const uint32_t cell1 = min(a.ncell, cell0 + a.cells);
 #define GLST_SF_CASE(n)                                                                            \
   case n:                                                                                          \
     for (uint32_t cell = cell0; cell < cell1; cell++)                                              \
@@ -578,7 +632,7 @@ __global__ void __launch_bounds__(kSfThreads, 4)
 k_structure_factors(const __grid_constant__ SfArgs a, uint32_t cell_base) {
   const uint32_t quads = a.n_tiles / kSfWarps;
   const uint32_t c = blockIdx.x / quads;
-  sf_block(a, blockIdx.x - c * quads, cell_base + c * kSfCells);
+  sf_block(a, blockIdx.x - c * quads, cell_base + c * a.cells);
 }
 
 // ----------------------------------------------------------------------------
@@ -1475,6 +1529,22 @@ constexpr int kCombineThreads = 256;
 constexpr int kCombineAtoms = 32;
 constexpr int kCombineWarps = kCombineThreads / 32;
 
+// Total energy 0.5 * sum of the per-CTA sums, fixed order (one CTA).
+__device__ __forceinline__ void energy_body(const double *block_energy, uint32_t nblocks,
+                                            double *__restrict__ total) {
+  __shared__ double s_red[32];
+  double e = 0.0;
+  for (uint32_t b = threadIdx.x; b < nblocks; b += blockDim.x) e += __ldcg(block_energy + b);
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (unsigned w = 0; w < (blockDim.x >> 5); w++) t += s_red[w];
+    *total = 0.5 * t;
+  }
+}
+
 __device__ __forceinline__ void combine_block(const double4 *__restrict__ sr, uint32_t sr_rows,
                                               const double4 *__restrict__ part,
                                               uint32_t nsplit, const uint32_t *__restrict__ sorted_idx,
@@ -1483,8 +1553,10 @@ __device__ __forceinline__ void combine_block(const double4 *__restrict__ sr, ui
                                               double *__restrict__ cen, double *__restrict__ ofx,
                                               double *__restrict__ ofy, double *__restrict__ ofz,
                                               double *__restrict__ oen, double *__restrict__ block_energy,
-                                              uint32_t bx) {
+                                              uint32_t nblocks, uint32_t *__restrict__ ticket,
+                                              double *__restrict__ energy, uint32_t bx) {
   __shared__ double4 s_rows[kCombineWarps][kCombineAtoms];
+  __shared__ bool s_last;
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
   const uint32_t p = bx * kCombineAtoms + lane;
   const bool live = p < natom;
@@ -1497,9 +1569,8 @@ __device__ __forceinline__ void combine_block(const double4 *__restrict__ sr, ui
   }
   s_rows[w][lane] = acc;
   __syncthreads();
-  if (w != 0) return;
   double e = 0.0;
-  if (live) {
+  if (w == 0 && live) {
     double4 t = s_rows[0][lane];
 #pragma unroll
     for (int k = 1; k < kCombineWarps; k++) {
@@ -1515,8 +1586,20 @@ __device__ __forceinline__ void combine_block(const double4 *__restrict__ sr, ui
     if (i < natom) { ofx[i] = t.x; ofy[i] = t.y; ofz[i] = t.z; oen[i] = t.w; }
     e = t.w;
   }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  if (lane == 0) block_energy[bx] = e;
+  if (w == 0) {
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+    if (lane == 0) {
+      block_energy[bx] = e;
+      // the CTA that draws the last ticket (they wrap to 0 by themselves)
+      // sums the blocks' energies, in their order whichever CTA it is
+      __threadfence();
+      s_last = ticket && atomicInc(ticket, nblocks - 1) == nblocks - 1;
+    }
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  energy_body(block_energy, nblocks, energy);
 }
 
 __global__ void __launch_bounds__(kCombineThreads)
@@ -1524,9 +1607,10 @@ k_combine(const double4 *__restrict__ sr, uint32_t sr_rows, const double4 *__res
           const uint32_t *__restrict__ sorted_idx, uint32_t natom, int use_far,
           double *__restrict__ cfx, double *__restrict__ cfy, double *__restrict__ cfz,
           double *__restrict__ cen, double *__restrict__ ofx, double *__restrict__ ofy,
-          double *__restrict__ ofz, double *__restrict__ oen, double *__restrict__ block_energy) {
+          double *__restrict__ ofz, double *__restrict__ oen, double *__restrict__ block_energy,
+          uint32_t *__restrict__ ticket, double *__restrict__ energy) {
   combine_block(sr, sr_rows, part, nsplit, sorted_idx, natom, use_far, cfx, cfy, cfz, cen, ofx, ofy, ofz, oen,
-                block_energy, blockIdx.x);
+                block_energy, gridDim.x, ticket, energy, blockIdx.x);
 }
 
 // ----------------------------------------------------------------------------
@@ -1564,22 +1648,6 @@ k_reduce_shards(ShardSet ss, uint32_t natom, double *__restrict__ block_energy) 
     double t = 0.0;
     for (int w = 0; w < kCombineThreads / 32; w++) t += s_red[w];
     block_energy[blockIdx.x] = t;
-  }
-}
-
-// Total energy 0.5 * sum of the per-CTA sums, fixed order (one CTA).
-__device__ __forceinline__ void energy_body(const double *__restrict__ block_energy, uint32_t nblocks,
-                                            double *__restrict__ total) {
-  __shared__ double s_red[32];
-  double e = 0.0;
-  for (uint32_t b = threadIdx.x; b < nblocks; b += blockDim.x) e += block_energy[b];
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = e;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (unsigned w = 0; w < (blockDim.x >> 5); w++) t += s_red[w];
-    *total = 0.5 * t;
   }
 }
 

@@ -25,6 +25,7 @@ struct SysDesc {
   SfArgs sf;    // structure-factor arguments
   LrArgs lr;    // gather arguments
   double4 *part, *sr;
+  uint32_t *ticket;
   double *cfx, *cfy, *cfz, *cen, *ofx, *ofy, *ofz, *oen, *block_energy, *energy;
 };
 
@@ -70,19 +71,19 @@ __global__ void __launch_bounds__(256) k_scatter_multi(const SysDesc *__restrict
   }
 }
 
-// item a = cell; kSortCap u32 of dynamic shared memory
+// item a = block of kSortCells cells; kSortCap u32 of dynamic shared memory
 __global__ void __launch_bounds__(256) k_sort_pack_multi(const SysDesc *__restrict__ sys,
                                                          const WorkItem *__restrict__ items, uint32_t n) {
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const SysDesc &d = sys[w.sys];
-    sort_pack_block(d.perm, d.cell_count, d.cell_point, d.g, d.atom_cell, d.natom, d.rx, d.ry, d.rz, d.qc,
+    sort_pack_cells(d.perm, d.cell_count, d.cell_point, d.g, d.atom_cell, d.natom, d.rx, d.ry, d.rz, d.qc,
                     d.sorted_idx, d.pk, d.pd, w.a);
     __syncthreads();
   }
 }
 
-// item (a, b) = (quad of direction tiles, first of kSfCells cells); always one
+// item (a, b) = (quad of direction tiles, first of sf.cells cells); always one
 // CTA per item (inside a loop over items the moments went to local memory)
 __global__ void __launch_bounds__(kSfThreads, 4) k_structure_factors_multi(const SysDesc *__restrict__ sys,
                                                                           const WorkItem *__restrict__ items,
@@ -144,17 +145,17 @@ __global__ void __launch_bounds__(kCombineThreads) k_combine_multi(const SysDesc
     const WorkItem w = items[it];
     const SysDesc &d = sys[w.sys];
     combine_block(d.sr, d.sr_rows, d.part, d.part_rows, d.sorted_idx, d.natom, d.use_far, d.cfx, d.cfy, d.cfz, d.cen, d.ofx,
-                  d.ofy, d.ofz, d.oen, d.block_energy, w.a);
+                  d.ofy, d.ofz, d.oen, d.block_energy, d.combine_blocks, d.ticket, d.energy, w.a);
     __syncthreads();
   }
 }
 
-// one item per system
+// one item per system without atoms
 __global__ void __launch_bounds__(256) k_energy_multi(const SysDesc *__restrict__ sys,
                                                       const WorkItem *__restrict__ items, uint32_t n) {
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const SysDesc &d = sys[items[it].sys];
-    energy_body(d.block_energy, d.combine_blocks, d.energy);
+    energy_body(d.block_energy, 0, d.energy);
     __syncthreads();
   }
 }
