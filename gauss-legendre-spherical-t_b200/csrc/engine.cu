@@ -101,6 +101,7 @@ static std::shared_ptr<TDesignStore> get_store() {
 
 // ---------------------------------------------------------------- handle
 static constexpr uint32_t kLrWaves = 4;  // waves of gather warps, untuned
+static constexpr size_t kLrSmemMax = 75 << 10;  // three gather CTAs per SM
 
 struct DevBuf {
   void *p = nullptr;
@@ -146,8 +147,9 @@ struct glst_handle {
   float4 *dirs = nullptr;       // unit directions, FP32
   float *kappa = nullptr;       // radial scales per group, FP32
   dev::DirTile *tiles = nullptr;    // runs of up to 32 directions of one group
-  float *cheb = nullptr;            // per group, n_radial x P: Chebyshev series of the phases
+  float *cheb = nullptr, *cheb_lr = nullptr;  // per group, n_radial x P: Chebyshev series of the phases
                                     // (structure factors: product basis; gather: plain)
+  uint32_t lr_tab4 = 0;             // float4s of the gather's tables
   dev::ChebScale cheb_scale{};
   std::vector<uint32_t> g_sf_P, g_sf_tab, g_lr_P, g_lr_tab;  // per group: series terms, offset of the table
   uint32_t sf_tab4 = 0;             // float4s of the largest structure-factor table
@@ -494,8 +496,10 @@ static glst_status set_kernel_attributes(int device, size_t shell_smem) {
   if (!(d & 1)) {
     CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dev::sf_smem_bytes(dev::kSfRadChunk, dev::kLrMaxRad * dev::kChebMaxP / 4)));
-    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dev::lr_smem_bytes(dev::kSfRadChunk)));
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kLrSmemMax));
     CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(dev::kSortCap * sizeof(uint32_t))));
     d |= 1;
@@ -564,7 +568,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   h->g_lr_tab.clear();
   h->max_rad = 1;
   h->sf_tab4 = 0;
-  std::vector<float> cheb;
+  std::vector<float> cheb, cheb_lr;
   uint32_t nquad = 0;
   {
     uint32_t ref_base = 0, ibase = 0;
@@ -591,11 +595,11 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
           cheb.insert(cheb.end(), c.begin(), c.end());
         }
         h->g_lr_P.push_back(lr_P);
-        h->g_lr_tab.push_back((uint32_t)cheb.size());
+        h->g_lr_tab.push_back((uint32_t)cheb_lr.size());
         for (unsigned r = 0; lr_P && r < g.n_radial; r++) {
           c.assign(dev::cheb_row((int)lr_P), 0.0);
           glst::phase_series(z[r], lr_P, c.data());
-          cheb.insert(cheb.end(), c.begin(), c.end());
+          cheb_lr.insert(cheb_lr.end(), c.begin(), c.end());
         }
       }
       dir_base.push_back((uint32_t)dirs.size());
@@ -628,6 +632,8 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     GLST_TRY(dalloc_n(h, &h->dirs, dirs.size()));
     GLST_TRY(dalloc_n(h, &h->kappa, kap.size()));
     GLST_TRY(dalloc_n(h, &h->cheb, cheb.size()));
+    GLST_TRY(dalloc_n(h, &h->cheb_lr, cheb_lr.size()));
+    h->lr_tab4 = (uint32_t)(cheb_lr.size() / 4);
   }
   GLST_TRY(dalloc_n(h, &h->atom_cell, N));
   GLST_TRY(dalloc_n(h, &h->atom_slot, N));
@@ -722,6 +728,8 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     CUDA_TRY(cudaMemcpyAsync(h->dirs, dirs.data(), dirs.size() * sizeof(float4), cudaMemcpyHostToDevice, h->side));
     CUDA_TRY(cudaMemcpyAsync(h->kappa, kap.data(), kap.size() * sizeof(float), cudaMemcpyHostToDevice, h->side));
     CUDA_TRY(cudaMemcpyAsync(h->cheb, cheb.data(), cheb.size() * sizeof(float), cudaMemcpyHostToDevice, h->side));
+    CUDA_TRY(cudaMemcpyAsync(h->cheb_lr, cheb_lr.data(), cheb_lr.size() * sizeof(float), cudaMemcpyHostToDevice,
+                             h->side));
   }
   if (shard > 0) CUDA_TRY(cudaMemsetAsync(h->sr, 0, (size_t)h->sr_rows * N * sizeof(double4), h->side));
   GLST_TRY(set_kernel_attributes(h->device, 0));
@@ -834,9 +842,10 @@ static glst_status shell_stage(glst_handle *h, const glst_handle::FarRange &rg, 
 static dev::LrArgs lr_args(const glst_handle *h, size_t stage) {
   const auto &rg = h->ranges[stage];
   return dev::LrArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
-                     reinterpret_cast<const float4 *>(h->cheb), h->R, h->part, h->cheb_scale, h->plan.ncell,
+                     reinterpret_cast<const float4 *>(h->cheb_lr), h->R, h->part, h->cheb_scale, h->plan.ncell,
                      rg.u1 - rg.u0, rg.tpc, h->max_rad, rg.kb, h->plan.natom,
-                     stage > 0 ? 1 : 0};  // stage 0 writes its rows, later stages add into the same rows
+                     stage > 0 ? 1 : 0,  // stage 0 writes its rows, later stages add into the same rows
+                     h->lr_tab4};
 }
 
 static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
@@ -844,7 +853,11 @@ static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
   if (rg.u1 <= rg.u0 || !h->plan.natom) return GLST_OK;
   const uint64_t ctas = ((uint64_t)rg.rows() * h->plan.ncell + dev::kLrWarps - 1) / dev::kLrWarps;
   if (ctas > 0x7fffffffu) return fail(GLST_ERR_SIZE, "too many cells for the gather's grid");
-  dev::k_long_range<<<(uint32_t)ctas, dev::kLrThreads, dev::lr_smem_bytes(h->max_rad), st>>>(lr_args(h, stage), rg.rows());
+  const size_t smem = dev::lr_smem_bytes(h->max_rad), tab = h->lr_tab4 * sizeof(float4);
+  if (smem + tab <= kLrSmemMax)
+    dev::k_long_range<true><<<(uint32_t)ctas, dev::kLrThreads, smem + tab, st>>>(lr_args(h, stage), rg.rows());
+  else
+    dev::k_long_range<false><<<(uint32_t)ctas, dev::kLrThreads, smem, st>>>(lr_args(h, stage), rg.rows());
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }

@@ -1049,7 +1049,9 @@ __global__ void k_gsat_shell(Grid g, GsatArgs a) {
 // with no CTA barriers (four warps on one cell's chunk waited for each other
 // a third of the time).  A tile's R' is copied to shared memory
 // asynchronously while the previous tile's series are evaluated -- the buffer
-// is free once its coefficients are formed.
+// is free once its coefficients are formed.  The groups' tables are copied to
+// shared memory where three CTAs per SM still fit with them (water10k 485 ->
+// 478 us, 168 atoms per cell 149 -> 143, 648 atoms 47 -> 42).
 // Measured: water10k 1.458 -> 0.485 ms, 3,000 atoms on 4^3 cells 0.141 ->
 // 0.076 ms, 168 atoms per cell 0.279 -> 0.148 ms, a million atoms 55 -> 17 ms;
 // forces 1.5e-8 -> 0.9e-8 off the FP64 path.
@@ -1072,6 +1074,7 @@ struct LrArgs {
   ChebScale cs;
   uint32_t ncell, n_tiles, tiles_per_chunk, max_rad, node_off, natom;
   int accumulate;      // a later node stage adds into the same rows
+  uint32_t tab4;       // float4s of all groups' tables
 };
 
 __host__ __device__ inline size_t lr_smem_bytes(uint32_t max_rad) {
@@ -1169,12 +1172,13 @@ __device__ __forceinline__ void lr_fetch(const LrArgs &a, const DirTile &u, uint
 
 // One tile's series at the warp's na atoms, added to acc.  `next`: the tile
 // whose R' is fetched meanwhile (if any).
-template <int P>
+template <int P, bool kTabShared>
 __device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const DirTile *next, uint32_t na,
                                         uint32_t cell, const float4 *__restrict__ s_at, double *__restrict__ acc,
                                         float2 *s_r) {
   constexpr int B = cheb_b(P);
   const uint32_t lane = threadIdx.x & 31u;
+  const float4 s = lane < u.n_dir ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   float2 c2[P / 2];  // (c_p, c_{p+1})
 #pragma unroll
   for (int m = 0; m < P / 2; m++) c2[m] = make_float2(0.f, 0.f);
@@ -1191,13 +1195,14 @@ __device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     const float2 *row = s_r + (lane < u.n_dir ? lane : 0) * sf_row(rc);
-    const float4 *t = a.tab + u.lr_tab / 4 + (size_t)r0 * (cheb_row(P) / 4);
+    extern __shared__ float4 s_lr[];
+    const float4 *t = (kTabShared ? s_lr : a.tab) + u.lr_tab / 4 + (size_t)r0 * (cheb_row(P) / 4);
 #pragma unroll 2
     for (uint32_t r = 0; r < rc; r++, t += cheb_row(P) / 4) {
       const float2 v = row[r];
 #pragma unroll
       for (int m = 0; m < cheb_row(P) / 4; m++) {
-        const float4 c = __ldg(t + m);
+        const float4 c = kTabShared ? t[m] : __ldg(t + m);
         c2[2 * m] = __ffma2_rn(v, make_float2(c.x, c.y), c2[2 * m]);
         if (2 * m + 1 < P / 2) c2[2 * m + 1] = __ffma2_rn(v, make_float2(c.z, c.w), c2[2 * m + 1]);
       }
@@ -1223,7 +1228,6 @@ __device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const
   }
   // inactive lanes contribute nothing
   const float live = lane < u.n_dir ? 1.0f : 0.0f;
-  const float4 s = lane < u.n_dir ? a.dirs[u.dir_begin + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   // g = -e' / U
   const float3 sg = make_float3(-a.cs.inv_u * s.x, -a.cs.inv_u * s.y, -a.cs.inv_u * s.z);
   const uint32_t slot = 4u * (((lane >> 4) & 1u) + 2u * ((lane >> 3) & 1u) + 4u * ((lane >> 2) & 1u)) + (lane & 3u);
@@ -1256,6 +1260,7 @@ __device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const
 }
 
 // Work item of a warp: a cell and a chunk of direction tiles.
+template <bool kTabShared>
 __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t chunk) {
   extern __shared__ float4 s_lr[];
   const uint32_t cnt = a.cell_count[cell];
@@ -1264,9 +1269,10 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
   const uint32_t start = a.cell_point[cell];
   const uint32_t t0 = chunk * a.tiles_per_chunk, t1 = min(a.n_tiles, t0 + a.tiles_per_chunk);
   const uint32_t rc = min(a.max_rad, (uint32_t)kSfRadChunk);
-  float4 *s_at = s_lr + warp * kLrAtomTile;
-  double *acc = reinterpret_cast<double *>(s_lr + kLrWarps * kLrAtomTile) + warp * (kLrAtomTile * 4);
-  float2 *s_r = reinterpret_cast<float2 *>(reinterpret_cast<double *>(s_lr + kLrWarps * kLrAtomTile) +
+  float4 *s_own = s_lr + (kTabShared ? a.tab4 : 0u);  // (the tables come first)
+  float4 *s_at = s_own + warp * kLrAtomTile;
+  double *acc = reinterpret_cast<double *>(s_own + kLrWarps * kLrAtomTile) + warp * (kLrAtomTile * 4);
+  float2 *s_r = reinterpret_cast<float2 *>(reinterpret_cast<double *>(s_own + kLrWarps * kLrAtomTile) +
                                            kLrWarps * kLrAtomTile * 4) + (size_t)warp * 32 * sf_row(rc);
   for (uint32_t a0 = 0; a0 < cnt; a0 += kLrAtomTile) {
     const uint32_t na = min((uint32_t)kLrAtomTile, cnt - a0), pad = (na + kLrBatch - 1) & ~(uint32_t)(kLrBatch - 1);
@@ -1298,7 +1304,7 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
       if (tn < t1) un = a.tiles[tn];
       const DirTile *next = tn < t1 ? &un : nullptr;
 #define GLST_LR_CASE(n) \
-  case n: lr_tile<n>(a, u, next, na, cell, s_at, acc, s_r); break;
+  case n: lr_tile<n, kTabShared>(a, u, next, na, cell, s_at, acc, s_r); break;
       switch (u.lr_P) {
       GLST_LR_CASE(4) GLST_LR_CASE(6) GLST_LR_CASE(8) GLST_LR_CASE(10) GLST_LR_CASE(12)
       GLST_LR_CASE(14) GLST_LR_CASE(16) GLST_LR_CASE(18) GLST_LR_CASE(20) GLST_LR_CASE(22)
@@ -1341,12 +1347,18 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
 
 // Items chunk by chunk, so that the first (largest) groups' work starts first
 // and a CTA's warps share a chunk's tables.
+template <bool kTabShared>
 __global__ void __launch_bounds__(kLrThreads, 3)
 k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
+  if constexpr (kTabShared) {
+    extern __shared__ float4 s_lr[];
+    for (uint32_t i = threadIdx.x; i < a.tab4; i += kLrThreads) s_lr[i] = a.tab[i];
+    __syncthreads();
+  }
   const uint64_t item = (uint64_t)blockIdx.x * kLrWarps + (threadIdx.x >> 5);
   const uint32_t chunk = (uint32_t)(item / a.ncell);
   if (chunk >= n_chunks) return;
-  lr_warp(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
+  lr_warp<kTabShared>(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
 }
 
 // ----------------------------------------------------------------------------

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kSatThreads, 3) k_shell_sums_multi(const SysDe
 
 // item (a, b) = (first of kLrWarps cells, long-range chunk); out of line, as
 // the structure factors
-__device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_warp(a, cell, chunk); }
+__device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_warp<false>(a, cell, chunk); }
 
 __global__ void __launch_bounds__(kLrThreads, 3) k_long_range_multi(const SysDesc *__restrict__ sys,
                                                                     const WorkItem *__restrict__ items,
