@@ -450,35 +450,41 @@ def run_ours(args, world, rank, local, dist):
     torch.cuda.synchronize()
     e2e_ms, e2e_val = weak_throughput(e0.elapsed_time(e1), n * e_steps, dist, dev)
 
-    # roofline of the dominant kernel (SFU-bound phase kernels)
+    # roofline of the dominant far-field kernel: FP32 FMAs of its Chebyshev
+    # series -- per (atom, direction) P terms in the structure factors and two
+    # series of P terms in the gather, per (cell, node) a product over P terms.
+    # P as the engine chooses it (planner.cpp): tail of the Bessel coefficients
+    # at the largest node, or weighted by the quadrature's w kappa.
     sfu_peak, fma_peak = g.measure_pipe_peaks()
     K = inf.num_nodes
     dom = max(("structure_factors", "long_range"), key=lambda k: phases[k])
-    pairs = float(n) * K  # (atom, node) phase evaluations per launch
-    achieved_sfu = 2.0 * pairs / (phases[dom] * 1e-3)  # sin + cos per pair
+    kx, ky, kz, w, group = f.nodes()
+    tau = (np.arange(512) + 0.5) * np.pi / 512
+    p_idx = np.arange(88)
+    fma_ops = 0.0
+    for gi in range(inf.ngroup):
+        m = group == gi
+        n_rad = inf.group_gl_degree[gi] // 2
+        n_dir = inf.group_nodes[gi] / n_rad
+        kap = np.sqrt(kx[m] ** 2 + ky[m] ** 2 + kz[m] ** 2).reshape(n_rad, -1)[:, 0]
+        z = kap * 1.02 * 0.5 * np.sqrt(3.0) * inf.cell_dim
+        bes = np.abs(np.mean(np.cos(p_idx[None, :, None] * tau - z[:, None, None] * np.sin(tau)), axis=-1))
+        wz = w[m].reshape(n_rad, -1)[:, 0] * z if dom == "long_range" else (z == z.max()).astype(float)
+        tail = np.cumsum((2.0 * wz[:, None] * bes).sum(0)[::-1])[::-1]
+        P = int(np.count_nonzero(tail > (1e-8 if dom == "long_range" else 2e-7) * wz.sum()))
+        P += P % 2
+        fma_ops += n_dir * P * (float(n) * (2.0 if dom == "long_range" else 1.0) + float(inf.ncell_total) * n_rad)
+    fma_ach = fma_ops / (phases[dom] * 1e-3)
     roofline = {
-        "bound": "sfu", "kernel": dom, "achieved": achieved_sfu / 1e9, "peak": sfu_peak / 1e9,
-        "unit": "G sincos-results/s", "frac": achieved_sfu / sfu_peak,
-        "peak_source": "measured on this GPU by glst_measure_pipe_peaks (MUFU sin+cos loop)",
-        "traffic": 3.197e8 if dom == "long_range" else 2.298e8,
+        "bound": "fp32", "kernel": dom, "achieved": fma_ach / 1e9, "peak": fma_peak / 1e9,
+        "unit": "G FP32 FMA/s", "frac": fma_ach / fma_peak, "ops_per_launch": fma_ops,
+        "peak_source": "measured on this GPU by glst_measure_pipe_peaks (FP32 FMA loop)",
+        "traffic": 2.898e8 if dom == "long_range" else 2.242e8,
         "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this "
                           "kernel on this workload (profiles/water10k_solve_kernels.md)",
-        "pairs_per_launch": pairs,
-        "fp32_fma_peak_per_s": fma_peak,
+        "pairs_per_launch": float(n) * K,
+        "sfu_peak_per_s": sfu_peak,
     }
-    # The same kernel's algorithmic FP32 work against the measured FMA-pipe
-    # peak: per (atom, node) the phase kappa*u and the accumulation (five
-    # operations in the gather: c R'x, s R'y, s R'x, c R'y, kappa*(...); two
-    # in the structure factors), per (atom, direction) u = s.d (three).  The
-    # FMA-pipe sine/cosine share is not counted: it stands in for MUFU work.
-    n_dir = sum(inf.group_nodes[i] / (inf.group_gl_degree[i] // 2) for i in range(inf.ngroup))
-    ops_pair = 6.0 if dom == "long_range" else 3.0
-    fma_ops = float(n) * (ops_pair * K + 3.0 * n_dir)
-    fma_ach = fma_ops / (phases[dom] * 1e-3)
-    roofline["fma"] = {"achieved": fma_ach / 1e9, "peak": fma_peak / 1e9, "unit": "G FP32 ops/s",
-                       "frac": fma_ach / fma_peak, "ops_per_launch": fma_ops,
-                       "peak_source": "measured on this GPU by glst_measure_pipe_peaks (FP32 FMA loop)",
-                       "reading": "not the bound: the FMA pipe carries this plus part of the sin/cos"}
     # The same kernel against the HBM roofline (MEASURED_PEAKS.json): its
     # algorithmic bytes are the cross-cell operand it streams once (R read
     # for the gather, S written for the structure factors: C x K float2).
@@ -494,12 +500,12 @@ def run_ours(args, world, rank, local, dist):
     hbm_ach = hbm_bytes / (phases[dom] * 1e-3) / 1e9
     roofline["hbm"] = {"achieved": hbm_ach, "peak": hbm_peak, "unit": "GB/s", "frac": hbm_ach / hbm_peak,
                        "bytes_per_launch": hbm_bytes, "peak_source": hbm_src,
-                       "reading": "not the bound: the kernel is SFU-bound, HBM carries its operand once"}
+                       "reading": "not the bound: the kernel is bound by FP32 work, HBM carries its operand once"}
 
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f32 phases/sincos + f64 cell-relative/shell/energy",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f32 phase series + f64 cell-relative/shell/energy",
         "data": "synthetic (seeded TIP3P-like water, no dataset)",
         "config": {"workload": args.workload, "atoms": n, "box_A": L, "rcut_A": sysd["rcut"],
                    "tol": sysd["tol"], "cells": list(inf.ncell), "groups": inf.ngroup, "nodes": K,
