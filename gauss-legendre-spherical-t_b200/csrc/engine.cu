@@ -26,6 +26,11 @@ using glst::PlanError;
 using glst::TDesignStore;
 namespace dev = glst::dev;
 
+// the planner's tables are laid out as the kernels read them
+static_assert(glst::kSeriesMaxP == (unsigned)dev::kChebMaxP, "series terms");
+static_assert(glst::series_b(24) == (unsigned)dev::cheb_b(24) && glst::series_b(26) == (unsigned)dev::cheb_b(26) &&
+              glst::series_row(26) == (unsigned)dev::cheb_row(26), "series tables");
+
 // ---------------------------------------------------------------- errors
 static thread_local std::string g_last_error;
 
@@ -555,13 +560,9 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   std::vector<uint32_t> radii(K);
   std::vector<float4> dirs;
   std::vector<float> kap;
-  // Chebyshev series of the phases on |u| <= U, U the radius of the cell's
-  // circumscribed sphere and 2 % (atoms slightly outside the box stay within)
-  // Coordinates are scaled by 1 / U in FP32, so U is the reciprocal of an
-  // FP32 number: a rounded scale would stretch every phase alike.
-  const float cheb_inv = (float)(1.0 / (1.02 * 0.5 * std::sqrt(3.0) * p.cell_dim));
-  const double cheb_u = 1.0 / (double)cheb_inv;
-  h->cheb_scale = dev::ChebScale{cheb_inv, (float)(cheb_u * cheb_u)};
+  // Chebyshev series of the phases on |u| <= U (planner)
+  const double cheb_u = 1.0 / (double)p.inv_u;
+  h->cheb_scale = dev::ChebScale{p.inv_u, (float)(cheb_u * cheb_u)};
   h->g_sf_P.clear();
   h->g_sf_tab.clear();
   h->g_lr_P.clear();
@@ -576,32 +577,13 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
       const auto &g = p.groups[gi];
       kappa_base.push_back((uint32_t)kap.size());
       h->max_rad = std::max(h->max_rad, g.n_radial);
-      {
-        // series of the structure factors (product basis), then of the gather
-        std::vector<double> z, w, c;
-        for (unsigned r = 0; r < g.n_radial; r++) {
-          z.push_back(g.kappa[r] * cheb_u);
-          w.push_back(p.w[ref_base + (size_t)r * g.n_dir]);
-        }
-        const uint32_t sf_P = glst::series_terms(z, nullptr, dev::kChebMaxP);
-        const uint32_t lr_P = glst::series_terms(z, w.data(), dev::kChebMaxP);
-        h->g_sf_P.push_back(sf_P);
-        h->sf_tab4 = std::max<uint32_t>(h->sf_tab4, g.n_radial * (dev::cheb_row((int)sf_P) / 4));
-        h->g_sf_tab.push_back((uint32_t)cheb.size());
-        for (unsigned r = 0; sf_P && r < g.n_radial; r++) {
-          c.assign(dev::cheb_row((int)sf_P), 0.0);
-          glst::phase_series(z[r], sf_P, c.data());
-          glst::product_basis(sf_P, dev::cheb_b((int)sf_P), c.data());
-          cheb.insert(cheb.end(), c.begin(), c.end());
-        }
-        h->g_lr_P.push_back(lr_P);
-        h->g_lr_tab.push_back((uint32_t)cheb_lr.size());
-        for (unsigned r = 0; lr_P && r < g.n_radial; r++) {
-          c.assign(dev::cheb_row((int)lr_P), 0.0);
-          glst::phase_series(z[r], lr_P, c.data());
-          cheb_lr.insert(cheb_lr.end(), c.begin(), c.end());
-        }
-      }
+      h->g_sf_P.push_back(g.sf_P);
+      h->g_sf_tab.push_back((uint32_t)cheb.size());
+      h->sf_tab4 = std::max<uint32_t>(h->sf_tab4, (uint32_t)(g.sf_tab.size() / 4));
+      cheb.insert(cheb.end(), g.sf_tab.begin(), g.sf_tab.end());
+      h->g_lr_P.push_back(g.lr_P);
+      h->g_lr_tab.push_back((uint32_t)cheb_lr.size());
+      cheb_lr.insert(cheb_lr.end(), g.lr_tab.begin(), g.lr_tab.end());
       dir_base.push_back((uint32_t)dirs.size());
       node_base.push_back(ibase);
       for (unsigned r = 0; r < g.n_radial; r++) kap.push_back((float)g.kappa[r]);

@@ -407,6 +407,7 @@ Plan make_plan(uint32_t natom, double tol, const double box[3], double rcut,
     throw PlanError{GLST_ERR_SIZE, "cell grid too large"};
   p.ncell = static_cast<uint32_t>(nc);
   p.has_far = p.n[0] > 2 && p.n[1] > 2 && p.n[2] > 2;
+  p.inv_u = static_cast<float>(1.0 / (1.02 * 0.5 * std::sqrt(3.0) * p.cell_dim));
 
   // The groups and the cubature depend only on (tol, CT, grid, cell edge,
   // t-design source), not on natom or the exact box: reuse earlier plans.
@@ -480,6 +481,24 @@ Plan make_plan(uint32_t natom, double tol, const double box[3], double rcut,
                       (kPi * static_cast<double>(m)));
         p.group.push_back(static_cast<uint32_t>(gi));
       }
+    }
+    // the phases' series, part of the (kept) plan, so that a new handle of a
+    // known plan does not tabulate them again
+    std::vector<double> z, wr, c;
+    for (size_t i = 0; i < xs.size(); i++) {
+      z.push_back(g.kappa[i] / static_cast<double>(p.inv_u));
+      wr.push_back(ws[i] * std::exp(-zc2 * xs[i] * xs[i]));
+    }
+    g.sf_P = series_terms(z, nullptr, kSeriesMaxP);
+    g.lr_P = series_terms(z, wr.data(), kSeriesMaxP);
+    for (size_t i = 0; i < z.size(); i++) {
+      c.assign(series_row(std::max(g.sf_P, g.lr_P)), 0.0);
+      phase_series(z[i], g.sf_P, c.data());
+      product_basis(g.sf_P, series_b(g.sf_P), c.data());
+      g.sf_tab.insert(g.sf_tab.end(), c.begin(), c.begin() + series_row(g.sf_P));
+      c.assign(c.size(), 0.0);
+      phase_series(z[i], g.lr_P, c.data());
+      g.lr_tab.insert(g.lr_tab.end(), c.begin(), c.begin() + series_row(g.lr_P));
     }
   }
   if (p.kx.size() > 0xFFFFFFFFull)

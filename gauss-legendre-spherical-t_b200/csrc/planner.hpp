@@ -45,7 +45,16 @@ struct GroupPlan {
   unsigned n_radial = 0, n_dir = 0;
   std::vector<double> kappa;  // radial scales 2 alpha zcut x_i (n_radial)
   std::vector<double> dirs;   // unit directions s_j, xyz interleaved (3 n_dir)
+  // Chebyshev series of the phases (below): terms, and n_radial rows of
+  // series_row(P) floats -- of the structure factors (product basis) and of the
+  // gather (plain)
+  unsigned sf_P = 0, lr_P = 0;
+  std::vector<float> sf_tab, lr_tab;
 };
+
+constexpr unsigned kSeriesMaxP = 64;                                            // terms, at most
+constexpr unsigned series_b(unsigned P) { return P > 24 ? 8 : 4; }              // basis T_{Bg} T_b
+constexpr unsigned series_row(unsigned P) { return (P + 3) / 4 * 4; }
 
 struct Plan {
   uint32_t natom = 0;
@@ -55,6 +64,11 @@ struct Plan {
   uint32_t n[3] = {0, 0, 0};
   uint32_t ncell = 0;
   double cell_dim = 0;  // CT value widened to double
+  // 1 / U in FP32, U the series' range: the radius of the cell's circumscribed
+  // sphere and 2 % (atoms slightly outside the box stay within).  Coordinates
+  // are scaled by it in FP32, so U is the reciprocal of an FP32 number: a
+  // rounded scale would stretch every phase alike.
+  float inv_u = 0;
   bool has_far = false;
   std::vector<GroupPlan> groups;
   // Node set in the reference's order, FP64 (pre-CT-rounding).
