@@ -5,17 +5,19 @@
 nvcc cross-compiles for sm_100a without a GPU.  The shared library is written
 next to this file, where the ctypes loader looks for it.
 """
+import glob
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
+CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libglst_b200.so")
-SOURCES = [os.path.join(HERE, "csrc", "engine.cu"), os.path.join(HERE, "csrc", "planner.cpp"),
-           os.path.join(HERE, "csrc", "noalloc.cu")]
-HEADERS = [os.path.join(HERE, "csrc", "kernels.cuh"), os.path.join(HERE, "csrc", "planner.hpp"),
-           os.path.join(ROOT, "include", "glst_c.h")]
+# (source, defines); the slowest first, all compiled at the same time
+UNITS = [("far_field.cu", ["-DGLST_PART=%d" % i]) for i in range(5)] + [
+    ("engine.cu", []), ("noalloc.cu", []), ("planner.cpp", [])]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -26,21 +28,38 @@ def nvcc():
     return "nvcc"
 
 
+def inputs():
+    """Every file the library is built from."""
+    return [os.path.join(CSRC, s) for s in dict(UNITS)] + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(
+        os.path.join(CSRC, "*.hpp")) + [os.path.join(ROOT, "include", "glst_c.h"), os.path.abspath(__file__)]
+
+
 def up_to_date():
     if not os.path.exists(LIB):
         return False
     t = os.path.getmtime(LIB)
-    return all(os.path.getmtime(s) <= t for s in SOURCES + HEADERS)
+    return all(os.path.getmtime(s) <= t for s in inputs())
 
 
 def build(force=False, verbose=False):
     if not force and up_to_date():
         return LIB
-    cmd = [nvcc(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC", "-shared",
-           "-I" + os.path.join(ROOT, "include"), "-o", LIB + ".tmp", *SOURCES]
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    subprocess.run(cmd, check=True)
+    base = [nvcc(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC"]
+    with tempfile.TemporaryDirectory() as tmp:
+        jobs = []
+        for i, (src, defines) in enumerate(UNITS):
+            obj = os.path.join(tmp, "%d.o" % i)
+            cmd = base + defines + ["-I" + os.path.join(ROOT, "include"), "-c", os.path.join(CSRC, src), "-o", obj]
+            if verbose:
+                print(" ".join(cmd), flush=True)
+            jobs.append((obj, cmd, subprocess.Popen(cmd)))
+        failed = [cmd for _, cmd, p in jobs if p.wait() != 0]
+        if failed:
+            raise subprocess.CalledProcessError(1, failed[0])
+        cmd = base + ["-shared", "-o", LIB + ".tmp"] + [obj for obj, _, _ in jobs]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.run(cmd, check=True)
     os.replace(LIB + ".tmp", LIB)
     return LIB
 

@@ -335,7 +335,7 @@ static uint32_t tiles_per_chunk(size_t n_tiles, size_t ncell, uint32_t waves, in
   return (uint32_t)std::max<size_t>(2, std::min<size_t>(16, n_tiles / chunks));
 }
 
-// Near-field rows (kernels.cuh): nine when three rows' CTAs (one per cell
+// Near-field rows (cells.cuh): nine when three rows' CTAs (one per cell
 // and x plane) would be fewer than six per SM (up to 6^3 cells on B200:
 // 13,500-18,000 atoms on 6^3 solve 2 % faster with nine; on 7^3 grids nine
 // rows gained nothing for 24,000 atoms and cost 0.2 % for 30,000).
@@ -501,9 +501,9 @@ static glst_status set_kernel_attributes(int device, size_t shell_smem) {
   if (!(d & 1)) {
     CUDA_TRY(cudaFuncSetAttribute(dev::k_structure_factors, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dev::sf_smem_bytes(dev::kSfRadChunk, dev::kLrMaxRad * dev::kChebMaxP / 4)));
-    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range_general, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)dev::lr_smem_bytes(dev::kSfRadChunk)));
-    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CUDA_TRY(cudaFuncSetAttribute(dev::k_long_range, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kLrSmemMax));
     CUDA_TRY(cudaFuncSetAttribute(dev::k_sort_pack, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(dev::kSortCap * sizeof(uint32_t))));
@@ -837,9 +837,9 @@ static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
   if (ctas > 0x7fffffffu) return fail(GLST_ERR_SIZE, "too many cells for the gather's grid");
   const size_t smem = dev::lr_smem_bytes(h->max_rad), tab = h->lr_tab4 * sizeof(float4);
   if (smem + tab <= kLrSmemMax)
-    dev::k_long_range<true><<<(uint32_t)ctas, dev::kLrThreads, smem + tab, st>>>(lr_args(h, stage), rg.rows());
+    dev::k_long_range<<<(uint32_t)ctas, dev::kLrThreads, smem + tab, st>>>(lr_args(h, stage), rg.rows());
   else
-    dev::k_long_range<false><<<(uint32_t)ctas, dev::kLrThreads, smem, st>>>(lr_args(h, stage), rg.rows());
+    dev::k_long_range_general<<<(uint32_t)ctas, dev::kLrThreads, smem, st>>>(lr_args(h, stage), rg.rows());
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }

@@ -25,7 +25,7 @@
 // The engine's kernels, compiled again here with internal linkage (this file
 // is a translation unit of its own and must not clash with engine.cu).
 namespace {
-#include "kernels.cuh"
+#include "cells.cuh"
 namespace kdev = glst::dev;  // this file's copy of the kernels
 }  // namespace
 

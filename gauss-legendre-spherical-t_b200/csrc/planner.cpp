@@ -563,7 +563,10 @@ unsigned series_terms(const std::vector<double> &z, const double *w, unsigned ma
   double tail = 0.0;
   unsigned P = n;
   while (P > 1 && tail + omit[P - 1] <= limit) tail += omit[--P];
-  P = std::max(4u, P <= 48 ? (P + 1) / 2 * 2 : (P + 3) / 4 * 4);
+  // the lengths the kernels are compiled for: every even one that the shipped
+  // designs reach (structure factors to 48, gather to 36), few beyond
+  const unsigned every = w ? (P <= 36 ? 2 : 8) : (P <= 48 ? 2 : 4);
+  P = std::max(4u, (P + every - 1) / every * every);
   return P <= max_terms && z_max < n - 16 ? P : 0;
 }
 

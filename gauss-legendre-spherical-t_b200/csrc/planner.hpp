@@ -84,12 +84,12 @@ double rcut_from_ncell(const double box[3], const uint32_t ncell[3]);
 
 // Chebyshev (Jacobi-Anger) series of the phases of one direction,
 //   e^{-i z x} = sum_p c_p(z) (-i or 1)^{p odd} T_p(x),  |x| <= 1.
-// series_terms: number of terms (even; above 48 a multiple of 4; 0 when more
-// than max_terms would be needed).  Without weights every z of the list is
-// exact to below the rounding of an FP32 phase; with the weights w of a sum
-// over the list, the sum and its derivative are.  phase_series: the signed
-// coefficients; product_basis: their conversion to the basis T_{Bg} T_b,
-// p = Bg + b, b < B (in place).
+// series_terms: number of terms (even; above 48, with weights above 36, in
+// larger steps; 0 when more than max_terms would be needed).  Without weights
+// every z of the list is exact to below the rounding of an FP32 phase; with the
+// weights w of a sum over the list, the sum and its derivative are.
+// phase_series: the signed coefficients; product_basis: their conversion to
+// the basis T_{Bg} T_b, p = Bg + b, b < B (in place).
 unsigned series_terms(const std::vector<double> &z, const double *w, unsigned max_terms);
 void phase_series(double z, unsigned P, double *c);
 void product_basis(unsigned P, unsigned B, double *c);

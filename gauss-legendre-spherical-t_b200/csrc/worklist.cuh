@@ -5,33 +5,17 @@
 // system's own launch would use -- and a grid of resident CTAs that take the
 // items in a fixed stride (CTA b: items b, b + gridDim.x, ...).  Every item
 // runs exactly the code of the one-system kernels (the *_block functions of
-// kernels.cuh) on the same tables, so a system's results are bit for bit the
-// ones it gets alone.
+// cells.cuh, shell_sums.cuh and kernels.cuh) on the same tables, so a system's
+// results are bit for bit the ones it gets alone.  (The structure factors and
+// the gather: far_field.cu.)
 #pragma once
 
+#include "cells.cuh"
 #include "kernels.cuh"
+#include "shell_sums.cuh"
 
 namespace glst {
 namespace dev {
-
-struct SysDesc {
-  Grid g;
-  uint32_t natom, combine_blocks, part_rows, use_far, sr_rows;
-  SatArgs sat;  // shell-sum arguments (S, node tables, nodes per CTA, row stride, R)
-  const double *rx, *ry, *rz, *qc;
-  uint32_t *atom_cell, *atom_slot, *perm, *sorted_idx, *cell_count, *cell_point;
-  float4 *pk;
-  double4 *pd;
-  SfArgs sf;    // structure-factor arguments
-  LrArgs lr;    // gather arguments
-  double4 *part, *sr;
-  uint32_t *ticket;
-  double *cfx, *cfy, *cfz, *cen, *ofx, *ofy, *ofz, *oen, *block_energy, *energy;
-};
-
-struct WorkItem {
-  uint32_t sys, a, b, pad;
-};
 
 // Cell counts to zero before binning: item a = block of 1024 cells.
 __global__ void __launch_bounds__(1024) k_zero_counts_multi(const SysDesc *__restrict__ sys,
@@ -83,16 +67,6 @@ __global__ void __launch_bounds__(256) k_sort_pack_multi(const SysDesc *__restri
   }
 }
 
-// item (a, b) = (quad of direction tiles, first of sf.cells cells); always one
-// CTA per item (inside a loop over items the moments went to local memory)
-__global__ void __launch_bounds__(kSfThreads, 4) k_structure_factors_multi(const SysDesc *__restrict__ sys,
-                                                                          const WorkItem *__restrict__ items,
-                                                                          uint32_t n) {
-  const WorkItem w = items[blockIdx.x];
-  const SfArgs a = sys[w.sys].sf;
-  sf_block(a, w.a, w.b);
-}
-
 // item a = block of nb nodes; dynamic shared memory: the largest system's
 // rows, twiddles and coordinate table
 __global__ void __launch_bounds__(kSatThreads, 3) k_shell_sums_multi(const SysDesc *__restrict__ sys,
@@ -102,24 +76,6 @@ __global__ void __launch_bounds__(kSatThreads, 3) k_shell_sums_multi(const SysDe
     const WorkItem w = items[it];
     const SysDesc &d = sys[w.sys];
     shell_block<3>(d.g, d.sat, w.a);
-    __syncthreads();
-  }
-}
-
-// item (a, b) = (first of kLrWarps cells, long-range chunk); out of line, as
-// the structure factors
-__device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_warp<false>(a, cell, chunk); }
-
-__global__ void __launch_bounds__(kLrThreads, 3) k_long_range_multi(const SysDesc *__restrict__ sys,
-                                                                    const WorkItem *__restrict__ items,
-                                                                    uint32_t n) {
-  __shared__ LrArgs s_args;
-  for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const WorkItem w = items[it];
-    if (threadIdx.x == 0) s_args = sys[w.sys].lr;
-    __syncthreads();
-    const uint32_t cell = w.a + (threadIdx.x >> 5);
-    if (cell < s_args.ncell) lr_item(s_args, cell, w.b);
     __syncthreads();
   }
 }

@@ -21,7 +21,7 @@ CSRC = os.path.join(ROOT, "gauss-legendre-spherical-t_b200", "csrc")
 SOURCE = r"""
 #include <cstdio>
 #include <vector>
-#include "kernels.cuh"
+#include "cells.cuh"
 __global__ void k(const double *x, double *own, double *lib, unsigned n) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
