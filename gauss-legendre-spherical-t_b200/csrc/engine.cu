@@ -22,11 +22,13 @@
 #include "planner.hpp"
 
 using glst::Plan;
+using glst::FarLayout;
 using glst::PlanError;
 using glst::TDesignStore;
 namespace dev = glst::dev;
 
 // the planner's tables are laid out as the kernels read them
+static_assert(glst::kTileQuad == (unsigned)dev::kSfWarps && glst::kNodePad == dev::kNodeBlock, "tile layout");
 static_assert(glst::kSeriesMaxP == (unsigned)dev::kChebMaxP, "series terms");
 static_assert(glst::series_b(24) == (unsigned)dev::cheb_b(24) && glst::series_b(26) == (unsigned)dev::cheb_b(26) &&
               glst::series_row(26) == (unsigned)dev::cheb_row(26), "series tables");
@@ -127,7 +129,7 @@ struct glst_handle {
   int nsm = 148;
   uint32_t sr_rows = dev::kSrRowsPlanes;  // near-field partial-sum rows
   size_t smem_sm = 0;  // shared memory per SM, less four CTAs' system reserve
-  std::vector<uint32_t> g_node_base, g_dir_base, g_kappa_base;  // per group, internal order
+  std::vector<uint32_t> g_dir_base, g_kappa_base;  // per group, internal order
   uint32_t sat_nb = 1, sat_stride = 0;
   bool sat_xyz = true;  // shell-sum cell-coordinate table in shared memory
   uint32_t combine_blocks = 1;
@@ -182,12 +184,7 @@ struct glst_handle {
   // sums, gather over a contiguous range of whole directions), so S and R
   // hold one stage's nodes; a large system needs a fraction of the C x K
   // operand the whole node set would take.
-  struct FarRange {
-    uint32_t kb, ke;          // nodes of one stage
-    uint32_t u0, u1;          // direction tiles of the same nodes
-    uint32_t tpc;             // tiles per long-range chunk
-    uint32_t rows() const { return (u1 - u0 + tpc - 1) / tpc; }  // long-range chunks
-  };
+  using FarRange = FarLayout::Stage;
   std::vector<FarRange> ranges;
   uint32_t stage_kmax = 0;    // nodes of the largest stage (S and R hold this many)
   uint32_t part_rows = 1;     // rows of `part` (chunks of the largest stage)
@@ -324,15 +321,12 @@ static uint64_t stage_budget() {
   return b;
 }
 
-// Direction tiles per gather chunk (a warp's work: a cell and a chunk).  Every
-// chunk writes a partial row of 32 bytes per atom that the combine reads back
-// and stages the cell's atoms, so at least two tiles, and no
-// more chunks than fill the GPU with `waves` waves of warps; at most 16 tiles, so that the last wave stays
-// short on large grids.
-static uint32_t tiles_per_chunk(size_t n_tiles, size_t ncell, uint32_t waves, int nsm) {
-  const size_t slots = (size_t)nsm * 12;
-  const size_t chunks = std::max<size_t>(1, ((size_t)waves * slots + ncell - 1) / ncell);
-  return (uint32_t)std::max<size_t>(2, std::min<size_t>(16, n_tiles / chunks));
+// Shell sums take their tables from global memory: a node's table exceeds the
+// shared memory, an axis the packed cell coordinates, or
+// GLST_GLOBAL_SHELL_SUMS=1 (read when a handle is set up).
+static bool global_shell_sums(const Plan &p, size_t per_node, size_t budget) {
+  const char *force = std::getenv("GLST_GLOBAL_SHELL_SUMS");
+  return p.n[0] >= 1024 || p.n[1] >= 1024 || p.n[2] >= 1024 || per_node > budget || (force && force[0] == '1');
 }
 
 // Near-field rows (cells.cuh): nine when three rows' CTAs (one per cell
@@ -349,103 +343,23 @@ static uint32_t pow2_floor(uint32_t v) {
   return p;
 }
 
-// Node stages, direction tiles and long-range chunks.  The nodes are cut into
-// tiles of up to 32 directions of one group, one warp each of the structure
-// factors and the gather.  First this handle's tiles: all of them, or -- when
-// the system is split over several devices -- a contiguous run holding about
-// K / nshards nodes (the reference splits its node list into contiguous
-// per-GPU ranges, src/glst_force.cu:276-293).  Then stages: contiguous runs
-// of tiles of about equal node count, as many as the S + R budget needs.
-// Then, per stage, long-range chunks: runs of tiles_per_chunk tiles.  (FP32
-// sums stay within a tile, everything across tiles is FP64, so neither the
-// shards nor the chunks change a result beyond FP64 rounding.)
+// The handle's tiles, node stages and gather chunks (far_layout), and the
+// buffers whose size they give.
 static glst_status build_tiles(glst_handle *h, bool in_arena = false) {
   const Plan &p = h->plan;
-  const size_t C = p.ncell, Kall = p.has_far ? p.K() : 0, N = p.natom;
-  struct Tile {
-    uint32_t gi, j, n;  // group, first direction within the group, directions
-    uint32_t k, ke;     // nodes (internal order)
-  };
-  std::vector<Tile> all;
-  for (size_t gi = 0; gi < (Kall ? p.groups.size() : 0); gi++) {
-    const auto &g = p.groups[gi];
-    for (uint32_t j = 0; j < g.n_dir; j += 32) {
-      const uint32_t n = std::min(32u, g.n_dir - j), k = h->g_node_base[gi] + j * g.n_radial;
-      all.push_back({(uint32_t)gi, j, n, k, k + n * g.n_radial});
-    }
-  }
-  const uint64_t kpad_sys = (Kall + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
-  const uint64_t nst_sys = std::max<uint64_t>(1, (C * kpad_sys * 16 + stage_budget() - 1) / stage_budget());
-  // the whole system's chunk size; a shard takes whole chunks of it
-  const uint32_t tpc_sys = tiles_per_chunk(all.size() / nst_sys, C, h->lr_waves, h->nsm);
-  // this handle's tiles [d0, d1)
-  size_t d0 = 0, d1 = all.size();
-  if (h->nshards > 1 && Kall) {
-    bool any = false;
-    for (size_t i = 0; i < all.size(); i += tpc_sys) {
-      const size_t e = std::min(all.size(), i + tpc_sys);
-      const uint64_t mid = ((uint64_t)all[i].k + all[e - 1].ke) / 2;
-      if (mid * h->nshards / Kall == h->shard) {
-        if (!any) d0 = i;
-        d1 = e;
-        any = true;
-      }
-    }
-    if (!any) d0 = d1 = 0;
-  }
-  const uint32_t kb = d0 < d1 ? all[d0].k : 0;
-  h->k_begin = kb;
-  h->K = (d0 < d1 ? all[d1 - 1].ke : 0) - kb;
-  const uint64_t K = h->K;
-  // stages
-  const uint64_t kpad_all = (K + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
-  uint64_t nst = std::max<uint64_t>(1, (C * kpad_all * 16 + stage_budget() - 1) / stage_budget());
-  nst = std::min<uint64_t>(nst, std::max<size_t>(1, d1 - d0));
+  const size_t N = p.natom;
+  const FarLayout lay = glst::far_layout(p, h->shard, h->nshards, h->lr_waves, h->nsm, stage_budget());
+  h->k_begin = lay.k_begin;
+  h->K = lay.K;
+  h->ranges = lay.stages;
+  h->stage_kmax = lay.stage_kmax;
+  h->part_rows = lay.part_rows;
   std::vector<dev::DirTile> tiles;
-  h->ranges.clear();
-  h->stage_kmax = 0;
-  h->part_rows = 1;
-  size_t i = d0;
-  for (uint64_t st = 0; st < nst && i < d1; st++) {
-    const uint64_t target_end = kb + K * (st + 1) / nst;  // node where this stage should end
-    size_t e = i + 1;
-    while (e < d1 && (st + 1 == nst || all[e].k < target_end)) e++;
-    glst_handle::FarRange rg{};
-    rg.kb = all[i].k - kb;
-    rg.ke = all[e - 1].ke - kb;
-    rg.u0 = (uint32_t)tiles.size();
-    rg.tpc = h->nshards > 1 ? tpc_sys : tiles_per_chunk(e - i, C, h->lr_waves, h->nsm);
-    // a group's tiles are padded to whole quads (a structure-factor CTA's
-    // warps share one group's table)
-    const size_t first = i;
-    auto pad_quad = [&]() {
-      while ((tiles.size() - rg.u0) % dev::kSfWarps) {
-        dev::DirTile u = tiles.back();
-        u.n_dir = 0;
-        tiles.push_back(u);
-      }
-    };
-    for (; i < e; i++) {
-      const uint32_t gi = all[i].gi;
-      if (i > first && gi != all[i - 1].gi) pad_quad();
-      dev::DirTile u{};
-      u.node_begin = all[i].k - kb;
-      u.dir_begin = h->g_dir_base[gi] + all[i].j;
-      u.n_dir = all[i].n;
-      u.n_rad = p.groups[gi].n_radial;
-      u.P = h->g_sf_P[gi];
-      u.tab = h->g_sf_tab[gi];
-      u.kappa_begin = h->g_kappa_base[gi];
-      u.lr_P = h->g_lr_P[gi];
-      u.lr_tab = h->g_lr_tab[gi];
-      tiles.push_back(u);
-    }
-    pad_quad();
-    rg.u1 = (uint32_t)tiles.size();
-    h->stage_kmax = std::max(h->stage_kmax, rg.ke - rg.kb);
-    h->part_rows = std::max(h->part_rows, rg.rows());
-    h->ranges.push_back(rg);
-  }
+  tiles.reserve(lay.tiles.size());
+  for (const auto &t : lay.tiles)
+    tiles.push_back(dev::DirTile{t.kb - lay.k_begin, h->g_dir_base[t.group] + t.dir, t.n_dir, p.groups[t.group].n_radial,
+                                 h->g_sf_P[t.group], h->g_sf_tab[t.group], h->g_kappa_base[t.group],
+                                 h->g_lr_P[t.group], h->g_lr_tab[t.group]});
   // rows a later stage writes beyond what stage 0 writes start at zero
   h->part_zero_from = h->ranges.empty() ? h->part_rows : h->ranges[0].rows();
   h->n_tiles = (uint32_t)tiles.size();
@@ -555,7 +469,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   // reference's is group -> radial -> direction, src/cubature.cu:120-145).
   // Nodes and weights are rounded to CT first, as the reference stores them
   // (src/cubature.cu:138-141).
-  std::vector<uint32_t> kappa_base, dir_base, node_base;
+  std::vector<uint32_t> kappa_base, dir_base;
   std::vector<double4> n64(K);
   std::vector<uint32_t> radii(K);
   std::vector<float4> dirs;
@@ -585,7 +499,6 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
       h->g_lr_tab.push_back((uint32_t)cheb_lr.size());
       cheb_lr.insert(cheb_lr.end(), g.lr_tab.begin(), g.lr_tab.end());
       dir_base.push_back((uint32_t)dirs.size());
-      node_base.push_back(ibase);
       for (unsigned r = 0; r < g.n_radial; r++) kap.push_back((float)g.kappa[r]);
       nquad += (g.n_radial + 3) / 4;
       if (nquad > dev::kLrMaxQuads)
@@ -659,9 +572,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
     const size_t xyz_bytes = (C * 4 + 15) & ~size_t(15);
     h->sat_xyz = per_node + xyz_bytes <= smem_total;
     const size_t budget = h->sat_xyz ? smem_total - xyz_bytes : smem_total;
-    const char *force_global = std::getenv("GLST_GLOBAL_SHELL_SUMS");
-    h->gsat = p.n[0] >= 1024 || p.n[1] >= 1024 || p.n[2] >= 1024 || per_node > budget ||
-              (force_global && force_global[0] == '1');
+    h->gsat = global_shell_sums(p, per_node, budget);
     h->sat_per_node = per_node;
     h->sat_budget = budget;
     GLST_TRY(set_kernel_attributes(h->device, smem_total));
@@ -676,7 +587,6 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
                           : pow2_floor((uint32_t)std::max<size_t>(1, std::min<size_t>(8, budget / per_node)));
     // ... but no fewer than four CTAs per SM's worth of node blocks (few nodes)
     while (h->sat_nb > 8 && (K + h->sat_nb - 1) / h->sat_nb < 4 * (size_t)nsm) h->sat_nb >>= 1;
-    h->g_node_base = node_base;
     h->g_dir_base = dir_base;
     h->g_kappa_base = kappa_base;
     {
@@ -2032,35 +1942,26 @@ struct SrvSlot {
   struct glst_server *owner = nullptr;
 };
 
-// Device bytes a handle for `p` will hold (an upper bound of setup's sizes).
+// Device bytes a handle for `p` will hold (an upper bound of setup's sizes):
+// tiles, stages and partial rows are set-up's own (far_layout, with the shape's
+// tuned waves), the rest is counted generously.
 uint64_t estimate_bytes(const Plan &p, int nsm) {
   const uint64_t N = p.natom, C = p.ncell, K = p.has_far ? p.K() : 0;
-  uint64_t b = N * (4 * 4 + 16 + 32 + 32 * (uint64_t)sr_rows_for(C, nsm) + 8 * 8 + 32) + C * 8 + 4096;
+  const uint64_t combine = (N + dev::kCombineAtoms - 1) / dev::kCombineAtoms;
+  uint64_t b = N * (4 * 4 + 16 + 32 + 32 * (uint64_t)sr_rows_for(C, nsm) + 8 * 8 + 32) + C * 8 + combine * 8 + 4096;
   if (K) {
-    const uint64_t kpad = (K + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
-    const uint64_t nst = std::max<uint64_t>(1, (C * kpad * 16 + stage_budget() - 1) / stage_budget());
-    // the largest stage: ~K / stages, plus up to one tile of directions
-    // (stages end on tile boundaries)
+    const uint32_t waves = tuned(p, (uint32_t)K).lr_waves;
+    const FarLayout lay = glst::far_layout(p, 0, 1, waves ? waves : kLrWaves, nsm, stage_budget());
     uint32_t max_nr = 1;
     for (const auto &g : p.groups) max_nr = std::max(max_nr, g.n_radial);
-    const uint64_t stage_k =
-        nst == 1 ? kpad : std::min<uint64_t>(kpad, (K + nst - 1) / nst + 32ull * max_nr);
-    // direction tiles (a stage holds no more than all), and a stage's gather
-    // chunks (partial rows)
-    uint64_t n_tiles = 0;
-    for (const auto &g : p.groups) n_tiles += (g.n_dir + 127) / 128 * 4;
-    uint64_t chunks = 1;
-    for (uint64_t t = std::max<uint64_t>(1, n_tiles / nst); t <= n_tiles / nst + 8; t++) {
-      const uint64_t tpc = tiles_per_chunk(t, C, kLrWaves, nsm);
-      chunks = std::max(chunks, (t + tpc - 1) / tpc + 1);
-    }
-    const uint64_t stage_kpad = (stage_k + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
+    const uint64_t kpad = ((uint64_t)lay.stage_kmax + dev::kNodeBlock - 1) / dev::kNodeBlock * dev::kNodeBlock;
     b += K * (32 + 4 + 16 + 4) + (uint64_t)max_nr * p.groups.size() * dev::kChebMaxP * 8 +
-         (n_tiles + 8 * nst) * sizeof(dev::DirTile) + C * stage_kpad * (8 + 8) + chunks * N * 32;
-    // global-memory shell-sum tables (grids whose per-node table exceeds the
-    // shared memory of a CTA): 64 MB or one block, and the twiddles
-    if ((C + 9 + p.n[0] + p.n[1] + p.n[2]) * 16 > (200ull << 10))
-      b += std::max<uint64_t>(64ull << 20, C * dev::kNodeBlock * 16) + stage_kpad * (p.n[0] + p.n[1] + p.n[2]) * 16;
+         lay.tiles.size() * sizeof(dev::DirTile) + C * kpad * (8 + 8) + lay.part_rows * N * 32;
+    // global-memory shell-sum tables (at the latest where a node's table
+    // exceeds the shared memory of a CTA): 64 MB or one block, and the twiddles
+    const uint64_t axes = (uint64_t)p.n[0] + p.n[1] + p.n[2];
+    if (global_shell_sums(p, (C + 9 + axes) * 16, 200u << 10))
+      b += std::max<uint64_t>(64ull << 20, C * dev::kNodeBlock * 16) + kpad * axes * 16;
   }
   return b + 64 * 16 * 64;  // per-buffer allocation granularity
 }

@@ -511,6 +511,82 @@ Plan make_plan(uint32_t natom, double tol, const double box[3], double rcut,
   return p;
 }
 
+// ------------------------------------------------------- tiles, stages, chunks
+// Tiles per gather chunk (a warp's work: a cell and a chunk).  Every chunk
+// writes a partial row of 32 bytes per atom that the combine reads back and
+// stages the cell's atoms, so at least two tiles, and no more chunks than fill
+// the GPU with `waves` waves of warps; at most 16 tiles, so that the last wave
+// stays short on large grids.
+static uint32_t tiles_per_chunk(size_t n_tiles, size_t ncell, uint32_t waves, int nsm) {
+  const size_t slots = static_cast<size_t>(nsm) * 12;
+  const size_t chunks = std::max<size_t>(1, (static_cast<size_t>(waves) * slots + ncell - 1) / ncell);
+  return static_cast<uint32_t>(std::max<size_t>(2, std::min<size_t>(16, n_tiles / chunks)));
+}
+
+FarLayout far_layout(const Plan &p, uint32_t shard, uint32_t nshards, uint32_t waves, int nsm, uint64_t stage_bytes) {
+  FarLayout out;
+  const uint64_t C = p.ncell, Kall = p.has_far ? p.K() : 0;
+  std::vector<FarLayout::Tile> all;
+  uint32_t base = 0;
+  for (size_t gi = 0; gi < (Kall ? p.groups.size() : 0); gi++) {
+    const auto &g = p.groups[gi];
+    for (uint32_t j = 0; j < g.n_dir; j += kTileDirs) {
+      const uint32_t n = std::min<uint32_t>(kTileDirs, g.n_dir - j), k = base + j * g.n_radial;
+      all.push_back({static_cast<uint32_t>(gi), j, n, k, k + n * g.n_radial});
+    }
+    base += g.n_dir * g.n_radial;
+  }
+  auto stage_count = [&](uint64_t K) {
+    const uint64_t kpad = (K + kNodePad - 1) / kNodePad * kNodePad;
+    return std::max<uint64_t>(1, (C * kpad * 16 + stage_bytes - 1) / stage_bytes);
+  };
+  // the whole system's chunk size; a shard takes whole chunks of it
+  const uint32_t tpc_all = tiles_per_chunk(all.size() / stage_count(Kall), C, waves, nsm);
+  size_t d0 = 0, d1 = all.size();  // the shard's tiles
+  if (nshards > 1 && Kall) {
+    d1 = 0;
+    for (size_t i = 0; i < all.size(); i += tpc_all) {
+      const size_t e = std::min<size_t>(all.size(), i + tpc_all);
+      const uint64_t mid = (static_cast<uint64_t>(all[i].kb) + all[e - 1].ke) / 2;
+      if (mid * nshards / Kall != shard) continue;
+      if (d1 == 0) d0 = i;
+      d1 = e;
+    }
+    if (d1 == 0) d0 = 0;
+  }
+  out.k_begin = d0 < d1 ? all[d0].kb : 0;
+  out.K = (d0 < d1 ? all[d1 - 1].ke : 0) - out.k_begin;
+  const uint64_t nst = std::min<uint64_t>(stage_count(out.K), std::max<size_t>(1, d1 - d0));
+  size_t i = d0;
+  for (uint64_t st = 0; st < nst && i < d1; st++) {
+    const uint64_t target_end = out.k_begin + static_cast<uint64_t>(out.K) * (st + 1) / nst;  // where it should end
+    size_t e = i + 1;
+    while (e < d1 && (st + 1 == nst || all[e].kb < target_end)) e++;
+    FarLayout::Stage sg{};
+    sg.kb = all[i].kb - out.k_begin;
+    sg.ke = all[e - 1].ke - out.k_begin;
+    sg.u0 = static_cast<uint32_t>(out.tiles.size());
+    sg.tpc = nshards > 1 ? tpc_all : tiles_per_chunk(e - i, C, waves, nsm);
+    auto pad_quad = [&]() {
+      while ((out.tiles.size() - sg.u0) % kTileQuad) {
+        FarLayout::Tile u = out.tiles.back();
+        u.n_dir = 0;
+        out.tiles.push_back(u);
+      }
+    };
+    for (const size_t first = i; i < e; i++) {
+      if (i > first && all[i].group != all[i - 1].group) pad_quad();
+      out.tiles.push_back(all[i]);
+    }
+    pad_quad();
+    sg.u1 = static_cast<uint32_t>(out.tiles.size());
+    out.stage_kmax = std::max(out.stage_kmax, sg.ke - sg.kb);
+    out.part_rows = std::max(out.part_rows, sg.rows());
+    out.stages.push_back(sg);
+  }
+  return out;
+}
+
 // ------------------------------------------------------- phase series
 // Bessel functions J_0(z) .. J_{n-1}(z) by Miller's backward recurrence,
 // normalised with J_0 + 2 (J_2 + J_4 + ...) = 1.

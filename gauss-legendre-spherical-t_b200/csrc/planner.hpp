@@ -82,6 +82,42 @@ Plan make_plan(uint32_t natom, double tol, const double box[3], double rcut,
                int ct_float, TDesignStore &store);
 double rcut_from_ncell(const double box[3], const uint32_t ncell[3]);
 
+// How a handle works through its nodes (internal order: group -> direction ->
+// radial).  They are cut into tiles of up to kTileDirs directions of one
+// group, one warp each of the structure factors and the gather.  A shard of a
+// system split over several devices takes a contiguous run of tiles (the
+// reference splits its node list into contiguous per-GPU ranges,
+// src/glst_force.cu:276-293).  Its tiles are run in stages of about equal node
+// count, as many as keep S + R within the stage budget, and a stage's in gather
+// chunks of tpc tiles, each with a partial row of 32 bytes per atom.  A group's
+// tiles in a stage are padded to whole quads (a structure-factor CTA's warps
+// share one group's table).  FP32 sums stay within a tile, everything across
+// tiles is FP64, so neither shards nor stages nor chunks change a result beyond
+// FP64 rounding.
+constexpr unsigned kTileDirs = 32, kTileQuad = 4, kNodePad = 32;  // nodes of S and R are padded to kNodePad
+
+struct FarLayout {
+  struct Tile {
+    uint32_t group, dir, n_dir;  // group, first direction within it, directions (0: padding)
+    uint32_t kb, ke;             // nodes of the system
+  };
+  struct Stage {
+    uint32_t kb, ke;             // nodes of the stage, from k_begin on
+    uint32_t u0, u1;             // its tiles
+    uint32_t tpc;                // tiles per gather chunk
+    uint32_t rows() const { return (u1 - u0 + tpc - 1) / tpc; }  // gather chunks
+  };
+  std::vector<Tile> tiles;
+  std::vector<Stage> stages;
+  uint32_t k_begin = 0, K = 0;   // the shard's nodes
+  uint32_t stage_kmax = 0;       // nodes of the largest stage
+  uint32_t part_rows = 1;        // gather chunks of the largest stage
+};
+
+// `waves`: waves of gather warps to cut a stage's chunks for; `nsm`: SMs;
+// `stage_bytes`: of S + R.
+FarLayout far_layout(const Plan &p, uint32_t shard, uint32_t nshards, uint32_t waves, int nsm, uint64_t stage_bytes);
+
 // Chebyshev (Jacobi-Anger) series of the phases of one direction,
 //   e^{-i z x} = sum_p c_p(z) (-i or 1)^{p odd} T_p(x),  |x| <= 1.
 // series_terms: number of terms (even; above 48, with weights above 36, in
