@@ -540,19 +540,15 @@ FarLayout far_layout(const Plan &p, uint32_t shard, uint32_t nshards, uint32_t w
     const uint64_t kpad = (K + kNodePad - 1) / kNodePad * kNodePad;
     return std::max<uint64_t>(1, (C * kpad * 16 + stage_bytes - 1) / stage_bytes);
   };
-  // the whole system's chunk size; a shard takes whole chunks of it
-  const uint32_t tpc_all = tiles_per_chunk(all.size() / stage_count(Kall), C, waves, nsm);
-  size_t d0 = 0, d1 = all.size();  // the shard's tiles
+  // the shard's tiles: those whose middle node lies in its share of the nodes
+  size_t d0 = 0, d1 = all.size();
   if (nshards > 1 && Kall) {
-    d1 = 0;
-    for (size_t i = 0; i < all.size(); i += tpc_all) {
-      const size_t e = std::min<size_t>(all.size(), i + tpc_all);
-      const uint64_t mid = (static_cast<uint64_t>(all[i].kb) + all[e - 1].ke) / 2;
-      if (mid * nshards / Kall != shard) continue;
-      if (d1 == 0) d0 = i;
-      d1 = e;
-    }
-    if (d1 == 0) d0 = 0;
+    auto owner = [&](const FarLayout::Tile &t) {
+      return (static_cast<uint64_t>(t.kb) + t.ke) / 2 * nshards / Kall;
+    };
+    while (d0 < all.size() && owner(all[d0]) < shard) d0++;
+    d1 = d0;
+    while (d1 < all.size() && owner(all[d1]) == shard) d1++;
   }
   out.k_begin = d0 < d1 ? all[d0].kb : 0;
   out.K = (d0 < d1 ? all[d1 - 1].ke : 0) - out.k_begin;
@@ -566,7 +562,7 @@ FarLayout far_layout(const Plan &p, uint32_t shard, uint32_t nshards, uint32_t w
     sg.kb = all[i].kb - out.k_begin;
     sg.ke = all[e - 1].ke - out.k_begin;
     sg.u0 = static_cast<uint32_t>(out.tiles.size());
-    sg.tpc = nshards > 1 ? tpc_all : tiles_per_chunk(e - i, C, waves, nsm);
+    sg.tpc = tiles_per_chunk(e - i, C, waves, nsm);
     auto pad_quad = [&]() {
       while ((out.tiles.size() - sg.u0) % kTileQuad) {
         FarLayout::Tile u = out.tiles.back();
