@@ -120,13 +120,15 @@ __global__ void k_scatter(const uint32_t *__restrict__ atom_cell,
 // src/glst_force.cu:510-517).  Then writes the packets.  A CTA takes one cell
 // (bitonic sort), or on sparse grids kSortCells cells: one warp each for cells
 // of up to kSortWarpCap atoms, an atom's place being the number of smaller
-// indices, then the whole CTA for each larger one.  Launched with 32
-// kSortCells threads and kSortCap u32 of dynamic shared memory.
-constexpr uint32_t kSortCells = 8;
-constexpr uint32_t kSortWarpCap = 32;
-__host__ __device__ inline uint32_t sort_cells(uint32_t natom, uint32_t ncell) {  // cells per CTA
-  return natom / ncell <= 16 ? kSortCells : 1u;
-}
+// indices, then the whole CTA for each larger one.  A CTA's cells are far apart
+// in the grid, so that a cluster's full cells, which lie together, go to
+// different CTAs.  Launched with 32 kSortCells threads and kSortCap u32 of
+// dynamic shared memory.
+// Measured, a warp per cell against a CTA per cell: 26^3 cells of 12 / 28 / 60 /
+// 87 atoms 16 / 30 / 67 / 130 us against 67 / 82 / 128 / 192; 7^3 cells 11 / 11 /
+// 13 / 15 against 11 / 13 / 14 / 14.  (Up to 32 atoms only, the rest by the CTA:
+// 7^3 cells of 28 atoms 24, of 40 atoms 40.)
+constexpr uint32_t kSortWarpCap = 128;
 __device__ __forceinline__ void pack_atom(uint32_t slot, uint32_t a, double cx, double cy, double cz,
                                           const double *__restrict__ rx, const double *__restrict__ ry,
                                           const double *__restrict__ rz, const double *__restrict__ qc,
@@ -221,7 +223,7 @@ __device__ __forceinline__ void sort_pack_cells(const uint32_t *__restrict__ per
     return;
   }
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t cell = bx * kSortCells + warp;
+  const uint32_t stride = (g.ncell + kSortCells - 1) / kSortCells, cell = bx + warp * stride;
   const uint32_t cnt = cell < g.ncell ? cell_count[cell] : 0u;
   if (cnt > 0 && cnt <= kSortWarpCap) {
     const uint32_t start = cell_point[cell];
@@ -240,7 +242,7 @@ __device__ __forceinline__ void sort_pack_cells(const uint32_t *__restrict__ per
   }
   if (!__syncthreads_or(cnt > kSortWarpCap)) return;
   for (uint32_t w = 0; w < kSortCells; w++) {
-    const uint32_t c = bx * kSortCells + w;
+    const uint32_t c = bx + w * stride;
     if (c < g.ncell && cell_count[c] > kSortWarpCap) {
       sort_pack_block(perm, cell_count, cell_point, g, atom_cell, natom, rx, ry, rz, qc, sorted_idx, pk, pd, c);
       __syncthreads();
@@ -420,19 +422,6 @@ k_short_range(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_
               const uint32_t *__restrict__ cell_point, Grid g, uint32_t natom,
               double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell, uint32_t max_width) {
   sr_block(pd, cell_count, cell_point, g, natom, sr, rows, warps_per_cell, max_width, blockIdx.x, blockIdx.y);
-}
-
-// Lanes per chunk, at most: the widest chunks of which there are still 2,048
-// (about four warps for each of the GPU's schedulers), else 8 atoms wide.
-__host__ __device__ inline uint32_t sr_width(uint32_t natom, uint32_t rows) {
-  const uint64_t lanes = (uint64_t)natom * rows;
-  return lanes >= 2048u * 32u ? 32u : lanes >= 2048u * 16u ? 16u : 8u;
-}
-
-// Warps per cell for a mean number of atoms per cell.
-__host__ __device__ inline uint32_t sr_warps_per_cell(uint32_t natom, uint32_t ncell, uint32_t width) {
-  const uint32_t mean = natom / ncell;
-  return 4 * mean <= 3 * width ? 1u : 4 * mean <= 7 * width ? 2u : 4u;
 }
 
 // ----------------------------------------------------------------------------

@@ -668,7 +668,7 @@ static dev::SfArgs sf_args(const glst_handle *h, const glst_handle::FarRange &rg
   return dev::SfArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
                      reinterpret_cast<const float4 *>(h->cheb), h->S, h->R, h->cheb_scale, h->plan.ncell,
                      rg.u1 - rg.u0, h->max_rad, rg.kb, h->sf_tab4,
-                     dev::sf_cells(h->plan.natom, h->plan.ncell)};
+                     dev::sf_cells(h->plan.natom, h->plan.ncell, (rg.u1 - rg.u0) / dev::kSfWarps)};
 }
 
 static glst_status sf_stage(glst_handle *h, const glst_handle::FarRange &rg, cudaStream_t st) {
@@ -1542,7 +1542,7 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
       if (!h->K || !h->plan.natom) return;
       const uint32_t quads = h->n_tiles / dev::kSfWarps;
       gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad, h->sf_tab4));
-      for (uint32_t c = 0; c < h->plan.ncell; c += dev::sf_cells(h->plan.natom, h->plan.ncell))
+      for (uint32_t c = 0; c < h->plan.ncell; c += dev::sf_cells(h->plan.natom, h->plan.ncell, quads))
         for (uint32_t u = 0; u < quads; u++) items.push_back({w, u, c, 0});
     });
     each(glst_batch::kShell, [&](uint32_t w, glst_handle *h) {

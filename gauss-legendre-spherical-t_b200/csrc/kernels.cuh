@@ -129,11 +129,6 @@ struct SfArgs {
   uint32_t cells;      // cells per CTA
 };
 
-// Cells per structure-factor CTA: one (four cost 5 % on water10k, 40 % on 1,000
-// waters), but eight where a cell's few atoms take less than copying the table
-// (26^3 cells of 6 atoms: 0.32 ms with one, 0.24 with four).
-__host__ __device__ inline uint32_t sf_cells(uint32_t natom, uint32_t ncell) { return natom / ncell <= 16 ? 8u : 1u; }
-
 // Rows of the staged results are an odd number of float2 apart (bank spread).
 __host__ __device__ constexpr uint32_t sf_row(uint32_t rc) { return rc | 1u; }
 

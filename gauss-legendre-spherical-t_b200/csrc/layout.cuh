@@ -55,5 +55,40 @@ struct SatArgs {
   float2 *R;
 };
 
+// ----------------------------------------------------------------------------
+// How the work over cells is divided (host and device).
+constexpr uint32_t kSms = 148;        // B200
+constexpr uint32_t kSortCells = 8;    // cells per CTA, sparse grids
+
+// Cells per CTA of the sort.
+__host__ __device__ inline uint32_t sort_cells(uint32_t natom, uint32_t ncell) {
+  return natom / ncell <= 16 ? kSortCells : 1u;
+}
+
+// Cells per structure-factor CTA, for `quads` quads of direction tiles.  The
+// group's table is copied once per CTA, so more cells help where they hold few
+// atoms and CTAs are still many: eight from 28 CTAs per SM on, four from 24
+// (12 at eight cells each).  Measured, one / four / eight cells, us: 26^3 cells
+// of 5 atoms at 1e-3 320 / 241 / 231 (11,000 CTAs of eight cells); 16^3 70 / 60
+// / 64 (2,000); 8^3 at the default order 222 / 223 / 239 (1,900); 6^3 93 / 100 /
+// 117 (700); 3^3 20 / 32 / 55 (50).
+__host__ __device__ inline uint32_t sf_cells(uint32_t natom, uint32_t ncell, uint32_t quads) {
+  const uint64_t ctas = (uint64_t)ncell * quads / 8;
+  return natom / ncell > 16 || ctas < 12 * kSms ? 1u : ctas < 28 * kSms ? 4u : 8u;
+}
+
+// Lanes per chunk, at most: the widest chunks of which there are still 2,048
+// (about four warps for each of the GPU's schedulers), else 8 atoms wide.
+__host__ __device__ inline uint32_t sr_width(uint32_t natom, uint32_t rows) {
+  const uint64_t lanes = (uint64_t)natom * rows;
+  return lanes >= 2048u * 32u ? 32u : lanes >= 2048u * 16u ? 16u : 8u;
+}
+
+// Warps per cell for a mean number of atoms per cell.
+__host__ __device__ inline uint32_t sr_warps_per_cell(uint32_t natom, uint32_t ncell, uint32_t width) {
+  const uint32_t mean = natom / ncell;
+  return 4 * mean <= 3 * width ? 1u : 4 * mean <= 7 * width ? 2u : 4u;
+}
+
 }  // namespace dev
 }  // namespace glst
