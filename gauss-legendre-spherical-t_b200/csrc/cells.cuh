@@ -55,10 +55,16 @@ __global__ void k_bin(const double *__restrict__ rx, const double *__restrict__ 
 }
 
 // K_scan: exclusive offsets of the cell counts (one CTA of 1024 threads, four
-// consecutive cells per thread and step: 26^3 cells in 5 steps instead of 18).
+// consecutive cells per thread and step: 26^3 cells in 5 steps instead of 18),
+// and the pieces of cells of more than `cap` atoms (layout.cuh; pieces may be null).
+// The pieces' order varies, what is computed of a piece does not depend on it.
 __device__ __forceinline__ void scan_body(const uint32_t *__restrict__ cell_count, uint32_t ncell,
-                                          uint32_t *__restrict__ cell_point) {
+                                          uint32_t *__restrict__ cell_point, uint32_t cap, uint2 *__restrict__ pieces,
+                                          uint32_t *__restrict__ n_pieces) {
   __shared__ uint32_t warp_sums[32];
+  __shared__ uint32_t s_pieces;
+  if (threadIdx.x == 0) s_pieces = 0;
+  __syncthreads();
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   uint32_t carry = 0;
   for (uint32_t base = 0; base < ncell; base += 4 * blockDim.x) {
@@ -88,14 +94,20 @@ __device__ __forceinline__ void scan_body(const uint32_t *__restrict__ cell_coun
     for (int u = 0; u < 4; u++) {
       if (c + u < ncell) cell_point[c + u] = p;
       p += v[u];
+      if (pieces && v[u] > cap) {
+        const uint32_t n = (v[u] - cap + kPieceAtoms - 1) / kPieceAtoms, at = atomicAdd(&s_pieces, n);
+        for (uint32_t t = 0; t < n; t++) pieces[at + t] = make_uint2(c + u, cap + t * kPieceAtoms);
+      }
     }
     __syncthreads();  // warp_sums is rewritten
   }
+  if (pieces && threadIdx.x == 0) *n_pieces = s_pieces;
 }
 
 __global__ void k_scan(const uint32_t *__restrict__ cell_count, uint32_t ncell,
-                       uint32_t *__restrict__ cell_point) {
-  scan_body(cell_count, ncell, cell_point);
+                       uint32_t *__restrict__ cell_point, uint32_t cap, uint2 *__restrict__ pieces,
+                       uint32_t *__restrict__ n_pieces) {
+  scan_body(cell_count, ncell, cell_point, cap, pieces, n_pieces);
 }
 
 __device__ __forceinline__ void scatter_block(const uint32_t *__restrict__ atom_cell,
@@ -279,9 +291,9 @@ __global__ void k_sort_pack(const uint32_t *__restrict__ perm,
 // three of an x plane, and writes its own partial row of per-atom sums, summed
 // by k_combine in a fixed order.
 // Measured (one thread per atom and CTA barriers between cells before):
-// water10k 0.291 -> 0.220 ms, 168 atoms per cell 0.400 -> 0.285 ms, 26^3 cells
-// of 6 atoms 0.485 -> 0.101 ms, 3,000 atoms on 4^3 cells 0.067 -> 0.052 ms, a
-// million atoms 4.44 -> 4.03 ms.
+// water10k 0.291 -> 0.187 ms, 168 atoms per cell 0.400 -> 0.258 ms, 26^3 cells
+// of 6 atoms 0.485 -> 0.102 ms, 3,000 atoms on 4^3 cells 0.067 -> 0.045 ms, a
+// million atoms 4.44 -> 4.03 ms (not measured again since).
 constexpr int kSrThreads = 128;
 constexpr int kSrWarps = kSrThreads / 32;
 constexpr int kSrRowsPlanes = 3;
@@ -346,23 +358,21 @@ __device__ __forceinline__ void sr_batch(const double4 *s_at, uint32_t n, uint32
   }
 }
 
-// A warp's share of a cell: chunks chunk0, chunk0 + warps_per_cell, ... of its
-// atoms against row `row` of `rows`.
+// A warp's share of a cell: its atoms first, first + step, ... (`width` of them
+// each time) below `end` against row `row` of `rows`.
 __device__ __forceinline__ void sr_warp(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
                                         const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
                                         double4 *__restrict__ sr, uint32_t rows, uint32_t row, uint32_t cell,
-                                        uint32_t chunk0, uint32_t warps_per_cell, uint32_t max_width,
+                                        uint32_t first, uint32_t step, uint32_t end, uint32_t width,
                                         double4 *s_at) {
-  const uint32_t cnt = cell_count[cell];
-  const uint32_t width = min(max_width, cnt > 16 ? 32u : cnt > 8 ? 16u : 8u), groups = 32u / width;
-  if (chunk0 * width >= cnt) return;
+  const uint32_t groups = 32u / width;
   const uint32_t lane = threadIdx.x & 31u, sub = lane / width, li = lane & (width - 1u);
   const uint32_t start = cell_point[cell];
   const int ix = cell / (g.ny * g.nz), iy = (cell / g.nz) % g.ny, iz = cell % g.nz;
   const uint32_t z0 = iz > 0 ? iz - 1 : 0, z1 = min(iz + 1, (int)g.nz - 1);
   const uint32_t n_runs = kSrRowsLines / rows;
-  for (uint32_t a0 = chunk0 * width; a0 < cnt; a0 += warps_per_cell * width) {
-    const bool active = a0 + li < cnt;
+  for (uint32_t a0 = first; a0 < end; a0 += step) {
+    const bool active = a0 + li < end;
     const uint32_t i = start + a0 + li;
     const double4 me = active ? pd[i] : make_double4(0., 0., 0., 0.);
     const double4 none = make_double4(1e30, 1e30, 1e30, 0.);
@@ -373,15 +383,15 @@ __device__ __forceinline__ void sr_warp(const double4 *__restrict__ pd, const ui
       if (jx < 0 || jy < 0 || jx >= (int)g.nx || jy >= (int)g.ny) continue;
       const uint32_t c = (jx * g.ny + jy) * g.nz;
       uint32_t b = cell_point[c + z0];
-      const uint32_t end = cell_point[c + z1] + cell_count[c + z1];
+      const uint32_t e = cell_point[c + z1] + cell_count[c + z1];
       const bool own = dx == 0 && dy == 0;
-      double4 ahead = b + lane < end ? pd[b + lane] : none;
-      for (; b < end; b += 32) {
+      double4 ahead = b + lane < e ? pd[b + lane] : none;
+      for (; b < e; b += 32) {
         __syncwarp();
         s_at[lane] = ahead;
         __syncwarp();
-        ahead = b + 32 + lane < end ? pd[b + 32 + lane] : none;
-        const uint32_t n = min(32u, end - b);
+        ahead = b + 32 + lane < e ? pd[b + 32 + lane] : none;
+        const uint32_t n = min(32u, e - b);
         if (own) sr_batch<true>(s_at, n, sub, groups, me, i - b, f4);
         else sr_batch<false>(s_at, n, sub, groups, me, 0, f4);
       }
@@ -404,24 +414,55 @@ __device__ __forceinline__ void sr_warp(const double4 *__restrict__ pd, const ui
   }
 }
 
-// CTA: kSrWarps / warps_per_cell cells.
+// Pieces next, next + step, ... of dense cells, `max_width` atoms at a time.  Out
+// of line: in one loop with the cells' own atoms both were 5-6 % slower.
+template <int kCtas>
+static __device__ __noinline__ void sr_pieces(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
+                                             const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
+                                             double4 *__restrict__ sr, uint32_t rows, uint32_t row, uint32_t max_width,
+                                             const Pieces &pieces, uint32_t next, uint32_t step, double4 *s_at) {
+  const uint32_t per = kPieceAtoms / max_width, n_pieces = *pieces.n * per;
+  for (; next < n_pieces; next += step) {
+    const uint2 r = pieces.list[next / per];
+    const uint32_t first = r.y + (next % per) * max_width, end = min(cell_count[r.x], first + max_width);
+    if (first < end)
+      sr_warp(pd, cell_count, cell_point, g, natom, sr, rows, row, r.x, first, kPieceAtoms, end, max_width, s_at);
+  }
+}
+
+// CTA: kSrWarps / warps_per_cell cells, up to pieces.cap atoms of each; then its
+// warps take pieces of dense cells.
+template <int kCtas>
 __device__ __forceinline__ void sr_block(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
                                          const uint32_t *__restrict__ cell_point, const Grid &g, uint32_t natom,
                                          double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell,
-                                         uint32_t max_width, uint32_t bx, uint32_t row) {
+                                         uint32_t max_width, const Pieces &pieces, uint32_t bx, uint32_t row) {
   __shared__ double4 s_at[kSrWarps][32];
   const uint32_t warp = threadIdx.x >> 5;
-  const uint32_t w = bx * kSrWarps + warp, cell = w / warps_per_cell;
+  const uint32_t w = bx * kSrWarps + warp, warps = g.ncell * warps_per_cell;
+  const uint32_t cell = w / warps_per_cell;
   if (cell >= g.ncell) return;
-  sr_warp(pd, cell_count, cell_point, g, natom, sr, rows, row, cell, w - cell * warps_per_cell, warps_per_cell,
-          max_width, s_at[warp]);
+  const uint32_t cnt = cell_count[cell];
+  const uint32_t width = min(max_width, cnt > 16 ? 32u : cnt > 8 ? 16u : 8u);
+  const uint32_t first = (w - cell * warps_per_cell) * width, end = min(cnt, pieces.cap);
+  const uint32_t back = warps - 1 - w;
+  const bool more = back < kPieceWarps && pieces.list && back < *pieces.n * (kPieceAtoms / max_width);
+  if (first < end)
+    sr_warp(pd, cell_count, cell_point, g, natom, sr, rows, row, cell, first, warps_per_cell * width, end, width,
+            s_at[warp]);
+  if (more)
+    sr_pieces<kCtas>(pd, cell_count, cell_point, g, natom, sr, rows, row, max_width, pieces, back,
+                     min(warps, kPieceWarps), s_at[warp]);
 }
 
-__global__ void __launch_bounds__(kSrThreads)
+// kCtas: CTAs per SM the registers are cut for (sr_ctas).
+template <int kCtas>
+__global__ void __launch_bounds__(kSrThreads, kCtas)
 k_short_range(const double4 *__restrict__ pd, const uint32_t *__restrict__ cell_count,
               const uint32_t *__restrict__ cell_point, Grid g, uint32_t natom,
-              double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell, uint32_t max_width) {
-  sr_block(pd, cell_count, cell_point, g, natom, sr, rows, warps_per_cell, max_width, blockIdx.x, blockIdx.y);
+              double4 *__restrict__ sr, uint32_t rows, uint32_t warps_per_cell, uint32_t max_width, Pieces pieces) {
+  sr_block<kCtas>(pd, cell_count, cell_point, g, natom, sr, rows, warps_per_cell, max_width, pieces, blockIdx.x,
+                  blockIdx.y);
 }
 
 // ----------------------------------------------------------------------------

@@ -145,7 +145,8 @@ struct glst_handle {
   // atoms
   uint32_t *atom_cell = nullptr, *atom_slot = nullptr, *perm = nullptr;
   uint32_t *sorted_idx = nullptr, *cell_count = nullptr, *cell_point = nullptr;
-  uint32_t *flags = nullptr;
+  uint32_t *flags = nullptr;  // [1]: the combine's ticket, [2]: pieces of dense cells
+  uint2 *pieces = nullptr;    // pieces of dense cells (layout.cuh)
   float4 *pk = nullptr;
   double4 *pd = nullptr;
   // nodes, internal order: group -> direction -> radial
@@ -537,6 +538,7 @@ static glst_status setup(glst_handle *h, uint32_t natom, double tol,
   GLST_TRY(dalloc_n(h, &h->cell_count, C));
   GLST_TRY(dalloc_n(h, &h->cell_point, C));
   GLST_TRY(dalloc_n(h, &h->flags, 4));
+  GLST_TRY(dalloc_n(h, &h->pieces, std::max<uint32_t>(1, dev::max_pieces(natom, p.ncell))));
   GLST_TRY(dalloc_n(h, &h->pk, N));
   GLST_TRY(dalloc_n(h, &h->pd, N));
   h->sr_rows = sr_rows_for(C, h->nsm);
@@ -645,7 +647,7 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
     dev::k_bin<<<nb, 256, 0, st>>>(rx, ry, rz, N, h->grid, h->atom_cell, h->atom_slot, h->cell_count);
     CUDA_TRY(cudaGetLastError());
   }
-  dev::k_scan<<<1, 1024, 0, st>>>(h->cell_count, C, h->cell_point);
+  dev::k_scan<<<1, 1024, 0, st>>>(h->cell_count, C, h->cell_point, dev::cell_cap(N, C), h->pieces, h->flags + 2);
   CUDA_TRY(cudaGetLastError());
   if (N) {
     const uint32_t nb = (N + 255) / 256;
@@ -659,6 +661,10 @@ static glst_status phase_assign(glst_handle *h, const double *rx, const double *
   }
   h->assigned = true;
   return GLST_OK;
+}
+
+static dev::Pieces pieces_of(const glst_handle *h) {
+  return dev::Pieces{h->pieces, h->flags + 2, dev::cell_cap(h->plan.natom, h->plan.ncell)};
 }
 
 // Far-field phases of one node stage: direction tiles [u0, u1),
@@ -737,7 +743,7 @@ static dev::LrArgs lr_args(const glst_handle *h, size_t stage) {
                      reinterpret_cast<const float4 *>(h->cheb_lr), h->R, h->part, h->cheb_scale, h->plan.ncell,
                      rg.u1 - rg.u0, rg.tpc, h->max_rad, rg.kb, h->plan.natom,
                      stage > 0 ? 1 : 0,  // stage 0 writes its rows, later stages add into the same rows
-                     h->lr_tab4};
+                     h->lr_tab4, rg.rows(), pieces_of(h)};
 }
 
 static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
@@ -747,9 +753,9 @@ static glst_status lr_stage(glst_handle *h, size_t stage, cudaStream_t st) {
   if (ctas > 0x7fffffffu) return fail(GLST_ERR_SIZE, "too many cells for the gather's grid");
   const size_t smem = dev::lr_smem_bytes(h->max_rad), tab = h->lr_tab4 * sizeof(float4);
   if (smem + tab <= kLrSmemMax)
-    dev::k_long_range<<<(uint32_t)ctas, dev::kLrThreads, smem + tab, st>>>(lr_args(h, stage), rg.rows());
+    dev::k_long_range<<<(uint32_t)ctas, dev::kLrThreads, smem + tab, st>>>(lr_args(h, stage));
   else
-    dev::k_long_range_general<<<(uint32_t)ctas, dev::kLrThreads, smem, st>>>(lr_args(h, stage), rg.rows());
+    dev::k_long_range_general<<<(uint32_t)ctas, dev::kLrThreads, smem, st>>>(lr_args(h, stage));
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }
@@ -794,17 +800,14 @@ static glst_status phase_lr(glst_handle *h, cudaStream_t st) {
   return (h->K && single_stage(h)) ? lr_stage(h, 0, st) : GLST_OK;
 }
 
-static uint32_t sr_blocks(uint32_t ncell, uint32_t warps_per_cell) {
-  return (uint32_t)(((uint64_t)ncell * warps_per_cell + dev::kSrWarps - 1) / dev::kSrWarps);
-}
-
 static glst_status phase_sr(glst_handle *h, cudaStream_t st) {
   if (!h->plan.natom || h->shard > 0) return GLST_OK;  // shard 0 owns the near field
   const uint32_t width = dev::sr_width(h->plan.natom, h->sr_rows);
   const uint32_t wpc = dev::sr_warps_per_cell(h->plan.natom, h->plan.ncell, width);
-  dim3 grid(sr_blocks(h->plan.ncell, wpc), h->sr_rows);
-  dev::k_short_range<<<grid, dev::kSrThreads, 0, st>>>(h->pd, h->cell_count, h->cell_point, h->grid,
-                                                       h->plan.natom, h->sr, h->sr_rows, wpc, width);
+  dim3 grid(dev::sr_blocks(h->plan.ncell, wpc), h->sr_rows);
+  const auto kernel = dev::sr_ctas(h->plan.natom, h->plan.ncell) == 4 ? dev::k_short_range<4> : dev::k_short_range<5>;
+  kernel<<<grid, dev::kSrThreads, 0, st>>>(h->pd, h->cell_count, h->cell_point, h->grid, h->plan.natom, h->sr,
+                                           h->sr_rows, wpc, width, pieces_of(h));
   CUDA_TRY(cudaGetLastError());
   return GLST_OK;
 }
@@ -1542,7 +1545,7 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
       if (!h->K || !h->plan.natom) return;
       const uint32_t quads = h->n_tiles / dev::kSfWarps;
       gr.sf_smem = std::max(gr.sf_smem, dev::sf_smem_bytes(h->max_rad, h->sf_tab4));
-      for (uint32_t c = 0; c < h->plan.ncell; c += dev::sf_cells(h->plan.natom, h->plan.ncell, quads))
+      for (uint32_t c = 0; c < h->plan.ncell; c += sf_args(h, h->ranges[0]).cells)
         for (uint32_t u = 0; u < quads; u++) items.push_back({w, u, c, 0});
     });
     each(glst_batch::kShell, [&](uint32_t w, glst_handle *h) {
@@ -1557,11 +1560,11 @@ static glst_status worklist_build(glst_batch *b, const std::vector<double> &cost
     });
     each(glst_batch::kSr, [&](uint32_t w, glst_handle *h) {
       if (!h->plan.natom) return;
+      const uint32_t width = dev::sr_width(h->plan.natom, h->sr_rows);
+      const uint32_t wpc = dev::sr_warps_per_cell(h->plan.natom, h->plan.ncell, width);
+      const uint32_t blocks = dev::sr_blocks(h->plan.ncell, wpc);
       for (uint32_t pl = 0; pl < h->sr_rows; pl++)
-        for (uint32_t c = 0; c < sr_blocks(h->plan.ncell, dev::sr_warps_per_cell(h->plan.natom, h->plan.ncell,
-                                                                              dev::sr_width(h->plan.natom, h->sr_rows)));
-             c++)
-          items.push_back({w, c, pl, 0});
+        for (uint32_t c = 0; c < blocks; c++) items.push_back({w, c, pl, 0});
     });
     each(glst_batch::kCombine, [&](uint32_t w, glst_handle *h) {
       if (h->plan.natom)
@@ -1651,6 +1654,9 @@ static glst_status worklist_descriptors(glst_batch *b, const double *const in[4]
     d.block_energy = h->block_energy;
     d.energy = b->energies + i;
     d.ticket = h->flags + 1;
+    d.n_pieces = h->flags + 2;
+    d.piece_list = h->pieces;
+    d.pieces = pieces_of(h);
   }
   if (!ds.empty()) CUDA_TRY(cudaMemcpy(b->d_desc, ds.data(), ds.size() * sizeof(dev::SysDesc), cudaMemcpyHostToDevice));
   return GLST_OK;
@@ -1948,7 +1954,7 @@ struct SrvSlot {
 uint64_t estimate_bytes(const Plan &p, int nsm) {
   const uint64_t N = p.natom, C = p.ncell, K = p.has_far ? p.K() : 0;
   const uint64_t combine = (N + dev::kCombineAtoms - 1) / dev::kCombineAtoms;
-  uint64_t b = N * (4 * 4 + 16 + 32 + 32 * (uint64_t)sr_rows_for(C, nsm) + 8 * 8 + 32) + C * 8 + combine * 8 + 4096;
+  uint64_t b = N * (4 * 4 + 16 + 32 + 32 * (uint64_t)sr_rows_for(C, nsm) + 8 * 8 + 32) + C * 8 + combine * 8 + N / 4 + 4096;
   if (K) {
     const uint32_t waves = tuned(p, (uint32_t)K).lr_waves;
     const FarLayout lay = glst::far_layout(p, 0, 1, waves ? waves : kLrWaves, nsm, stage_budget());

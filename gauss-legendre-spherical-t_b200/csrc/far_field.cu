@@ -15,24 +15,20 @@ k_structure_factors(const __grid_constant__ SfArgs a, uint32_t cell_base) {
 }
 
 #elif GLST_PART == 1
-__global__ void __launch_bounds__(kLrThreads, 3)
-k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
+__global__ void __launch_bounds__(kLrThreads, 3) k_long_range(const __grid_constant__ LrArgs a) {
   extern __shared__ float4 s_lr[];
   for (uint32_t i = threadIdx.x; i < a.tab4; i += kLrThreads) s_lr[i] = a.tab[i];
   __syncthreads();
   const uint64_t item = (uint64_t)blockIdx.x * kLrWarps + (threadIdx.x >> 5);
   const uint32_t chunk = (uint32_t)(item / a.ncell);
-  if (chunk >= n_chunks) return;
-  lr_warp<true>(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
+  if (chunk < a.n_chunks) lr_items<true>(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
 }
 
 #elif GLST_PART == 2
-__global__ void __launch_bounds__(kLrThreads, 3)
-k_long_range_general(const __grid_constant__ LrArgs a, uint32_t n_chunks) {
+__global__ void __launch_bounds__(kLrThreads, 3) k_long_range_general(const __grid_constant__ LrArgs a) {
   const uint64_t item = (uint64_t)blockIdx.x * kLrWarps + (threadIdx.x >> 5);
   const uint32_t chunk = (uint32_t)(item / a.ncell);
-  if (chunk >= n_chunks) return;
-  lr_warp<false>(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
+  if (chunk < a.n_chunks) lr_items<false>(a, (uint32_t)(item - (uint64_t)chunk * a.ncell), chunk);
 }
 
 #elif GLST_PART == 3
@@ -49,7 +45,7 @@ __global__ void __launch_bounds__(kSfThreads, 4) k_structure_factors_multi(const
 #elif GLST_PART == 4
 // item (a, b) = (first of kLrWarps cells, long-range chunk); out of line, as
 // the structure factors
-static __device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_warp<false>(a, cell, chunk); }
+static __device__ __noinline__ void lr_item(const LrArgs &a, uint32_t cell, uint32_t chunk) { lr_items<false>(a, cell, chunk); }
 
 __global__ void __launch_bounds__(kLrThreads, 3) k_long_range_multi(const SysDesc *__restrict__ sys,
                                                                     const WorkItem *__restrict__ items,

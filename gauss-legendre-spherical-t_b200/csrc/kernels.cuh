@@ -304,7 +304,9 @@ __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const
 }
 
 // Work item: kSfWarps consecutive tiles (of one group) and a.cells cells from
-// `cell0` on.
+// `cell0` on (cells far apart, which would spread a cluster's full cells, cost
+// 2 % on 26^3 cells of 6 atoms and 6-10 % on a droplet and a slab there: S is
+// written in longer runs this way).
 __device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_t cell0) {
   extern __shared__ float4 s_sf[];
   const uint32_t warp = threadIdx.x >> 5;
@@ -361,8 +363,8 @@ __global__ void k_structure_factors(const __grid_constant__ SfArgs a, uint32_t c
 // tiles and warps.  Atoms beyond the series' range and tiles of too few atoms
 // for the product take a sine and cosine per node (lr_direct).
 //
-// Warps are independent: each takes a cell and a chunk of direction tiles,
-// with no CTA barriers (four warps on one cell's chunk waited for each other
+// Warps are independent: each takes a cell (up to its cap, then pieces of denser
+// cells: layout.cuh) and a chunk of direction tiles, with no CTA barriers (four warps on one cell's chunk waited for each other
 // a third of the time).  A tile's R' is copied to shared memory
 // asynchronously while the previous tile's series are evaluated -- the buffer
 // is free once its coefficients are formed.  The groups' tables are copied to
@@ -391,6 +393,8 @@ struct LrArgs {
   uint32_t ncell, n_tiles, tiles_per_chunk, max_rad, node_off, natom;
   int accumulate;      // a later node stage adds into the same rows
   uint32_t tab4;       // float4s of all groups' tables
+  uint32_t n_chunks;
+  Pieces pieces;
 };
 
 __host__ __device__ inline size_t lr_smem_bytes(uint32_t max_rad) {
@@ -575,12 +579,12 @@ __device__ __forceinline__ void lr_tile(const LrArgs &a, const DirTile &u, const
   }
 }
 
-// Work item of a warp: a cell and a chunk of direction tiles.
+// Work item of a warp: the atoms [first, end) of a cell and a chunk of direction
+// tiles.
 template <bool kTabShared>
-__device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t chunk) {
+__device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t first, uint32_t end, uint32_t chunk) {
   extern __shared__ float4 s_lr[];
-  const uint32_t cnt = a.cell_count[cell];
-  if (cnt == 0) return;
+  const uint32_t cnt = min(a.cell_count[cell], end);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t start = a.cell_point[cell];
   const uint32_t t0 = chunk * a.tiles_per_chunk, t1 = min(a.n_tiles, t0 + a.tiles_per_chunk);
@@ -590,7 +594,7 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
   double *acc = reinterpret_cast<double *>(s_own + kLrWarps * kLrAtomTile) + warp * (kLrAtomTile * 4);
   float2 *s_r = reinterpret_cast<float2 *>(reinterpret_cast<double *>(s_own + kLrWarps * kLrAtomTile) +
                                            kLrWarps * kLrAtomTile * 4) + (size_t)warp * 32 * sf_row(rc);
-  for (uint32_t a0 = 0; a0 < cnt; a0 += kLrAtomTile) {
+  for (uint32_t a0 = first; a0 < cnt; a0 += kLrAtomTile) {
     const uint32_t na = min((uint32_t)kLrAtomTile, cnt - a0), pad = (na + kLrBatch - 1) & ~(uint32_t)(kLrBatch - 1);
     // the first series tile
     auto is_series = [&](const DirTile &u) { return u.n_dir > 0 && u.lr_P > 0 && 16u * na > u.lr_P; };
@@ -660,11 +664,26 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
   }
 }
 
-// Items chunk by chunk, so that the first (largest) groups' work starts first
-// and a CTA's warps share a chunk's tables; the general form reads the tables
-// from global memory.
-__global__ void k_long_range(const __grid_constant__ LrArgs a, uint32_t n_chunks);
-__global__ void k_long_range_general(const __grid_constant__ LrArgs a, uint32_t n_chunks);
+// A warp's items: a cell (up to its cap) and a chunk, then pieces of dense cells
+// with the same chunk.  Items chunk by chunk, so that the first (largest) groups'
+// work starts first and a CTA's warps share a chunk's tables.
+template <bool kTabShared>
+__device__ __forceinline__ void lr_items(const LrArgs &a, uint32_t cell, uint32_t chunk) {
+  uint32_t next = a.ncell - 1 - cell;
+  const uint32_t n_pieces = next < kPieceWarps ? *a.pieces.n : 0u;
+  for (uint32_t first = 0, end = a.pieces.cap;; next += min(a.ncell, kPieceWarps)) {
+    lr_warp<kTabShared>(a, cell, first, end, chunk);
+    if (next >= n_pieces) return;
+    const uint2 r = a.pieces.list[next];
+    cell = r.x;
+    first = r.y;
+    end = first + kPieceAtoms;
+  }
+}
+
+// the general form reads the tables from global memory
+__global__ void k_long_range(const __grid_constant__ LrArgs a);
+__global__ void k_long_range_general(const __grid_constant__ LrArgs a);
 
 // ----------------------------------------------------------------------------
 // Many systems per launch (worklist.cuh).
@@ -679,7 +698,9 @@ struct SysDesc {
   SfArgs sf;    // structure-factor arguments
   LrArgs lr;    // gather arguments
   double4 *part, *sr;
-  uint32_t *ticket;
+  uint32_t *ticket, *n_pieces;
+  uint2 *piece_list;
+  Pieces pieces;    // the same for its readers
   double *cfx, *cfy, *cfz, *cen, *ofx, *ofy, *ofz, *oen, *block_energy, *energy;
 };
 

@@ -77,11 +77,54 @@ __host__ __device__ inline uint32_t sf_cells(uint32_t natom, uint32_t ncell, uin
   return natom / ncell > 16 || ctas < 12 * kSms ? 1u : ctas < 28 * kSms ? 4u : 8u;
 }
 
+// Atoms of a cell that the cell's own warps of the near field and the gather
+// take, at most: 2.5 times the mean, in whole 32s.  Evenly filled boxes stay
+// below it (from 4 cells per axis on their full cells hold at most 2.4 times the
+// mean of a grid whose outer layers are empty); at 1.25 times the mean full
+// cells were cut just before their end, which cost batches of such boxes 2.5 %.
+// The rest of a denser cell (a droplet or a slab in a wide box: the mean says
+// nothing about its cells) is listed by the scan as pieces of up to kPieceAtoms
+// atoms, and the last kPieceWarps warps of a near-field row or a gather chunk take
+// pieces when they are done with their own cell (the outer layers are the emptiest;
+// on large grids the others' look at the list would cost 0.7 %).
+// Measured, all of a cell's atoms by its own warps against this: near field of
+// 8,000 atoms in one of 26^3 cells 167 against 0.9 ms, 12,000 atoms in a droplet
+// on 20^3 cells 1.6 against 0.21 ms and their gather 0.46 against 0.14.
+constexpr uint32_t kPieceAtoms = 32;
+constexpr uint32_t kPieceWarps = 2048;
+__host__ __device__ inline uint32_t cell_cap(uint32_t natom, uint32_t ncell) {
+  const uint64_t cap = ((uint64_t)natom * 5 / 2 / ncell + kPieceAtoms) / kPieceAtoms * kPieceAtoms;
+  return cap < natom ? (uint32_t)cap : (natom + kPieceAtoms) / kPieceAtoms * kPieceAtoms;
+}
+
+// Pieces there can be: every piece's cell holds another 32 atoms of its own.
+__host__ __device__ inline uint32_t max_pieces(uint32_t natom, uint32_t ncell) {
+  return natom > cell_cap(natom, ncell) ? natom / kPieceAtoms : 0u;
+}
+
+// The list of pieces: {cell, first atom within the cell}.
+struct Pieces {
+  const uint2 *list;
+  const uint32_t *n;
+  uint32_t cap;  // cell_cap
+};
+
 // Lanes per chunk, at most: the widest chunks of which there are still 2,048
 // (about four warps for each of the GPU's schedulers), else 8 atoms wide.
 __host__ __device__ inline uint32_t sr_width(uint32_t natom, uint32_t rows) {
   const uint64_t lanes = (uint64_t)natom * rows;
   return lanes >= 2048u * 32u ? 32u : lanes >= 2048u * 16u ? 16u : 8u;
+}
+
+// Near-field CTAs per SM: four (128 registers) where warps have many atoms to
+// pair, five where cells hold few and latency counts.  Measured, four against
+// five: 87 atoms per cell 157 against 167 us, 168 per cell 175 against 192, 6 per
+// cell on 26^3 cells 105 against 98.
+__host__ __device__ inline int sr_ctas(uint32_t natom, uint32_t ncell) { return natom / ncell > 16 ? 4 : 5; }
+
+// Near-field CTAs (four warps) for the cells of one row.
+__host__ __device__ inline uint32_t sr_blocks(uint32_t ncell, uint32_t warps_per_cell) {
+  return (uint32_t)(((uint64_t)ncell * warps_per_cell + 3) / 4);
 }
 
 // Warps per cell for a mean number of atoms per cell.

@@ -181,13 +181,14 @@ extern "C" glst_status glst_near_field_noalloc(uint32_t natom, const double *d_r
   if (natom) {
     const uint32_t nb = (natom + 255) / 256;
     dev::k_bin<<<nb, 256, 0, st>>>(d_rx, d_ry, d_rz, natom, g, atom_cell, atom_slot, cell_count);
-    dev::k_scan<<<1, 1024, 0, st>>>(cell_count, (uint32_t)ncell, cell_point);
+    dev::k_scan<<<1, 1024, 0, st>>>(cell_count, (uint32_t)ncell, cell_point, 0, nullptr, nullptr);
     dev::k_scatter<<<nb, 256, 0, st>>>(atom_cell, atom_slot, cell_point, natom, perm);
     const uint32_t spc = dev::sort_cells(natom, (uint32_t)ncell);
     dev::k_sort_pack<<<((uint32_t)ncell + spc - 1) / spc, 32 * dev::kSortCells, dev::kSortCap * sizeof(uint32_t), st>>>(
         perm, cell_count, cell_point, g, atom_cell, natom, d_rx, d_ry, d_rz, d_qc, sorted, pk, pd);
-    dev::k_short_range<<<dim3((uint32_t)ncell, dev::kSrRowsPlanes), dev::kSrThreads, 0, st>>>(
-        pd, cell_count, cell_point, g, natom, sr, dev::kSrRowsPlanes, dev::kSrWarps, dev::sr_width(natom, dev::kSrRowsPlanes));
+    dev::k_short_range<4><<<dim3((uint32_t)ncell, dev::kSrRowsPlanes), dev::kSrThreads, 0, st>>>(
+        pd, cell_count, cell_point, g, natom, sr, dev::kSrRowsPlanes, dev::kSrWarps,
+        dev::sr_width(natom, dev::kSrRowsPlanes), dev::Pieces{nullptr, nullptr, 0xffffffffu});
     dev::k_combine<<<(natom + dev::kCombineAtoms - 1) / dev::kCombineAtoms, dev::kCombineThreads, 0, st>>>(
         sr, dev::kSrRowsPlanes, nullptr, 0, sorted, natom, 0, cell_out, cell_out + kMaxAtoms, cell_out + 2ull * kMaxAtoms,
         cell_out + 3ull * kMaxAtoms, d_fx, d_fy, d_fz, d_en, block_e, nullptr, nullptr);

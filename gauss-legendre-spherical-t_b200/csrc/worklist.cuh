@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(1024) k_scan_multi(const SysDesc *__restrict__
                                                      const WorkItem *__restrict__ items, uint32_t n) {
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const SysDesc &d = sys[items[it].sys];
-    scan_body(d.cell_count, d.g.ncell, d.cell_point);
+    scan_body(d.cell_count, d.g.ncell, d.cell_point, d.pieces.cap, d.piece_list, d.n_pieces);
     __syncthreads();
   }
 }
@@ -87,8 +87,9 @@ __global__ void __launch_bounds__(kSrThreads) k_short_range_multi(const SysDesc 
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const WorkItem w = items[it];
     const SysDesc &d = sys[w.sys];
-    sr_block(d.pd, d.cell_count, d.cell_point, d.g, d.natom, d.sr, d.sr_rows, sr_warps_per_cell(d.natom, d.g.ncell, sr_width(d.natom, d.sr_rows)),
-             sr_width(d.natom, d.sr_rows), w.a, w.b);
+    const uint32_t width = sr_width(d.natom, d.sr_rows);
+    sr_block<4>(d.pd, d.cell_count, d.cell_point, d.g, d.natom, d.sr, d.sr_rows,
+             sr_warps_per_cell(d.natom, d.g.ncell, width), width, d.pieces, w.a, w.b);
     __syncthreads();
   }
 }
