@@ -34,34 +34,35 @@ def inputs():
         os.path.join(CSRC, "*.hpp")) + [os.path.join(ROOT, "include", "glst_c.h"), os.path.abspath(__file__)]
 
 
-def up_to_date():
-    if not os.path.exists(LIB):
+def up_to_date(lib=LIB):
+    if not os.path.exists(lib):
         return False
-    t = os.path.getmtime(LIB)
+    t = os.path.getmtime(lib)
     return all(os.path.getmtime(s) <= t for s in inputs())
 
 
-def build(force=False, verbose=False):
-    if not force and up_to_date():
-        return LIB
-    base = [nvcc(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC"]
+def build(force=False, verbose=False, lib=LIB, defines=()):
+    """Compile to `lib`, with extra -D options `defines`; returns its path."""
+    if not force and up_to_date(lib):
+        return lib
+    base = [nvcc(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC", *defines]
     with tempfile.TemporaryDirectory() as tmp:
         jobs = []
-        for i, (src, defines) in enumerate(UNITS):
+        for i, (src, part) in enumerate(UNITS):
             obj = os.path.join(tmp, "%d.o" % i)
-            cmd = base + defines + ["-I" + os.path.join(ROOT, "include"), "-c", os.path.join(CSRC, src), "-o", obj]
+            cmd = base + part + ["-I" + os.path.join(ROOT, "include"), "-c", os.path.join(CSRC, src), "-o", obj]
             if verbose:
                 print(" ".join(cmd), flush=True)
             jobs.append((obj, cmd, subprocess.Popen(cmd)))
         failed = [cmd for _, cmd, p in jobs if p.wait() != 0]
         if failed:
             raise subprocess.CalledProcessError(1, failed[0])
-        cmd = base + ["-shared", "-o", LIB + ".tmp"] + [obj for obj, _, _ in jobs]
+        cmd = base + ["-shared", "-o", lib + ".tmp"] + [obj for obj, _, _ in jobs]
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-    os.replace(LIB + ".tmp", LIB)
-    return LIB
+    os.replace(lib + ".tmp", lib)
+    return lib
 
 
 if __name__ == "__main__":

@@ -89,8 +89,14 @@ __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
 constexpr int kSfWarps = 4;
 constexpr int kSfThreads = 32 * kSfWarps;
 constexpr int kSfAtomTile = 128;
-constexpr int kSfRadChunk = 64;   // radial nodes staged at a time, at most
-constexpr int kChebMaxP = 64;     // series terms, at most (the lengths compiled: series_terms, planner.cpp)
+#ifndef GLST_RAD_CHUNK  // (smaller in a test's build, as GLST_MAX_TERMS)
+#define GLST_RAD_CHUNK 64
+#endif
+#ifndef GLST_MAX_TERMS
+#define GLST_MAX_TERMS 64
+#endif
+constexpr int kSfRadChunk = GLST_RAD_CHUNK;  // radial nodes staged at a time, at most
+constexpr int kChebMaxP = GLST_MAX_TERMS;    // series terms, at most (the lengths compiled: planner, series_terms)
 __host__ __device__ constexpr int cheb_b(int P) { return P > 24 ? 8 : 4; }
 __host__ __device__ constexpr int cheb_row(int P) { return (P + 3) / 4 * 4; }  // table row, in floats
 
@@ -319,10 +325,10 @@ __device__ __forceinline__ void sf_block(const SfArgs &a, uint32_t quad, uint32_
   float4 *s_at = s_sf + a.tab4 + warp * 32;
   float2 *s_f = reinterpret_cast<float2 *>(s_sf + a.tab4 + kSfWarps * 32) + (size_t)warp * 32 * sf_row(rc);
   const uint32_t cell1 = min(a.ncell, cell0 + a.cells);
-#define GLST_SF_CASE(n)                                                                            \
-  case n:                                                                                          \
-    for (uint32_t cell = cell0; cell < cell1; cell++)                                              \
-      sf_tile<n>(a, u, a.pk + a.cell_point[cell], a.cell_count[cell], cell, s_sf, s_at, s_f);      \
+#define GLST_SF_CASE(n)                                                                                           \
+  case n:                                                                                                         \
+    for (uint32_t cell = cell0; cell < cell1; cell++)                                                             \
+      sf_tile<(n <= kChebMaxP ? n : 0)>(a, u, a.pk + a.cell_point[cell], a.cell_count[cell], cell, s_sf, s_at, s_f); \
     break;
   switch (u.P) {
     GLST_SF_CASE(0) GLST_SF_CASE(4) GLST_SF_CASE(6) GLST_SF_CASE(8) GLST_SF_CASE(10)
@@ -624,7 +630,7 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
       if (tn < t1) un = a.tiles[tn];
       const DirTile *next = tn < t1 ? &un : nullptr;
 #define GLST_LR_CASE(n) \
-  case n: lr_tile<n, kTabShared>(a, u, next, na, cell, s_at, acc, s_r); break;
+  case n: lr_tile<(n <= kChebMaxP ? n : 4), kTabShared>(a, u, next, na, cell, s_at, acc, s_r); break;
       switch (u.lr_P) {
       GLST_LR_CASE(4) GLST_LR_CASE(6) GLST_LR_CASE(8) GLST_LR_CASE(10) GLST_LR_CASE(12)
       GLST_LR_CASE(14) GLST_LR_CASE(16) GLST_LR_CASE(18) GLST_LR_CASE(20) GLST_LR_CASE(22)

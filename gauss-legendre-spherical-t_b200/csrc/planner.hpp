@@ -52,7 +52,12 @@ struct GroupPlan {
   std::vector<float> sf_tab, lr_tab;
 };
 
-constexpr unsigned kSeriesMaxP = 64;                                            // terms, at most
+// Terms, at most (a test builds the library with less, to reach the kernels'
+// forms for plans that the shipped designs do not give).
+#ifndef GLST_MAX_TERMS
+#define GLST_MAX_TERMS 64
+#endif
+constexpr unsigned kSeriesMaxP = GLST_MAX_TERMS;
 constexpr unsigned series_b(unsigned P) { return P > 24 ? 8 : 4; }              // basis T_{Bg} T_b
 constexpr unsigned series_row(unsigned P) { return (P + 3) / 4 * 4; }
 
@@ -119,7 +124,8 @@ struct FarLayout {
 FarLayout far_layout(const Plan &p, uint32_t shard, uint32_t nshards, uint32_t waves, int nsm, uint64_t stage_bytes);
 
 // Chebyshev (Jacobi-Anger) series of the phases of one direction,
-//   e^{-i z x} = sum_p c_p(z) (-i or 1)^{p odd} T_p(x),  |x| <= 1.
+//   e^{-i z x} = sum_p c_p(z) i^{p mod 2} T_p(x),  |x| <= 1,
+// even p giving the real and odd p the imaginary part.
 // series_terms: number of terms (even; above 48, with weights above 36, in
 // larger steps; 0 when more than max_terms would be needed).  Without weights
 // every z of the list is exact to below the rounding of an FP32 phase; with the
