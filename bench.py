@@ -472,7 +472,8 @@ def run_ours(args, world, rank, local, dist):
         wz = w[m].reshape(n_rad, -1)[:, 0] * z if dom == "long_range" else (z == z.max()).astype(float)
         tail = np.cumsum((2.0 * wz[:, None] * bes).sum(0)[::-1])[::-1]
         P = int(np.count_nonzero(tail > (1e-8 if dom == "long_range" else 2e-7) * wz.sum()))
-        P += P % 2
+        every = (2 if P <= 36 else 8) if dom == "long_range" else (2 if P <= 48 else 4)
+        P = max(4, -(-P // every) * every)
         fma_ops += n_dir * P * (float(n) * (2.0 if dom == "long_range" else 1.0) + float(inf.ncell_total) * n_rad)
     fma_ach = fma_ops / (phases[dom] * 1e-3)
     roofline = {

@@ -11,17 +11,19 @@ namespace glst {
 namespace dev {
 
 // ----------------------------------------------------------------------------
-// Sine and cosine on the FP32 FMA pipe, for part of the (atom, node) pairs so
-// that the FMA pipe carries some of the work the MUFU pipe would otherwise
-// serialise.  Method: theta = n pi + r with n = rint(theta / pi) (rounded by
-// adding 1.5 * 2^23), r = theta - n pi in two FMA steps (pi = kPiHi + kPiLo,
+// Sine and cosine on the FP32 FMA pipe, for what the series below do not take:
+// atoms beyond their range, and groups that would need too many terms.  Method:
+// theta = n pi + r with n = rint(theta / pi) (rounded by adding 1.5 * 2^23),
+// r = theta - n pi in two FMA steps (pi = kPiHi + kPiLo,
 // kPiHi with 8 significant bits so n * kPiHi is exact), then
 //   sin r = r + r^3 P(r^2),  cos r = Q(r^2)   on |r| <= pi/2,
 // with P of degree 3 and Q of degree 4, coefficients fitted by this project
 // (Lawson-weighted least squares on [0, (pi/2)^2], csrc/fit_sincos.py).
 // sin(theta) = (-1)^n sin r, cos(theta) = (-1)^n cos r: the common sign is
 // returned folded into a factor (the atom's charge) instead of applied to
-// both results.  Max abs error 1.8e-7 for |theta| <= 30.
+// both results.  Max abs error 1.8e-7 for |theta| <= 30; n kPiHi is exact to
+// |theta| = 2e5, where the phase itself is an FP32 number of 0.01 rad.  (Beyond
+// 1e7 rad -- an atom 1e7 A outside the box -- the reduction fails.)
 constexpr float kInvPi = 0.318309886183790672f;
 constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr float kPiHi = 3.140625f;
@@ -60,7 +62,7 @@ __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
 // circumscribed sphere and a margin), and
 //   e^{-i kappa u} = sum_p (2 - [p = 0]) (-i)^p J_p(kappa U) T_p(u / U)
 // (Jacobi-Anger) falls off faster than geometrically beyond p = kappa U (18,
-// 8 and 4 rad in water10k's groups): P = 36, 24 and 16 terms carry all 33,
+// 8 and 4 rad in water10k's groups): P = 36, 22 and 16 terms carry all 33,
 // 27 and 19 radial nodes to below the rounding of an FP32 phase.  So a
 // direction takes P real moments sum_j q_j T_p(x_j), one FMA each per atom,
 // and one P x n_rad product per cell -- where one sine and cosine per (atom,
@@ -81,8 +83,11 @@ __device__ __forceinline__ float2 bcast(float v) { return make_float2(v, v); }
 // kSfAtomTile atoms, then FP64 over the tiles of a denser cell.  S is stored
 // cell-relative in FP32; its twiddle e^{-ik.c} is applied by the shell sums
 // as they load S.  Atoms beyond U (outside the box by more than the margin,
-// or not a number) and tiles of too few atoms for the product (16 atoms cost
-// as much as P terms) take one sine and cosine per node instead.
+// or not a number) take one sine and cosine per node instead.  So did tiles of
+// up to P / 16 atoms, by a count of the issue slots; measured, the series wins
+// from one atom on: 8^3 cells of 1 / 2 / 3 atoms at the default order 196 / 199 /
+// 202 us against 265 / 353 / 403 (gather 230 / 230 / 230 against 448 / 632 / 767),
+// 20^3 cells of one atom at 1e-3 103 against 128 (gather 135 against 133).
 // Measured: water10k 1.112 -> 0.297 ms, 1,000 waters on 4^3 cells 0.144 ->
 // 0.056 ms, 168 atoms per cell 0.313 -> 0.094 ms; forces 3.3e-8 -> 1.5e-8 off
 // the FP64 path.
@@ -247,9 +252,7 @@ __device__ __forceinline__ void sf_tile(const SfArgs &a, const DirTile &u, const
   uint32_t a0 = 0;
   do {
     const uint32_t na = min((uint32_t)kSfAtomTile, cnt - a0);
-    // few atoms: a sine and cosine per node cost 16 issue slots of the SFU,
-    // the product P FMAs per node
-    const bool series = P > 0 && 16u * na > (uint32_t)P;
+    const bool series = P > 0 && na > 0;
     bool beyond = !series;
     float2 N[P > 0 ? P / 2 : 1];
     if constexpr (P > 0) {
@@ -366,16 +369,18 @@ __global__ void k_structure_factors(const __grid_constant__ SfArgs a, uint32_t c
 // and the outer sum over g another P / B.  The 32 directions are then summed
 // across the warp for eight atoms at a time: 31 shuffles leave one of the 8 x
 // 4 sums in each lane.  FP32 over the 32 directions, FP64 across direction
-// tiles and warps.  Atoms beyond the series' range and tiles of too few atoms
-// for the product take a sine and cosine per node (lr_direct).
+// tiles and warps.  Atoms beyond the series' range take a sine and cosine per
+// node (lr_direct).
 //
 // Warps are independent: each takes a cell (up to its cap, then pieces of denser
-// cells: layout.cuh) and a chunk of direction tiles, with no CTA barriers (four warps on one cell's chunk waited for each other
-// a third of the time).  A tile's R' is copied to shared memory
-// asynchronously while the previous tile's series are evaluated -- the buffer
-// is free once its coefficients are formed.  The groups' tables are copied to
-// shared memory where three CTAs per SM still fit with them (water10k 485 ->
-// 478 us, 168 atoms per cell 149 -> 143, 648 atoms 47 -> 42).
+// cells: layout.cuh) and a chunk of direction tiles, with no CTA barriers (four
+// warps on one cell's chunk waited for each other a third of the time).  A tile's
+// R' is copied to shared memory asynchronously while the previous tile's series
+// are evaluated -- the buffer is free once its coefficients are formed.  The
+// groups' tables are copied to shared memory where three CTAs per SM still fit
+// with them (water10k 485 -> 478 us, 168 atoms per cell 149 -> 143, 648 atoms 47
+// -> 42).  At 168 registers only the lengths above 48, which no shipped design
+// reaches, spill.
 // Measured: water10k 1.458 -> 0.485 ms, 3,000 atoms on 4^3 cells 0.141 ->
 // 0.076 ms, 168 atoms per cell 0.279 -> 0.148 ms, a million atoms 55 -> 17 ms;
 // forces 1.5e-8 -> 0.9e-8 off the FP64 path.
@@ -383,8 +388,10 @@ constexpr int kLrWarps = 4;
 constexpr int kLrThreads = 32 * kLrWarps;
 constexpr int kLrAtomTile = 128;
 constexpr int kLrBatch = 8;       // atoms reduced across the warp together
-constexpr uint32_t kLrMaxRad = 256;    // radial nodes per direction, at most (set-up checks)
-constexpr uint32_t kLrMaxQuads = 128;  // radial nodes of all groups, in fours, at most (set-up checks)
+// Refused by set-up, as ever (neither occurs for the shipped designs): more radial
+// nodes per direction, more quads of radial nodes over all groups.
+constexpr uint32_t kLrMaxRad = 256;
+constexpr uint32_t kLrMaxQuads = 128;
 
 struct LrArgs {
   const float4 *pk;
@@ -603,7 +610,7 @@ __device__ __forceinline__ void lr_warp(const LrArgs &a, uint32_t cell, uint32_t
   for (uint32_t a0 = first; a0 < cnt; a0 += kLrAtomTile) {
     const uint32_t na = min((uint32_t)kLrAtomTile, cnt - a0), pad = (na + kLrBatch - 1) & ~(uint32_t)(kLrBatch - 1);
     // the first series tile
-    auto is_series = [&](const DirTile &u) { return u.n_dir > 0 && u.lr_P > 0 && 16u * na > u.lr_P; };
+    auto is_series = [&](const DirTile &u) { return u.n_dir > 0 && u.lr_P > 0; };
     uint32_t t = t0;
     while (t < t1 && !is_series(a.tiles[t])) t++;
     DirTile u;

@@ -1,8 +1,8 @@
 """GPU parity of the far field's Chebyshev series and of the near field's lane
 groups at the sizes where they change form, against the FP64 oracle.
 
-* cells of 0 to 8 and of 9 to 40 atoms: one sine and cosine per node below P /
-  16 atoms, the series above; 8, 16 and 32 lanes per near-field chunk;
+* cells of 0 to 8 and of 9 to 40 atoms: the series of a few atoms and of many;
+  8, 16 and 32 lanes per near-field chunk;
 * atoms outside the box beyond the series' range (the cell's circumscribed
   sphere and 2 %) and slightly outside it (within the range);
 * cells of 128 and 129 atoms (a whole atom tile, and one atom of the next);
