@@ -293,7 +293,7 @@ __global__ void k_sort_pack(const uint32_t *__restrict__ perm,
 // Measured (one thread per atom and CTA barriers between cells before):
 // water10k 0.291 -> 0.187 ms, 168 atoms per cell 0.400 -> 0.258 ms, 26^3 cells
 // of 6 atoms 0.485 -> 0.102 ms, 3,000 atoms on 4^3 cells 0.067 -> 0.045 ms, a
-// million atoms 4.44 -> 4.03 ms (not measured again since).
+// million atoms 4.44 -> 4.25 ms.
 constexpr int kSrThreads = 128;
 constexpr int kSrWarps = kSrThreads / 32;
 constexpr int kSrRowsPlanes = 3;

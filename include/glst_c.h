@@ -230,8 +230,8 @@ glst_status glst_direct_coulomb(uint32_t natom, const double *d_rx,
                                 double *d_fz, double *d_en, void *stream);
 
 /* Measured pipe peaks of the current device, the denominators of the
- * roofline of the phase kernels (which are bound by the SFU sin/cos and FP32
- * pipes, not by tensor cores or HBM): `sfu_per_s` = MUFU sin+cos results per
+ * roofline of the far-field kernels (which are bound by the FP32 pipe, not by
+ * tensor cores or HBM): `sfu_per_s` = MUFU sin+cos results per
  * second, `fma_per_s` = FP32 fused multiply-adds per second, each from a
  * dependent-chain loop over every SM.  Waits for the device. */
 glst_status glst_measure_pipe_peaks(double *sfu_per_s, double *fma_per_s);
