@@ -7,6 +7,8 @@ pieces of 32 and taken by further warps.
   in a work-list batch (bitwise the same), against the FP64 oracle: the far
   field's forces to 1e-5 of the far field (an FP32 phase of up to 30 rad carries
   2e-6 rad), per-atom energies to 1e-5 of theirs, the near field in FP64;
+* near-field grids (two cells per axis), FP64 throughout: 1e-13 of the RMS force
+  and energy (a sum of some hundred terms of 1e-16, the largest a few times the RMS);
 * the same dense cell in a small and in a large empty box: its near field takes
   the same work, and no more than 2.5 times as long.
 """
@@ -67,6 +69,29 @@ def test_dense_cells_match_the_oracle(pkg, store, n_axis, tol):
         assert np.all(np.asarray(b.energies()) == energy)
     for o, g in zip(out, got):
         assert np.array_equal(o.cpu().numpy(), np.concatenate([g, g]))
+
+
+@pytest.mark.parametrize("counts", [[300, 1, 0, 2, 0, 0, 33, 0], [97, 97, 0, 0, 0, 0, 0, 1], [0, 0, 0, 0, 0, 0, 0, 129],
+                                    [40, 30, 20, 10, 9, 8, 17, 16]])
+def test_near_field_of_uneven_cells(pkg, store, counts):
+    rng = np.random.default_rng(sum(counts))
+    pts = []
+    for c, n in enumerate(counts):
+        m = max(1, int(np.ceil(n ** (1 / 3))))
+        lat = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+        pts.append(10.0 * np.array([c // 4, c // 2 % 2, c % 2]) + (lat + 0.5 + rng.uniform(-0.3, 0.3, lat.shape)) * 9.9 / m)
+    p = np.concatenate(pts)[rng.permutation(sum(counts))]
+    x, y, z = (np.ascontiguousarray(p[:, i]) for i in range(3))
+    q = rng.choice([-0.834, 0.417, 0.417], len(p))
+    plan = planner.make_plan(len(p), 1e-4, (20.0,) * 3, 10.0, store)
+    assert not plan.has_far
+    ref = oracle.glst(x, y, z, q, plan)
+    with pkg.GlstForce(len(p), 1e-4, 20.0, 20.0, 20.0, rcut=10.0) as f:
+        f.calc_ener_force(*_dev((x, y, z, q)))
+        got = f.get_ef()
+    for part in (slice(0, 3), slice(3, 4)):
+        err = np.sqrt(np.mean(sum((g - r) ** 2 for g, r in zip(got[part], ref[part]))))
+        assert err <= 1e-13 * np.sqrt(np.mean(sum(r * r for r in ref[part]))), err
 
 
 def test_a_dense_cell_costs_the_same_in_a_wide_box(pkg):

@@ -8,10 +8,11 @@ groups at the sizes where they change form, against the FP64 oracle.
 * cells of 128 and 129 atoms (a whole atom tile, and one atom of the next);
 * tolerances from 1e-2 to 1e-7: 4 to 42 series terms, 2 to 41 radial nodes.
 
-Bars: the far field's forces 1e-5 relative RMS of the far field itself (an FP32
-phase carries about |k.d| x 6e-8 <= 2e-6 rad at |k.d| <= 30 rad, the atoms far
-outside twice that; measured 1e-7 to 4e-7), the near field 1e-12; the energy
-1e-6 of the sum of its terms' magnitudes.
+Bars: forces 1e-5 of the far field's RMS (an FP32 phase carries about |k.d| x 6e-8
+<= 2e-6 rad at |k.d| <= 30 rad, the atoms far outside twice that; measured 1e-7 to
+4e-7) and 1e-12 of the total for the near field's FP64 sums beside it; per-atom
+energies the same; the total energy 1e-6 of the sum of its terms' magnitudes.
+(The near field by itself: test_gpu_clusters.py.)
 """
 import numpy as np
 import pytest
@@ -75,4 +76,6 @@ def test_series_forms_match_oracle(pkg, store, kind, tol):
     rms = np.sqrt(np.mean(sum(a * a for a in err[:3])))
     total = np.sqrt(np.mean(sum(a * a for a in ref[:3])))
     assert rms <= 1e-5 * scale + 1e-12 * total, (kind, tol, rms / scale)
+    e_rms, e_far, e_total = (np.sqrt(np.mean(a[3] * a[3])) for a in (err, far, ref))
+    assert e_rms <= 1e-5 * e_far + 1e-12 * e_total, (kind, tol, e_rms / e_far)
     assert abs(np.sum(err[3])) <= 1e-6 * np.sum(np.abs(ref[3])), (kind, tol)
