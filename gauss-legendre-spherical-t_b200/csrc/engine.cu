@@ -123,6 +123,7 @@ struct glst_handle {
   uint32_t shard = 0, nshards = 1;  // node split across devices (1 = whole system)
   uint32_t k_begin = 0;             // first node (internal order) of this shard
   uint32_t lr_waves = kLrWaves;     // gather warps ~ lr_waves x resident slots
+  uint32_t beside = 1;              // systems that share the GPU (a batch's branches)
   size_t part_cap = 0;              // rows the part buffer holds
   size_t sat_per_node = 0;          // shell-sum shared bytes per node
   size_t sat_budget = 0;            // shell-sum shared bytes per CTA, at most
@@ -674,7 +675,7 @@ static dev::SfArgs sf_args(const glst_handle *h, const glst_handle::FarRange &rg
   return dev::SfArgs{h->pk, h->cell_count, h->cell_point, h->tiles + rg.u0, h->dirs, h->kappa,
                      reinterpret_cast<const float4 *>(h->cheb), h->S, h->R, h->cheb_scale, h->plan.ncell,
                      rg.u1 - rg.u0, h->max_rad, rg.kb, h->sf_tab4,
-                     dev::sf_cells(h->plan.natom, h->plan.ncell, (rg.u1 - rg.u0) / dev::kSfWarps)};
+                     dev::sf_cells(h->plan.natom, h->plan.ncell, (rg.u1 - rg.u0) / dev::kSfWarps * h->beside)};
 }
 
 static glst_status sf_stage(glst_handle *h, const glst_handle::FarRange &rg, cudaStream_t st) {
@@ -1812,6 +1813,7 @@ glst_status glst_batch_create(glst_batch **out, uint32_t nsys, const uint32_t *n
       j = 1 + (uint32_t)(std::min_element(load.begin() + 1, load.end()) - (load.begin() + 1));
     b->branch_of[i] = j;
     load[j] += cost[i];
+    if (j > 0) b->sys[i]->beside = ns;
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking));
   CUDA_TRY(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming));

@@ -71,7 +71,9 @@ __host__ __device__ inline uint32_t sort_cells(uint32_t natom, uint32_t ncell) {
 // (12 at eight cells each).  Measured, one / four / eight cells, us: 26^3 cells
 // of 5 atoms at 1e-3 320 / 241 / 231 (11,000 CTAs of eight cells); 16^3 70 / 60
 // / 64 (2,000); 8^3 at the default order 222 / 223 / 239 (1,900); 6^3 93 / 100 /
-// 117 (700); 3^3 20 / 32 / 55 (50).
+// 117 (700); 3^3 20 / 32 / 55 (50).  (A batch's systems count the quads of all
+// that run beside each other: 24 boxes of 8^3 cells at 1e-4, 4.8 ms a pass
+// against 4.9 with one cell per CTA.)
 __host__ __device__ inline uint32_t sf_cells(uint32_t natom, uint32_t ncell, uint32_t quads) {
   const uint64_t ctas = (uint64_t)ncell * quads / 8;
   return natom / ncell > 16 || ctas < 12 * kSms ? 1u : ctas < 28 * kSms ? 4u : 8u;

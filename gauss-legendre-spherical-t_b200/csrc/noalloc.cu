@@ -186,7 +186,8 @@ extern "C" glst_status glst_near_field_noalloc(uint32_t natom, const double *d_r
     const uint32_t spc = dev::sort_cells(natom, (uint32_t)ncell);
     dev::k_sort_pack<<<((uint32_t)ncell + spc - 1) / spc, 32 * dev::kSortCells, dev::kSortCap * sizeof(uint32_t), st>>>(
         perm, cell_count, cell_point, g, atom_cell, natom, d_rx, d_ry, d_rz, d_qc, sorted, pk, pd);
-    dev::k_short_range<4><<<dim3((uint32_t)ncell, dev::kSrRowsPlanes), dev::kSrThreads, 0, st>>>(
+    const auto near = dev::sr_ctas(natom, (uint32_t)ncell) == 4 ? dev::k_short_range<4> : dev::k_short_range<5>;
+    near<<<dim3((uint32_t)ncell, dev::kSrRowsPlanes), dev::kSrThreads, 0, st>>>(
         pd, cell_count, cell_point, g, natom, sr, dev::kSrRowsPlanes, dev::kSrWarps,
         dev::sr_width(natom, dev::kSrRowsPlanes), dev::Pieces{nullptr, nullptr, 0xffffffffu});
     dev::k_combine<<<(natom + dev::kCombineAtoms - 1) / dev::kCombineAtoms, dev::kCombineThreads, 0, st>>>(
